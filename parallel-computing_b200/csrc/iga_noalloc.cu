@@ -134,13 +134,32 @@ Layout layout_for(int P, int nex, int ney, int TY, bool with_id)
     return L;
 }
 
+// Warps per CTA the register budget and the shared memory allow.
 template <int P>
-int launch(int dev, unsigned char *base, const Layout &Ly, int TY, int nex, int ney, const double *d_CP,
+int max_warps()
+{
+    int W = iga::apply_max_threads<P, double, 1>() / 32;
+    while (W > 1 && iga::apply_smem_bytes<P, double, 1, 2>(W, 2) > 220 * 1024) --W;
+    return W;
+}
+
+int max_warps_for(int p)
+{
+    switch (p) {
+    case 1: return max_warps<1>();
+    case 2: return max_warps<2>();
+    case 3: return max_warps<3>();
+    case 4: return max_warps<4>();
+    default: return max_warps<5>();
+    }
+}
+
+template <int P>
+int launch(int dev, int nsm, unsigned char *base, const Layout &Ly, int TY, int nex, int ney, const double *d_CP,
            const int *d_ID, const double *d_in, double *d_out, cudaStream_t s)
 {
     using namespace iga;
-    int W = apply_max_threads<P, double, 1>() / 32;
-    while (W > 1 && apply_smem_bytes<P, double, 1, 2>(W, 2) > 220 * 1024) --W;
+    int W = max_warps<P>();
     const size_t smem_max = apply_smem_bytes<P, double, 1, 2>(W, 2);
     auto kern = apply_kernel<P, double, 1, 2>;
     {
@@ -183,6 +202,7 @@ int launch(int dev, unsigned char *base, const Layout &Ly, int TY, int nex, int 
     // strips dealt to warps one by one; with shared tables the CTA's strips
     // lie in at most two column strips (W - 1 <= NSY)
     constexpr bool percol = apply_percolumn<P, double, 1>();
+    W = (int)std::max(1LL, std::min<long long>(W, ((long long)g.NSX * g.NSY + nsm - 1) / nsm));
     if (apply_txshared<P, double, 1>() && !percol) W = std::max(1, std::min(W, g.NSY + 1));
     const long long nstrips = (long long)g.NSX * g.NSY;
     const dim3 grid = percol ? dim3(g.NSX, (g.NSY + W - 1) / W) : dim3((unsigned)((nstrips + W - 1) / W)),
@@ -240,10 +260,15 @@ extern "C" int iga_MatrixFreeMatMultCUDA_noalloc(int p, int q, int nex, int ney,
                        "arrays 8-byte and d_IEN / d_ID 4-byte aligned");
         return IGA_ERR_ARG;
     }
-    // Strip height: the smallest of these whose tables and frames fit the scratch.
+    int nsm = 148, cur = 0;
+    if (cudaGetDevice(&cur) != cudaSuccess ||
+        cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, cur) != cudaSuccess)
+        nsm = 148;
+    // Strip height: that of a plan (patches of up to one wave of strips),
+    // then the smallest of these whose tables and frames fit the scratch.
     int TY = 0;
     Layout Ly{};
-    for (int cand : {32, 64, 128, 256, 512, 1024}) {
+    for (int cand : {iga::one_wave_rows(nex, ney, p, max_warps_for(p), nsm), 32, 64, 128, 256, 512, 1024}) {
         if (cand < p) continue;
         Ly = layout_for(p, nex, ney, cand, d_ID != nullptr);
         if (Ly.total <= kScratchBytes) {
@@ -281,11 +306,11 @@ extern "C" int iga_MatrixFreeMatMultCUDA_noalloc(int p, int q, int nex, int ney,
         d_dB2, d_C1, d_C2, qw1, qw2, p, nex, ney, NSX);
     int st;
     switch (p) {
-    case 1: st = launch<1>(dev, base, Ly, TY, nex, ney, d_CP, id_rows, d_in, d_out, s); break;
-    case 2: st = launch<2>(dev, base, Ly, TY, nex, ney, d_CP, id_rows, d_in, d_out, s); break;
-    case 3: st = launch<3>(dev, base, Ly, TY, nex, ney, d_CP, id_rows, d_in, d_out, s); break;
-    case 4: st = launch<4>(dev, base, Ly, TY, nex, ney, d_CP, id_rows, d_in, d_out, s); break;
-    default: st = launch<5>(dev, base, Ly, TY, nex, ney, d_CP, id_rows, d_in, d_out, s); break;
+    case 1: st = launch<1>(dev, nsm, base, Ly, TY, nex, ney, d_CP, id_rows, d_in, d_out, s); break;
+    case 2: st = launch<2>(dev, nsm, base, Ly, TY, nex, ney, d_CP, id_rows, d_in, d_out, s); break;
+    case 3: st = launch<3>(dev, nsm, base, Ly, TY, nex, ney, d_CP, id_rows, d_in, d_out, s); break;
+    case 4: st = launch<4>(dev, nsm, base, Ly, TY, nex, ney, d_CP, id_rows, d_in, d_out, s); break;
+    default: st = launch<5>(dev, nsm, base, Ly, TY, nex, ney, d_CP, id_rows, d_in, d_out, s); break;
     }
     if (st) return st;
     // Synchronous, like the reference's entry: the kernels' own error slot

@@ -628,9 +628,30 @@ static double strip_cost(int NSX, int ney, int TY, WarpShape ws, int nsm)
     return work * (1.0 + 0.5 * 3.0 / TY);
 }
 
-static int rows_for(int nex, int ney, const std::vector<WarpShape> &Ws, int nsm)
+// A patch whose 16-row strips do not fill one wave of warps (nsm SMs of W) is
+// bound by the time one warp takes to walk its strip, about 1 us a row
+// whatever the SM's other warps do (p=3 FP64: 1.0 us a row with 1-4 warps per
+// SM, 1.8 us with 12), not by bandwidth or issue. So it gets the shortest
+// strips that still fit one wave, down to the max(P, 2) rows the seams need;
+// the launch then spreads them over all SMs (launch_apply_t). Measured (B200,
+// MatMult in a graph, 16 rows in full CTAs before): p=2 64^2 FP64 29.3 -> 7.6
+// us (2 rows), p=3 256^2 31.9 -> 12.2 us (3 rows), p=3 512^2 33.1 -> 25.1 us
+// (10 rows), p=4 512^2 FP32 41.6 -> 25.6 us, on-the-fly p=5 256^2 168.9 ->
+// 53.8 us. Beyond one wave shorter strips lose to their seams and prologues
+// (p=3 512^2 in two waves of 5 rows: 29.5 us): 0 then.
+int one_wave_rows(int nex, int ney, int P, int W, int nsm)
+{
+    const long long NSX = (nex + kSW - 1) / kSW, warps = (long long)nsm * W;
+    if (NSX * ((ney + 15) / 16) > warps) return 0;
+    const long long nsy = warps / NSX;
+    return std::max({(int)((ney + nsy - 1) / nsy), P, 2});
+}
+
+static int rows_for(int nex, int ney, int P, const std::vector<WarpShape> &Ws, int nsm)
 {
     const int NSX = (nex + kSW - 1) / kSW;
+    if (Ws.size() == 1)
+        if (const int TY = one_wave_rows(nex, ney, P, Ws[0].W, nsm)) return TY;
     std::vector<int> cands = {64, 56, 48, 40, 32, 28, 24, 20, 16};
     for (const WarpShape &ws : Ws)
         if (ws.waves && ws.flat)
@@ -785,8 +806,12 @@ static int launch_apply_t(iga_plan *pl, const OperatorData &op, const T *x, T *y
     // W - 1 <= rows, in one when W divides rows (one slot: the shared memory
     // of the one-column layout, which matters where a kernel's spills live
     // in L1: FP64 on-the-fly p=5 512^2 189 -> 257 us with a second slot)
+    // Fewer strips than one wave of full CTAs: as many warps per CTA as spread
+    // them over all SMs (p=3 512^2 FP64, 16-row strips: 33.1 us in 86 CTAs of
+    // 12 warps, 29.4 us in 147 of 7).
     constexpr bool percol = apply_percolumn<P, T, GEOM>();
-    const int W = apply_txshared<P, T, GEOM>() && !percol ? std::max(1, std::min(op.warps, rows + 1)) : op.warps;
+    int W = (int)std::max(1LL, std::min<long long>(op.warps, ((long long)g.NSX * rows + pl->nsm - 1) / pl->nsm));
+    if (apply_txshared<P, T, GEOM>() && !percol) W = std::max(1, std::min(W, rows + 1));
     const size_t smem = apply_smem_bytes<P, T, GEOM, NST>(W, !percol && rows % W ? 2 : 1);
     if (win.gyn >= 0) {
         a.gy0 = win.gy0;
@@ -985,6 +1010,7 @@ int iga_plan_create(const iga_mesh_desc *d, const iga_opts *opts_in, iga_plan **
     pl->sign = opts.sign;
     pl->bc = opts.bc;
     pl->device = opts.device;
+    pl->nsm = nsm;
     pl->arena = plan_arena();
     // Rows per strip, per operator: a MIXED plan's FP64 and FP32 operators
     // have their own G layouts, so each gets the strip height that fills the
@@ -992,7 +1018,7 @@ int iga_plan_create(const iga_mesh_desc *d, const iga_opts *opts_in, iga_plan **
     auto rows_of = [&](int prec) {
         if (opts.rows_per_strip > 0) return opts.rows_per_strip;
         const bool shared_flat = prec == IGA_FP64 && (opts.geometry == IGA_GEOM_PRECOMPUTED ? P.p >= 4 : P.p <= 2);
-        return rows_for(P.nex, P.ney, {{warps_for(P.p, prec, opts.geometry), apply_flat(P.p, prec, opts.geometry),
+        return rows_for(P.nex, P.ney, P.p, {{warps_for(P.p, prec, opts.geometry), apply_flat(P.p, prec, opts.geometry),
                                          shared_flat}},
                         nsm);
     };

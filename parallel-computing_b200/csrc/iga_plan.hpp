@@ -127,6 +127,10 @@ int refentry_status(int flags);
 // (IGA_FP64 / IGA_FP32) and geometry mode that fits the shared-memory budget.
 int warps_for(int P, int prec, int geom);
 
+// Rows per strip of a patch whose strips fit one wave of W warps on each of
+// nsm SMs (0: it does not, or 16-row strips already fill it).
+int one_wave_rows(int nex, int ney, int P, int W, int nsm);
+
 }  // namespace iga
 
 struct iga_plan {
@@ -134,6 +138,7 @@ struct iga_plan {
     long long nfunc = 0;
     int precision = IGA_FP64, geometry = IGA_GEOM_PRECOMPUTED, sign = IGA_SIGN_REFERENCE, bc = IGA_BC_REFERENCE;
     int device = 0;
+    int nsm = 148;   // SMs of the device
     iga::StripGrid grid{};
     iga::Patch patch;
     iga::OperatorData op64, op32;
