@@ -37,7 +37,14 @@ struct DevScalars {
     int done, breakdown, idone, iiters, ibreak, imax;
     int err;                                        // a bounded wait in a kernel gave up
     int it, maxit;                                  // outer PCG in a device-side loop
+    long long ipc;                                  // inner iterations of one call's cluster FEM-CG solves
 };
+
+}  // namespace iga
+
+#include "iga_femcg.cuh"
+
+namespace iga {
 
 // ------------------------------------------------------------ reductions
 // Block sums of K values; the last block to finish sums the per-block
@@ -358,7 +365,7 @@ __global__ void pcg_pq_kernel(const T *__restrict__ p, const T *__restrict__ q, 
     });
     double tot[1];
     if (reduce_last<1>(v, partials, counter, tot) && threadIdx.x == 0) {
-        if (!(tot[0] > 0.0)) {
+        if (!(tot[0] > 0.0) || s->breakdown) {   // breakdown already set: by the preconditioner
             s->breakdown = 1;
             s->alpha = 0.0;
         } else {
@@ -433,10 +440,11 @@ __global__ void loop_init_kernel(DevScalars *s, double tol2, int maxit)
 }
 
 // Flexible (Polak-Ribiere) beta = r.(z - z_old) / rz_old with r.z_old = rzo
-// from the update kernel; rz = r.z.
+// from the update kernel; rz = r.z. loop: in the device-side loop, whose first
+// pass has no old direction (beta = 0).
 template <typename T>
 __global__ void pcg_beta_kernel(const T *__restrict__ r, const T *__restrict__ z, long long N, DevScalars *s,
-                                double *partials, unsigned *counter)
+                                double *partials, unsigned *counter, int loop)
 {
     pdl_begin();
     double v[1] = {0.0};
@@ -448,15 +456,18 @@ __global__ void pcg_beta_kernel(const T *__restrict__ r, const T *__restrict__ z
     });
     double tot[1];
     if (reduce_last<1>(v, partials, counter, tot) && threadIdx.x == 0) {
-        s->beta = (tot[0] - s->rzo) / s->rz;
+        s->beta = loop && s->it == 0 ? 0.0 : (tot[0] - s->rzo) / s->rz;
         s->rz = tot[0];
     }
 }
 
+// first: 1 the first direction (p = z), 0 a later one, -1 by the device-side
+// loop's iteration count.
 template <typename T>
 __global__ void pcg_p_kernel(T *__restrict__ p, const T *__restrict__ z, long long N, const DevScalars *s, int first)
 {
     pdl_begin();
+    if (first < 0) first = s->it == 0;
     const T be = first ? T(0) : (T)s->beta;
     vloop<T>(N, al16(p) && al16(z), [&](long long i, int c) {
         const Pk<T> zv = ldc(z, i, c);
@@ -897,6 +908,9 @@ struct PrecState {
     // iteration per pass (built for one preconditioner / kappa-scaling choice)
     cudaGraphExec_t loop = nullptr;
     int loop_pc = -1, loop_scaled = -1, loop_prec = -1;
+    double loop_pc_rtol = 0.0;   // IGA_PC_FEM_CG: the inner solve's parameters in the loop
+    int loop_pc_max_it = 0;
+    IcgShape icg;                // IGA_PC_FEM_CG in one cluster (C = 0: the grid does not fit)
     bool loop_failed = false;   // the loop graph could not be instantiated: host-driven loop
     FemCoef<T> coef() const
     {
@@ -910,6 +924,7 @@ struct PrecState {
 struct SolverState {
     int device = 0;
     cudaStream_t stream = nullptr;
+    bool pc_sync = false;   // IGA_PC_FEM_CG: the call wants the inner solve's status at once
     bool fd_host = false;
     // host x eigenpairs (built once). Split by parity (fold): even modes
     // 0 .. fe-1 then odd modes, Vx = the fe x fe even block followed by the
@@ -1004,6 +1019,48 @@ void net_lengths(const Patch &P, double &Lx, double &Ly)
     } while (0)
 
 template <typename T>
+static void (*icg_kernel(int L))(IcgArgs<T>)
+{
+    return L == 1 ? icg_cluster_kernel<T, 1> : L == 2 ? icg_cluster_kernel<T, 2> : L == 4 ? icg_cluster_kernel<T, 4>
+                                                                                           : icg_cluster_kernel<T, 8>;
+}
+
+// The cluster shape of the inner FEM-CG for this plan's grid: the largest
+// cluster (16 CTAs needs the non-portable size) the device can place.
+template <typename T>
+static int icg_prepare(PrecState<T> &ps, const iga_plan *pl)
+{
+    for (int cmax = kIcgMaxCluster; cmax >= 8; cmax /= 2) {
+        const IcgShape sh = icg_shape<T>(pl->m, pl->n, cmax);
+        if (!sh.C) continue;
+        auto kern = icg_kernel<T>(sh.L);
+        if (sh.C > 8 && cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) {
+            cudaGetLastError();
+            continue;
+        }
+        SOLVE_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sh.smem));
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3(sh.C);
+        cfg.blockDim = dim3(sh.threads);
+        cfg.dynamicSmemBytes = sh.smem;
+        cudaLaunchAttribute at[1];
+        at[0].id = cudaLaunchAttributeClusterDimension;
+        at[0].val.clusterDim.x = sh.C;
+        at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+        cfg.attrs = at;
+        cfg.numAttrs = 1;
+        int fit = 0;
+        if (cudaOccupancyMaxActiveClusters(&fit, kern, &cfg) != cudaSuccess || fit < 1) {
+            cudaGetLastError();
+            continue;
+        }
+        ps.icg = sh;
+        return IGA_OK;
+    }
+    return IGA_OK;
+}
+
+template <typename T>
 static int alloc_prec(PrecState<T> &ps, const iga_plan *pl, const SolverState &S)
 {
     if (ps.ready) return IGA_OK;
@@ -1023,6 +1080,7 @@ static int alloc_prec(PrecState<T> &ps, const iga_plan *pl, const SolverState &S
         return st;
     for (T **v : {&ps.x, &ps.r, &ps.z, &ps.tz, &ps.p, &ps.q, &ps.b, &ps.sc, &ps.iz, &ps.ir, &ps.ip, &ps.iq})
         SOLVE_TRY(cudaMalloc((void **)v, sizeof(T) * N));
+    if ((st = icg_prepare(ps, pl))) return st;
     ps.ready = true;
     return IGA_OK;
 }
@@ -1395,6 +1453,13 @@ static int fd_apply(PrecState<T> &ps, const iga_plan *pl, SolverState *S, const 
     return IGA_OK;
 }
 
+static int sync_scalars(SolverState *S)
+{
+    SOLVE_TRY(cudaMemcpyAsync(S->h, S->s, sizeof(DevScalars), cudaMemcpyDeviceToHost, S->stream));
+    SOLVE_TRY(cudaStreamSynchronize(S->stream));
+    return IGA_OK;
+}
+
 template <typename T>
 static int pc_apply_core(PrecState<T> &ps, const iga_plan *pl, SolverState *S, const iga_solve_opts &o, const T *r,
                          T *z, double pc_rtol, int64_t &pc_iters);
@@ -1483,6 +1548,40 @@ static int pc_apply_core(PrecState<T> &ps, const iga_plan *pl, SolverState *S, c
         if ((st = fd_upload(ps, pl, S))) return st;
         return fd_apply<T, T>(ps, pl, S, r, z, nullptr);
     }
+    if (ps.icg.C) {   // one cluster runs the whole inner solve
+        IcgArgs<T> a;
+        a.kd = ps.kd; a.ko = ps.ko; a.md = ps.md; a.mo = ps.mo;
+        a.ld = ps.ld; a.lo = ps.lo; a.nd = ps.nd; a.no = ps.no;
+        a.m = pl->m;
+        a.n = pl->n;
+        a.rows = ps.icg.rows;
+        a.rhs = r;
+        a.z = z;
+        a.rtol = pc_rtol;
+        a.maxit = o.pc_max_it;
+        a.zero_on_break = !S->pc_sync;
+        a.s = S->s;
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3(ps.icg.C);
+        cfg.blockDim = dim3(ps.icg.threads);
+        cfg.dynamicSmemBytes = ps.icg.smem;
+        cfg.stream = S->stream;
+        cudaLaunchAttribute at[2];
+        at[0].id = cudaLaunchAttributeClusterDimension;
+        at[0].val.clusterDim.x = ps.icg.C;
+        at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+        at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        at[1].val.programmaticStreamSerializationAllowed = 1;
+        cfg.attrs = at;
+        cfg.numAttrs = pdl_capture() ? 2 : 1;
+        if (S->pc_sync) SOLVE_TRY(cudaMemsetAsync(&S->s->ibreak, 0, sizeof(int), S->stream));
+        SOLVE_TRY(cudaLaunchKernelEx(&cfg, icg_kernel<T>(ps.icg.L), a));
+        if (S->pc_sync) {
+            if ((st = sync_scalars(S))) return st;
+            if (S->h->ibreak) return IGA_ERR_BREAKDOWN;
+        }
+        return IGA_OK;
+    }
     if ((st = inner_chunk_graph(ps, pl, S))) return st;
     InnerCG<T> a = inner_of(ps, pl, S);
     icg_init_kernel<T><<<kRedBlocks, kThreads, 0, S->stream>>>(a, r, pc_rtol, o.pc_max_it);
@@ -1510,13 +1609,6 @@ static int pc_apply_core(PrecState<T> &ps, const iga_plan *pl, SolverState *S, c
     return IGA_OK;
 }
 
-static int sync_scalars(SolverState *S)
-{
-    SOLVE_TRY(cudaMemcpyAsync(S->h, S->s, sizeof(DevScalars), cudaMemcpyDeviceToHost, S->stream));
-    SOLVE_TRY(cudaStreamSynchronize(S->stream));
-    return IGA_OK;
-}
-
 // Flexible PCG on K x = b in precision T, from the current x; stops when the
 // recurrence residual satisfies ||r|| <= rtol ||b_ref||. Returns iterations.
 template <typename T>
@@ -1531,10 +1623,10 @@ static int pcg(iga_plan *pl, SolverState *S, PrecState<T> &ps, const iga_solve_o
     sub_kernel<T><<<kRedBlocks, kThreads, 0, s>>>(b, ps.q, ps.r, N, S->s, S->partials, S->counter);
     if ((st = sync_scalars(S))) return st;
     if (std::sqrt(S->h->rr) <= rtol * bnorm) return IGA_OK;
+    cudaMemsetAsync(&S->s->breakdown, 0, sizeof(int), s);
     if ((st = pc_apply(ps, pl, S, o, ps.r, ps.z, pc_rtol, pc_iters))) return st;
     dot_kernel<T><<<kRedBlocks, kThreads, 0, s>>>(ps.r, ps.z, N, &S->s->rz, S->partials, S->counter);
     pcg_p_kernel<T><<<kRedBlocks, kThreads, 0, s>>>(ps.p, ps.z, N, S->s, 1);
-    cudaMemsetAsync(&S->s->breakdown, 0, sizeof(int), s);
     for (int it = 0; it < o.max_it; ++it) {
         if ((st = iga_apply_internal_sb(pl, prec, ps.p, ps.q, s, IGA_SIGN_SPD, IGA_BC_IDENTITY))) return st;
         pcg_pq_kernel<T><<<kRedBlocks, kThreads, 0, s>>>(ps.p, ps.q, N, S->s, S->partials, S->counter);
@@ -1546,20 +1638,24 @@ static int pcg(iga_plan *pl, SolverState *S, PrecState<T> &ps, const iga_solve_o
         if (!std::isfinite(S->h->rr)) return IGA_ERR_NONFINITE;
         if (std::sqrt(S->h->rr) <= rtol * bnorm) return IGA_OK;
         if ((st = pc_apply(ps, pl, S, o, ps.r, ps.z, pc_rtol, pc_iters))) return st;
-        pcg_beta_kernel<T><<<kRedBlocks, kThreads, 0, s>>>(ps.r, ps.z, N, S->s, S->partials, S->counter);
+        pcg_beta_kernel<T><<<kRedBlocks, kThreads, 0, s>>>(ps.r, ps.z, N, S->s, S->partials, S->counter, 0);
         pcg_p_kernel<T><<<kRedBlocks, kThreads, 0, s>>>(ps.p, ps.z, N, S->s, 0);
     }
     return IGA_ERR_NOT_CONVERGED;
 }
 
 // Builds the device-side loop for the current preconditioner choice: body =
-// q = K p; alpha; x += alpha p, r -= alpha q, r.z_old (+ loop condition);
-// z = M^-1 r; beta; p = z + beta p, on the fixed buffers of ps.
+// z = M^-1 r; beta; p = z + beta p (p = z in the first pass); q = K p; alpha;
+// x += alpha p, r -= alpha q, r.z (+ loop condition), on the fixed buffers of
+// ps. With the preconditioner first no pass ends on one whose result nobody
+// reads (a 12-iteration solve of four sweeps otherwise applies it 16 times).
 template <typename T>
 static int build_loop(iga_plan *pl, SolverState *S, PrecState<T> &ps, const iga_solve_opts &o, int prec)
 {
     const int scaled = pl->kappa_dev ? 1 : 0;
-    if (ps.loop_pc == o.pc && ps.loop_scaled == scaled && ps.loop_prec == o.precision && (ps.loop || ps.loop_failed))
+    const bool same_pc = ps.loop_pc == o.pc && (o.pc != IGA_PC_FEM_CG || (ps.loop_pc_rtol == o.pc_rtol &&
+                                                                         ps.loop_pc_max_it == o.pc_max_it));
+    if (same_pc && ps.loop_scaled == scaled && ps.loop_prec == o.precision && (ps.loop || ps.loop_failed))
         return ps.loop ? IGA_OK : IGA_ERR_UNSUPPORTED;
     if (ps.loop) {
         cudaGraphExecDestroy(ps.loop);
@@ -1581,10 +1677,9 @@ static int build_loop(iga_plan *pl, SolverState *S, PrecState<T> &ps, const iga_
     cudaGraph_t body = np.conditional.phGraph_out[0];
     SOLVE_TRY(cudaStreamBeginCaptureToGraph(s, body, nullptr, nullptr, 0, cudaStreamCaptureModeRelaxed));
     int64_t dummy = 0;
-    // Programmatic dependencies between the body's kernels (the inner-CG
-    // preconditioner runs child graphs and keeps ordinary edges).
-    pdl_capture() = o.pc != IGA_PC_FEM_CG;
-    int st = iga_apply_internal_sb(pl, prec, ps.p, ps.q, s, IGA_SIGN_SPD, IGA_BC_IDENTITY);
+    // Programmatic dependencies between the body's kernels.
+    pdl_capture() = true;
+    int st = pc_apply(ps, pl, S, o, ps.r, ps.z, o.pc_rtol, dummy);
     auto launched = [&](cudaError_t e) {
         if (e != cudaSuccess && !st) {
             set_error(std::string("PCG loop launch: ") + cudaGetErrorString(e));
@@ -1592,17 +1687,17 @@ static int build_loop(iga_plan *pl, SolverState *S, PrecState<T> &ps, const iga_
         }
     };
     if (!st) {
+        launched(launch_k(pcg_beta_kernel<T>, dim3(kRedBlocks), dim3(kThreads), 0, s, (const T *)ps.r,
+                          (const T *)ps.z, N, S->s, S->partials, S->counter, 1));
+        launched(launch_k(pcg_p_kernel<T>, dim3(kRedBlocks), dim3(kThreads), 0, s, ps.p, (const T *)ps.z, N,
+                          (const DevScalars *)S->s, -1));
+        if (!st) st = iga_apply_internal_sb(pl, prec, ps.p, ps.q, s, IGA_SIGN_SPD, IGA_BC_IDENTITY);
+    }
+    if (!st) {
         launched(launch_k(pcg_pq_kernel<T>, dim3(kRedBlocks), dim3(kThreads), 0, s, (const T *)ps.p, (const T *)ps.q,
                           N, S->s, S->partials, S->counter));
         launched(launch_k(pcg_xr_cond_kernel<T>, dim3(kRedBlocks), dim3(kThreads), 0, s, ps.x, ps.r, (const T *)ps.p,
                           (const T *)ps.q, (const T *)ps.z, N, S->s, S->partials, S->counter, h));
-        if (!st) st = pc_apply(ps, pl, S, o, ps.r, ps.z, o.pc_rtol, dummy);
-    }
-    if (!st) {
-        launched(launch_k(pcg_beta_kernel<T>, dim3(kRedBlocks), dim3(kThreads), 0, s, (const T *)ps.r,
-                          (const T *)ps.z, N, S->s, S->partials, S->counter));
-        launched(launch_k(pcg_p_kernel<T>, dim3(kRedBlocks), dim3(kThreads), 0, s, ps.p, (const T *)ps.z, N,
-                          (const DevScalars *)S->s, 0));
     }
     pdl_capture() = false;
     cudaGraph_t captured = body;
@@ -1625,6 +1720,8 @@ static int build_loop(iga_plan *pl, SolverState *S, PrecState<T> &ps, const iga_
         ps.loop_pc = o.pc;
         ps.loop_scaled = scaled;
         ps.loop_prec = o.precision;
+        ps.loop_pc_rtol = o.pc_rtol;
+        ps.loop_pc_max_it = o.pc_max_it;
         ps.loop_failed = true;
         return IGA_ERR_UNSUPPORTED;
     }
@@ -1633,6 +1730,8 @@ static int build_loop(iga_plan *pl, SolverState *S, PrecState<T> &ps, const iga_
     ps.loop_pc = o.pc;
     ps.loop_scaled = scaled;
     ps.loop_prec = o.precision;
+    ps.loop_pc_rtol = o.pc_rtol;
+    ps.loop_pc_max_it = o.pc_max_it;
     return IGA_OK;
 }
 
@@ -1664,13 +1763,9 @@ static int pcg_graph(iga_plan *pl, SolverState *S, PrecState<T> &ps, const iga_s
         if ((st = sync_scalars(S))) return st;
         if (std::sqrt(S->h->rr) <= rtol * bnorm) return IGA_OK;
     }
-    int64_t dummy = 0;
-    if ((st = pc_apply(ps, pl, S, o, ps.r, ps.z, o.pc_rtol, dummy))) return st;
-    dot_kernel<T><<<kRedBlocks, kThreads, 0, s>>>(ps.r, ps.z, N, &S->s->rz, S->partials, S->counter);
-    pcg_p_kernel<T><<<kRedBlocks, kThreads, 0, s>>>(ps.p, ps.z, N, S->s, 1);
     st = pl->solver_graph ? build_loop(pl, S, ps, o, prec) : IGA_ERR_UNSUPPORTED;
     if (st == IGA_ERR_UNSUPPORTED) {   // e.g. a library kernel not allowed in a conditional body, or the host loop asked for
-        int64_t pcits = 0;
+        int64_t pcits = 0;   // the cluster FEM-CG counts on the device
         st = pcg<T>(pl, S, ps, o, ps.b, ps.x, rtol, bnorm, o.pc_rtol, prec, its, pcits);
         if (x != ps.x) copy_kernel<T><<<kRedBlocks, kThreads, 0, s>>>(x, ps.x, N);
         return st;
@@ -1748,13 +1843,15 @@ int iga_pc_apply(iga_plan *pl, int pc, int prec, const void *r, void *z, double 
     o.pc = pc;
     o.pc_max_it = pc_max_it;
     int64_t its = 0;
+    S->pc_sync = true;
     if (prec == IGA_FP64) {
-        if ((st = alloc_prec(S->d, pl, *S))) return st;
-        st = pc_apply<double>(S->d, pl, S, o, (const double *)r, (double *)z, pc_rtol, its);
+        if (!(st = alloc_prec(S->d, pl, *S)))
+            st = pc_apply<double>(S->d, pl, S, o, (const double *)r, (double *)z, pc_rtol, its);
     } else {
-        if ((st = alloc_prec(S->f, pl, *S))) return st;
-        st = pc_apply<float>(S->f, pl, S, o, (const float *)r, (float *)z, pc_rtol, its);
+        if (!(st = alloc_prec(S->f, pl, *S)))
+            st = pc_apply<float>(S->f, pl, S, o, (const float *)r, (float *)z, pc_rtol, its);
     }
+    S->pc_sync = false;
     SOLVE_TRY(cudaEventRecord(ev, S->stream));
     SOLVE_TRY(cudaStreamWaitEvent((cudaStream_t)stream, ev, 0));
     cudaEventDestroy(ev);
@@ -1868,6 +1965,8 @@ int iga_solve(iga_plan *pl, const double *b, double *x, const iga_solve_opts *o_
     const long long N = pl->nfunc;
     iga_solve_stats stt{};
     SOLVE_TRY(cudaMemsetAsync(&S->s->err, 0, sizeof(int), S->stream));
+    SOLVE_TRY(cudaMemsetAsync(&S->s->ibreak, 0, sizeof(int), S->stream));
+    SOLVE_TRY(cudaMemsetAsync(&S->s->ipc, 0, sizeof(long long), S->stream));
     if (!o.x0_nonzero) zero_kernel<double><<<kRedBlocks, kThreads, 0, S->stream>>>(x, N);
     if ((st = true_residual(pl, S, b, x))) return st;
     if (!std::isfinite(S->h->bb) || !std::isfinite(S->h->rr)) {
@@ -1888,7 +1987,9 @@ int iga_solve(iga_plan *pl, const double *b, double *x, const iga_solve_opts *o_
         if (o.precision == IGA_MIXED_PC && o.pc != IGA_PC_NONE && (st = alloc_prec(S->f, pl, *S))) return st;
         // Restart from the true residual until it meets rtol (recurrence drift).
         for (int restart = 0; restart < 4 && rel > o.rtol; ++restart) {
-            st = o.pc == IGA_PC_FEM_CG
+            // the inner FEM-CG of grids past one cluster is driven by the host
+            const bool host = o.pc == IGA_PC_FEM_CG && !(o.precision == IGA_MIXED_PC ? S->f.icg.C : S->d.icg.C);
+            st = host
                      ? pcg<double>(pl, S, S->d, o, b, x, o.rtol, bnorm, o.pc_rtol, IGA_FP64, stt.iterations,
                                    stt.pc_iterations)
                      : pcg_graph<double>(pl, S, S->d, o, b, x, o.rtol, bnorm, IGA_FP64, stt.iterations);
@@ -1915,7 +2016,7 @@ int iga_solve(iga_plan *pl, const double *b, double *x, const iga_solve_opts *o_
             const double srtol = std::max(o.sweep_rtol, std::min(0.2 * need, 0.5));
             scale_down_kernel<<<kRedBlocks, kThreads, 0, S->stream>>>(S->r64, S->f.b, N, S->s);
             zero_kernel<float><<<kRedBlocks, kThreads, 0, S->stream>>>(S->f.x, N);
-            st = o.pc == IGA_PC_FEM_CG
+            st = o.pc == IGA_PC_FEM_CG && !S->f.icg.C
                      ? pcg<float>(pl, S, S->f, o, S->f.b, S->f.x, srtol, 1.0, o.pc_rtol, IGA_FP32, stt.iterations,
                                   stt.pc_iterations)
                      : pcg_graph<float>(pl, S, S->f, o, S->f.b, S->f.x, srtol, 1.0, IGA_FP32, stt.iterations, true);
@@ -1938,6 +2039,7 @@ int iga_solve(iga_plan *pl, const double *b, double *x, const iga_solve_opts *o_
     SOLVE_TRY(cudaStreamSynchronize(S->stream));
     cudaEventDestroy(ev);
     stt.relres = rel;
+    stt.pc_iterations += S->h->ipc;
     if (S->h->err) {   // host copy current as of the last true residual
         set_error("a bounded device wait gave up in the preconditioner");
         result = IGA_ERR_TIMEOUT;
@@ -1981,11 +2083,13 @@ int iga_spectrum_estimate(iga_plan *pl, int pc, int steps, uint64_t seed, double
     SOLVE_TRY(cudaMemcpyAsync(ps.r, h.data(), sizeof(double) * N, cudaMemcpyHostToDevice, s));
     zero_kernel<double><<<kRedBlocks, kThreads, 0, s>>>(ps.x, N);
     int64_t pcits = 0;
+    SOLVE_TRY(cudaMemsetAsync(&S->s->breakdown, 0, sizeof(int), s));
+    SOLVE_TRY(cudaMemsetAsync(&S->s->ibreak, 0, sizeof(int), s));
     if ((st = pc_apply(ps, pl, S, o, ps.r, ps.z, o.pc_rtol, pcits))) return st;
     dot_kernel<double><<<kRedBlocks, kThreads, 0, s>>>(ps.r, ps.z, N, &S->s->rz, S->partials, S->counter);
     pcg_p_kernel<double><<<kRedBlocks, kThreads, 0, s>>>(ps.p, ps.z, N, S->s, 1);
-    SOLVE_TRY(cudaMemsetAsync(&S->s->breakdown, 0, sizeof(int), s));
     if ((st = sync_scalars(S))) return st;
+    if (S->h->ibreak) return IGA_ERR_BREAKDOWN;
     const double rr0 = S->h->rz;
     std::vector<double> alpha, beta;
     for (int k = 0; k < steps; ++k) {
@@ -1997,6 +2101,7 @@ int iga_spectrum_estimate(iga_plan *pl, int pc, int steps, uint64_t seed, double
         if ((st = pc_apply(ps, pl, S, o, ps.r, ps.z, o.pc_rtol, pcits))) return st;
         dot_kernel<double><<<kRedBlocks, kThreads, 0, s>>>(ps.r, ps.z, N, &S->s->rz, S->partials, S->counter);
         if ((st = sync_scalars(S))) return st;
+        if (S->h->ibreak) return IGA_ERR_BREAKDOWN;
         if (S->h->breakdown || !(S->h->alpha > 0.0)) break;
         alpha.push_back(S->h->alpha);
         const double rz_new = S->h->rz;

@@ -51,3 +51,45 @@ def test_strip_height_of_small_patches(torch_cuda, ib, orc, p, nex, ney, geom):
         plan.apply(xd, yd, precision=prec)
         assert rel(yd.double().cpu().numpy(), ref) < tol
     plan.close()
+
+
+# The inner FEM-CG in one cluster: one row per thread (64^2), two, four and
+# eight, fewer grid rows than CTAs, a 3-node direction, the first sizes past
+# the cluster (600 x 300: the launch-per-step path). Its stop is the recurrence
+# residual at pc_rtol; the true residual may exceed it by the rounding of the
+# iteration, well under pc_rtol itself in FP64 (condition ~ 1e4 x 1e-16); in
+# FP32 (condition 4e3 x 6e-8 = 2.4e-4) under a pc_rtol of 1e-3.
+@pytest.mark.parametrize("p,nex,ney", [(2, 64, 64), (2, 1, 1), (3, 40, 1), (1, 2, 30), (2, 17, 90), (3, 96, 128),
+                                       (2, 255, 62), (3, 300, 125), (2, 600, 300)])
+@pytest.mark.parametrize("prec", [0, 1])
+def test_fem_cg_in_a_cluster(torch_cuda, ib, orc, p, nex, ney, prec):
+    plan = ib.Plan(ib.unit_square(p, nex, ney))
+    gx, gy = plan.fem_nodes()
+    r = splitmix_uniform(p + 7 * nex, -1.0, 1.0, plan.nfunc)   # boundary entries not zero
+    dt = torch_cuda.float32 if prec else torch_cuda.float64
+    rd = torch_cuda.from_numpy(r).to("cuda", dt)
+    zd = torch_cuda.full_like(rd, float("nan"))
+    tol = 1e-3 if prec else 1e-10
+    plan.pc_apply(rd, zd, pc=ib.PC_FEM_CG, precision=prec, pc_rtol=tol)
+    rr = rd.double().cpu().numpy()
+    res = orc.fem_matvec(gx, gy, zd.double().cpu().numpy()) - rr
+    assert np.linalg.norm(res) <= 2 * tol * np.linalg.norm(rr)
+    # the same call twice gives the same bits; one iteration at most: z = alpha r / diag
+    z2 = torch_cuda.full_like(rd, float("nan"))
+    plan.pc_apply(rd, z2, pc=ib.PC_FEM_CG, precision=prec, pc_rtol=tol)
+    assert torch_cuda.equal(zd, z2)
+    plan.close()
+
+
+def test_fem_cg_breakdown_and_zero(torch_cuda, ib):
+    plan = ib.Plan(ib.unit_square(2, 40, 33))
+    r = torch_cuda.ones(plan.nfunc, dtype=torch_cuda.float64, device="cuda")
+    r[500] = float("nan")
+    z = torch_cuda.full_like(r, 3.0)
+    with pytest.raises(ib.IgaError):
+        plan.pc_apply(r, z, pc=ib.PC_FEM_CG)
+    assert torch_cuda.equal(z, torch_cuda.full_like(r, 3.0))   # left as it was
+    r.zero_()
+    plan.pc_apply(r, z, pc=ib.PC_FEM_CG)
+    assert float(z.abs().max()) == 0.0
+    plan.close()
