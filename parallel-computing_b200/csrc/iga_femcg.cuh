@@ -4,18 +4,21 @@
 // one thread-block cluster.
 //
 // What bounds it: latency. A 66 x 66 grid has 4356 unknowns; as three
-// launches per iteration (stencil + p.q, update, direction; 16 launches'
-// worth captured per graph) an iteration took 16 us, nearly all of it launch
-// gaps and grid-wide reductions. Here one cluster of up to 16 CTAs runs every
-// iteration: CTA k owns a band of grid rows, thread (i, g) the L consecutive
-// rows of column i in group g, with r, z and 1 / diag in registers and p in
-// shared memory (one halo row on either side). Per iteration two cluster
-// barriers: the warps' partial sums go straight into every CTA's slots
-// through distributed shared memory, and after the barrier every warp sums
-// all slots in the same order, so all threads hold the same totals without a
-// broadcast (deterministic; sums in FP64). The direction's halo rows are
-// recomputed locally: the neighbours send r / diag of their edge rows with
-// the second reduction, which saves a third barrier.
+// launches per iteration (stencil + p.q, update, direction) an iteration took
+// 16.4 us, nearly all of it launch gaps and grid-wide reductions. Here one
+// cluster of CTAs runs every iteration: CTA k owns a band of grid rows, thread
+// (i, g) the L consecutive rows of column i in group g, with r, z and 1 / diag
+// in registers and p in shared memory (one halo row on either side). The
+// warps' partial sums go straight into every CTA's slots (st.async through
+// distributed shared memory, counted by the receiver's mbarrier), and every
+// warp sums all slots in the same order, so all threads hold the same totals
+// without a broadcast (deterministic; sums in FP64). The direction's halo
+// rows are recomputed locally: the neighbours send r / diag of their edge rows
+// with the second sum, which saves a third exchange. So an iteration has two
+// exchanges and one CTA barrier but no cluster barrier: with two cluster
+// barriers (arrive.release / wait.acquire) in their place an iteration at 64^2
+// took 2.9 us, 22% of the stalls on the release fence, against 2.2 us (128^2:
+// 4.1 against 2.9).
 #pragma once
 #include <cuda_runtime.h>
 
@@ -25,8 +28,6 @@
 
 namespace iga {
 
-constexpr int kIcgMaxCluster = 16;
-
 // Launch shape of icg_cluster_kernel for an m x n grid: cluster CTAs (0: the
 // grid does not fit), rows per CTA, rows per thread, threads, shared bytes.
 struct IcgShape {
@@ -34,38 +35,45 @@ struct IcgShape {
     size_t smem = 0;
 };
 
-// Threads a CTA of L rows per thread may have (the kernel's launch bounds).
-__host__ __device__ constexpr int icg_max_threads(int L) { return L <= 2 ? 1024 : 512; }
+constexpr int kIcgMaxThreads = 512;   // of a CTA (the kernel's launch bounds)
 
 template <typename T>
 inline size_t icg_smem(int m, int rows, int C, int nw)
 {
-    // reduction slots (p.q; r.z and r.r), p with halo rows (one entry of
-    // slack at both ends), the neighbours' r / diag, the y coefficients
-    return sizeof(double) * 3 * (size_t)C * nw +
+    // three mbarriers, the slots (r.z and r.r; p.q), p with halo rows (one entry
+    // of slack at both ends), the neighbours' r / diag, the y coefficients
+    return 32 + sizeof(double) * 3 * (size_t)C * nw +
            sizeof(T) * ((size_t)m * (rows + 2) + 2 + 2 * (size_t)m + 6 * (size_t)rows);
 }
 
-// The fewest rows per thread whose CTAs fit, with as many CTAs as cmax (a
-// power of two) allows but no more than the rows: an iteration's time is its
-// barriers plus one thread's rows.
+// Shape k = 0 .. 3 in the order of preference (C = 0: does not fit, or no
+// further shape). Eight CTAs (the portable cluster size) before sixteen, whose
+// sums have twice the slots (64^2 with cluster
+// barriers: 3.2 us an iteration against 2.9), and four
+// rows per thread where the band has them: with fewer, more warps share the
+// SM's shuffle and shared-memory pipes for their sums (64^2, eight CTAs: 3.27
+// us with one row per thread, 3.15 with two, 2.90 with four), with eight a
+// thread's own rows dominate (4.13; 128^2: 5.0 us in eight CTAs of eight
+// rows, 4.1 in sixteen of four).
 template <typename T>
-inline IcgShape icg_shape(int m, int n, int cmax)
+inline IcgShape icg_shape(int m, int n, int k)
 {
+    const int cmax = k == 0 || k == 2 ? 8 : 16, L = k < 2 ? 4 : 8;
     IcgShape s;
     int C = 1;
     while (2 * C <= cmax && 2 * C <= n) C *= 2;
     const int rows = (n + C - 1) / C;
-    for (int L = 1; L <= 8; L *= 2) {
-        const long long threads = (long long)m * ((rows + L - 1) / L);
-        if (threads > icg_max_threads(L)) continue;
-        s.C = C;
-        s.rows = rows;
+    const long long threads = (long long)m * ((rows + L - 1) / L);
+    if (threads > kIcgMaxThreads) return s;
+    s.C = C;
+    s.rows = rows;
+    s.L = L == 4 && rows < 4 ? (rows >= 2 ? 2 : 1) : L;
+    s.threads = (int)(((long long)m * ((rows + s.L - 1) / s.L) + 31) / 32 * 32);
+    if (s.threads > kIcgMaxThreads) {
         s.L = L;
         s.threads = (int)((threads + 31) / 32 * 32);
-        s.smem = icg_smem<T>(m, rows, C, s.threads / 32);
-        return s;
     }
+    s.smem = icg_smem<T>(m, rows, C, s.threads / 32);
     return s;
 }
 
@@ -94,13 +102,44 @@ __device__ __forceinline__ uint32_t cluster_addr(const void *p, int rank)
     asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(smem_u32(p)), "r"(rank));
     return a;
 }
-__device__ __forceinline__ void cluster_store(uint32_t a, double v)
+// Store into a CTA of the cluster, counted in bytes by the mbarrier there.
+__device__ __forceinline__ void cluster_store(uint32_t a, double v, uint32_t bar)
 {
-    asm volatile("st.shared::cluster.f64 [%0], %1;" ::"r"(a), "d"(v) : "memory");
+    asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.f64 [%0], %1, [%2];" ::"r"(a), "d"(v),
+                 "r"(bar)
+                 : "memory");
 }
-__device__ __forceinline__ void cluster_store(uint32_t a, float v)
+__device__ __forceinline__ void cluster_store(uint32_t a, float v, uint32_t bar)
 {
-    asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(a), "f"(v) : "memory");
+    asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.f32 [%0], %1, [%2];" ::"r"(a), "f"(v),
+                 "r"(bar)
+                 : "memory");
+}
+__device__ __forceinline__ void cluster_store(uint32_t a, double2 v, uint32_t bar)
+{
+    asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.v2.f64 [%0], {%1, %2}, [%3];" ::"r"(a),
+                 "d"(v.x), "d"(v.y), "r"(bar)
+                 : "memory");
+}
+// Bounded wait of a whole warp: the same answer in every lane.
+__device__ __forceinline__ bool cluster_wait(uint64_t *bar, uint32_t parity)
+{
+    bool done = false;
+    for (long long it = 0; it < kWaitLimit; ++it) {
+        uint32_t ok;
+        asm volatile(
+            "{\n\t.reg .pred p;\n\t"
+            "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
+            "selp.u32 %0, 1, 0, p;\n\t}"
+            : "=r"(ok)
+            : "r"(smem_u32(bar)), "r"(parity)
+            : "memory");
+        if (ok) {
+            done = true;
+            break;
+        }
+    }
+    return __all_sync(0xffffffffu, done);
 }
 
 __device__ __forceinline__ double warp_sum(double v)
@@ -111,7 +150,7 @@ __device__ __forceinline__ double warp_sum(double v)
 }
 
 template <typename T, int L>
-__global__ void __launch_bounds__(icg_max_threads(L), 1) icg_cluster_kernel(IcgArgs<T> a)
+__global__ void __launch_bounds__(kIcgMaxThreads, 1) icg_cluster_kernel(IcgArgs<T> a)
 {
     pdl_begin();
     extern __shared__ __align__(16) unsigned char icg_smem_raw[];
@@ -121,12 +160,24 @@ __global__ void __launch_bounds__(icg_max_threads(L), 1) icg_cluster_kernel(IcgA
     const int rank = (int)rank_u, C = (int)C_u, t = threadIdx.x, nt = blockDim.x;
     const int lane = t & 31, wid = t >> 5, nw = nt >> 5;
     const int m = a.m, n = a.n, rows = a.rows;
-    double *red1 = reinterpret_cast<double *>(icg_smem_raw);   // p.q slots [C][nw]
-    double *red2 = red1 + C * nw;                                // r.z and r.r slots [2][C][nw]
-    T *ps = reinterpret_cast<T *>(red2 + 2 * C * nw) + 1;        // p: rows -1 .. rows, m per row
+    uint64_t *bar = reinterpret_cast<uint64_t *>(icg_smem_raw);         // p.q; r.z, r.r and halo rows; CTA
+    double2 *red2 = reinterpret_cast<double2 *>(icg_smem_raw + 32);     // (r.z, r.r) slots [C][nw]
+    double *red1 = reinterpret_cast<double *>(red2 + C * nw);           // p.q slots [C][nw]
+    T *ps = reinterpret_cast<T *>(red1 + C * nw) + 1;                   // p: rows -1 .. rows, m per row
     T *hz = ps + (size_t)m * (rows + 2) + 1;                     // r / diag of the halo rows [2][m]
     T *yc = hz + 2 * m;                                          // y coefficients [rows][ky -1,0,1, my -1,0,1]
-    const int j0 = rank * rows, nr = max(0, min(rows, n - j0));  // this CTA's rows
+    const int j0 = rank * rows, nr = max(0, min(rows, n - j0));         // this CTA's rows
+    // bytes an exchange brings: every warp's partial sums, and the halo rows
+    const uint32_t tx1 = (uint32_t)(C * nw * 8), tx2 = (uint32_t)(C * nw * 16);
+    const uint32_t txh = (uint32_t)(m * sizeof(T)) * ((nr > 0 && rank > 0 ? 1u : 0u) + (nr > 0 && j0 + nr < n ? 1u : 0u));
+    if (t == 0) {
+        mbar_init(&bar[0], 1);
+        mbar_init(&bar[1], 1);
+        mbar_init(&bar[2], nw);
+        fence_mbar_init();
+        mbar_arrive_expect_tx(&bar[0], tx1);
+        mbar_arrive_expect_tx(&bar[1], tx2);
+    }
 
     // couplings of row j: none across the boundary ring
     for (int k = t; k < nr; k += nt) {
@@ -174,25 +225,49 @@ __global__ void __launch_bounds__(icg_max_threads(L), 1) icg_cluster_kernel(IcgA
     }
     if (t == 0) ps[-1] = ps[(size_t)m * (rows + 2)] = T(0);
 
-    // sum over the cluster of v (slot array red, its K-th part)
-    auto post = [&](double *red, double v) {
+    // Exchanges: every warp stores its sum into each CTA's slots, then each
+    // warp sums all slots. A slot array is written again only after its
+    // readers have taken part in the other exchange, so one copy is enough.
+    uint32_t ph1 = 0, ph2 = 0, ph3 = 0;
+    auto post1 = [&](double v) {
         v = warp_sum(v);
-        if (lane < C) cluster_store(cluster_addr(red + rank * nw + wid, lane), v);
+        if (lane < C) cluster_store(cluster_addr(red1 + rank * nw + wid, lane), v, cluster_addr(&bar[0], lane));
     };
-    auto total = [&](const double *red) -> double {
+    auto post2 = [&](double va, double vb) {
+        const double2 v = make_double2(warp_sum(va), warp_sum(vb));
+        if (lane < C) cluster_store(cluster_addr(red2 + rank * nw + wid, lane), v, cluster_addr(&bar[1], lane));
+    };
+    bool ok = true;
+    auto total1 = [&]() -> double {
+        ok = cluster_wait(&bar[0], ph1);
+        ph1 ^= 1u;
+        if (t == 0) mbar_arrive_expect_tx(&bar[0], tx1);
         double v = 0.0;
-        for (int u = lane; u < C * nw; u += 32) v += red[u];
+        for (int u = lane; u < C * nw; u += 32) v += red1[u];
         return warp_sum(v);
     };
+    auto total2 = [&](double &va, double &vb) {
+        ok = cluster_wait(&bar[1], ph2);
+        ph2 ^= 1u;
+        if (t == 0) mbar_arrive_expect_tx(&bar[1], tx2 + txh);
+        va = vb = 0.0;
+        for (int u = lane; u < C * nw; u += 32) {
+            const double2 w = red2[u];
+            va += w.x;
+            vb += w.y;
+        }
+        va = warp_sum(va);
+        vb = warp_sum(vb);
+    };
 
-    cluster_barrier();   // every CTA of the cluster runs: its slots may be written
-    post(red2, v0);
-    post(red2 + C * nw, v1);
-    cluster_barrier();
-    double rz = total(red2), rr = total(red2 + C * nw);
+    cluster_barrier();   // every CTA of the cluster has set up its mbarriers; p is in place
+    post2(v0, v1);
+    double rz, rr;
+    total2(rz, rr);
     const double tol2 = a.rtol * a.rtol * rr;
     int its = 0, brk = 0;
-    if (rr != 0.0) {
+    if (ok && rr != 0.0) {
+        double inv_rz = 1.0 / rz;
         for (;;) {
             // q = K p: p's row contracted with the x stiffness and mass, then
             // combined along y (three rows of contractions roll through)
@@ -225,10 +300,9 @@ __global__ void __launch_bounds__(icg_max_threads(L), 1) icg_cluster_kernel(IcgA
                     }
                 }
             }
-            post(red1, pq);
-            cluster_barrier();
-            pq = total(red1);
-            if (!(pq > 0.0)) {
+            post1(pq);
+            pq = total1();
+            if (!ok || !(pq > 0.0)) {
                 brk = 1;
                 break;
             }
@@ -244,19 +318,17 @@ __global__ void __launch_bounds__(icg_max_threads(L), 1) icg_cluster_kernel(IcgA
                     v0 += (double)r[l] * (double)rd;
                     v1 += (double)r[l] * (double)r[l];
                     const int k = k0 + l;
-                    if (k == 0 && rank > 0) cluster_store(cluster_addr(hz + m + i, rank - 1), rd);
-                    if (k == nr - 1 && j0 + nr < n) cluster_store(cluster_addr(hz + i, rank + 1), rd);
+                    if (k == 0 && rank > 0) cluster_store(cluster_addr(hz + m + i, rank - 1), rd, cluster_addr(&bar[1], rank - 1));
+                    if (k == nr - 1 && j0 + nr < n) cluster_store(cluster_addr(hz + i, rank + 1), rd, cluster_addr(&bar[1], rank + 1));
                 }
             }
-            post(red2, v0);
-            post(red2 + C * nw, v1);
-            cluster_barrier();
-            const double rzn = total(red2);
-            rr = total(red2 + C * nw);
-            const T be = (T)(rzn / rz);
-            rz = rzn;
+            post2(v0, v1);
+            const double inv_old = inv_rz;
+            total2(rz, rr);
+            const T be = (T)(rz * inv_old);
+            inv_rz = 1.0 / rz;   // next iteration's, off the critical path
             ++its;
-            if (rr <= tol2 || its >= a.maxit || !(rr == rr)) break;
+            if (!ok || rr <= tol2 || its >= a.maxit || !(rr == rr)) break;
 #pragma unroll
             for (int l = 0; l < L; ++l) {
                 if (l < cnt) {
@@ -271,21 +343,30 @@ __global__ void __launch_bounds__(icg_max_threads(L), 1) icg_cluster_kernel(IcgA
                     *pp = fma(be, *pp, hz[u]);
                 }
             }
-            __syncthreads();
+            // the CTA's warps meet on an mbarrier too, so that a wait that
+            // gave up in one warp cannot leave the others at a barrier
+            __syncwarp();
+            if (lane == 0)
+                asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(&bar[2])) : "memory");
+            ok = __all_sync(0xffffffffu, mbar_wait_bounded(&bar[2], ph3));
+            ph3 ^= 1u;
+            if (!ok) break;
         }
     }
-    if (!brk || a.zero_on_break) {
+    if ((!brk && ok) || a.zero_on_break) {
 #pragma unroll
         for (int l = 0; l < L; ++l)
-            if (l < cnt) a.z[(size_t)(j0 + k0 + l) * m + i] = brk ? T(0) : z[l];
+            if (l < cnt) a.z[(size_t)(j0 + k0 + l) * m + i] = brk || !ok ? T(0) : z[l];
     }
+    if (!ok) a.s->err = a.s->breakdown = 1;   // a bounded wait gave up
     if (rank == 0 && t == 0) {
         a.s->iiters = its;
         a.s->ipc += its;
-        if (brk) a.s->ibreak = a.s->breakdown = 1;
+        if (brk && ok) a.s->ibreak = a.s->breakdown = 1;
     }
-    // no CTA leaves while another may still store into its shared memory: the
-    // last stores come before the barrier every CTA has just passed
+    // no CTA leaves while another may still store into its shared memory (a
+    // CTA whose wait gave up leaves early)
+    cluster_barrier();
 }
 
 }  // namespace iga

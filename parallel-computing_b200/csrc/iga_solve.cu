@@ -1025,13 +1025,13 @@ static void (*icg_kernel(int L))(IcgArgs<T>)
                                                                                            : icg_cluster_kernel<T, 8>;
 }
 
-// The cluster shape of the inner FEM-CG for this plan's grid: the largest
-// cluster (16 CTAs needs the non-portable size) the device can place.
+// The cluster shape of the inner FEM-CG for this plan's grid: the first one
+// that fits and that the device can place.
 template <typename T>
 static int icg_prepare(PrecState<T> &ps, const iga_plan *pl)
 {
-    for (int cmax = kIcgMaxCluster; cmax >= 8; cmax /= 2) {
-        const IcgShape sh = icg_shape<T>(pl->m, pl->n, cmax);
+    for (int k = 0; k < 4; ++k) {
+        const IcgShape sh = icg_shape<T>(pl->m, pl->n, k);
         if (!sh.C) continue;
         auto kern = icg_kernel<T>(sh.L);
         if (sh.C > 8 && cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) {
@@ -1055,7 +1055,7 @@ static int icg_prepare(PrecState<T> &ps, const iga_plan *pl)
             continue;
         }
         ps.icg = sh;
-        return IGA_OK;
+        break;
     }
     return IGA_OK;
 }
@@ -1574,10 +1574,17 @@ static int pc_apply_core(PrecState<T> &ps, const iga_plan *pl, SolverState *S, c
         at[1].val.programmaticStreamSerializationAllowed = 1;
         cfg.attrs = at;
         cfg.numAttrs = pdl_capture() ? 2 : 1;
-        if (S->pc_sync) SOLVE_TRY(cudaMemsetAsync(&S->s->ibreak, 0, sizeof(int), S->stream));
+        if (S->pc_sync) {
+            SOLVE_TRY(cudaMemsetAsync(&S->s->ibreak, 0, sizeof(int), S->stream));
+            SOLVE_TRY(cudaMemsetAsync(&S->s->err, 0, sizeof(int), S->stream));
+        }
         SOLVE_TRY(cudaLaunchKernelEx(&cfg, icg_kernel<T>(ps.icg.L), a));
         if (S->pc_sync) {
             if ((st = sync_scalars(S))) return st;
+            if (S->h->err) {
+                set_error("a bounded device wait gave up in the preconditioner");
+                return IGA_ERR_TIMEOUT;
+            }
             if (S->h->ibreak) return IGA_ERR_BREAKDOWN;
         }
         return IGA_OK;
