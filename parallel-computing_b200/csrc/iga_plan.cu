@@ -13,193 +13,49 @@
 #include <vector>
 
 #include "iga_apply.cuh"
+#include "iga_column.cuh"
 #include "iga_host.hpp"
 #include "iga_plan.hpp"
 
 namespace iga {
 
 // ---------------------------------------------------------------- setup kernels
-// Precomputed geometry (the mult_sf path): G = w kappa det(J) J^-1 J^-T at
-// every quadrature point, in the order apply_kernel streams it:
-// [strip][row][qy][qx][3][column of the strip]. Padding elements get G = 0.
-// Quadrature points (padding included) of a strip grid's G.
-__host__ __device__ __forceinline__ long long geom_points(const StripGrid &g)
+// Every job of a batch's plans in one launch: CTA u runs unit u of the jobs'
+// concatenated units (geom_units), whose job a binary search over the jobs'
+// first units finds.
+__global__ void __launch_bounds__(96) geom_jobs_kernel(const GeomJob *__restrict__ jobs, int njobs)
 {
-    return (long long)g.NSX * g.NSY * g.TY * (g.P + 1) * (g.P + 1) * kSW;
-}
-
-// G at point t of grid g, into G64 and / or G32 (either may be null).
-__device__ __forceinline__ void geom_point(double *__restrict__ G64, float *__restrict__ G32,
-                                           const double *__restrict__ tabX64, const double *__restrict__ tabY64,
-                                           const double *__restrict__ CP, const double *__restrict__ qw,
-                                           const double *__restrict__ kappa, const StripGrid &g, int *err, long long t)
-{
-    const int P = g.P, NB = P + 1, NQ = P + 1, NQ2 = NQ * NQ;
-    {
-        // Point u of the step block, in the order the block is stored, so that
-        // consecutive threads write consecutive words: lane-major layouts
-        // (g_lane_major) [qy][lane = 2c + h][j] (qx = h QH + j), else
-        // [qy][qx][column]. (At p = 3 the column-fastest order scattered the
-        // lane-major writes 12 words apart: 2048^2 G64 + G32 18.4 ms.)
-        const int u = (int)(t % (NQ2 * kSW));
-        long long r = t / (NQ2 * kSW);
-        int c, qx, qy;
-        if (g_lane_major(NQ)) {
-            const int QH = NQ / 2;
-            qy = u / (32 * QH);
-            const int rem = u - qy * 32 * QH, lane = rem / QH, j = rem - lane * QH;
-            c = lane >> 1;
-            qx = (lane & 1) * QH + j;
-        } else {
-            c = u % kSW;
-            const int qp = u / kSW;
-            qx = qp % NQ;
-            qy = qp / NQ;
-        }
-        const int qp = qy * NQ + qx;
-        const int s = (int)(r % g.TY);
-        r /= g.TY;
-        const int gy = (int)(r % g.NSY);
-        const int gx = (int)(r / g.NSY);
-        const int ex = kSW * gx + c, ey = g.TY * gy + s;
-        double g00 = 0, g01 = 0, g11 = 0;
-        if (ex < g.nex && ey < g.ney) {
-            double x_xi = 0, x_eta = 0, y_xi = 0, y_eta = 0;
-            for (int jl = 0; jl < NB; ++jl) {
-                const double n2 = tabY64[((size_t)(ey * 2 + 0) * NQ + qy) * NB + jl];
-                const double d2 = tabY64[((size_t)(ey * 2 + 1) * NQ + qy) * NB + jl];
-                for (int il = 0; il < NB; ++il) {
-                    const double n1 = tabX64[((size_t)(ex * 2 + 0) * NQ + qx) * NB + il];
-                    const double d1 = tabX64[((size_t)(ex * 2 + 1) * NQ + qx) * NB + il];
-                    const size_t A = (size_t)(ey + jl) * g.m + (ex + il);
-                    const double cx = CP[2 * A], cy = CP[2 * A + 1];
-                    x_xi += cx * d1 * n2;
-                    x_eta += cx * n1 * d2;
-                    y_xi += cy * d1 * n2;
-                    y_eta += cy * n1 * d2;
-                }
-            }
-            const double det = x_xi * y_eta - x_eta * y_xi;
-            if (!(det > 0.0)) atomicExch(err, 1 /* IGA_ERR_ARG: non-positive Jacobian */);
-            double wgt = qw[qx] * qw[qy];
-            if (kappa) wgt *= kappa[((size_t)ey * g.nex + ex) * NQ2 + qp];
-            const double f = wgt / det;
-            g00 = f * (x_eta * x_eta + y_eta * y_eta);
-            g01 = -f * (x_xi * x_eta + y_xi * y_eta);
-            g11 = f * (x_xi * x_xi + y_xi * y_xi);
-        }
-        const size_t base = (((size_t)gx * g.NSY + gy) * g.TY + s) * NQ2 * 3 * kSW;
-        if (G64) {
-            double *Gs = G64 + base;
-            Gs[g_index(NQ, 8, qy, qx, 0, c)] = g00;
-            Gs[g_index(NQ, 8, qy, qx, 1, c)] = g01;
-            Gs[g_index(NQ, 8, qy, qx, 2, c)] = g11;
-        }
-        if (G32) {
-            float *Gs = G32 + base;
-            Gs[g_index(NQ, 4, qy, qx, 0, c)] = (float)g00;
-            Gs[g_index(NQ, 4, qy, qx, 1, c)] = (float)g01;
-            Gs[g_index(NQ, 4, qy, qx, 2, c)] = (float)g11;
-        }
+    __shared__ double stage[3 * 96];
+    const long long u = blockIdx.x;
+    int lo = 0, hi = njobs - 1;
+    while (lo < hi) {
+        const int mid = (lo + hi + 1) >> 1;
+        if (jobs[mid].t0 <= u) lo = mid;
+        else hi = mid - 1;
+    }
+    const GeomJob &J = jobs[lo];
+    const int k = (int)(u - J.t0), nc = column_chunks(J.g.ney, J.rows), gx = k / nc, chunk = k - gx * nc;
+    const int t = threadIdx.x;
+    if (t >= kSW * (J.g.P + 1)) return;   // whole warps where the unit's threads write through the stage
+    double *st = stage + (t >> 5) * 96;
+    switch (J.g.P) {
+    case 1: geom_unit<1>(J, gx, chunk, t, st); break;
+    case 2: geom_unit<2>(J, gx, chunk, t, st); break;
+    case 3: geom_unit<3>(J, gx, chunk, t, st); break;
+    case 4: geom_unit<4>(J, gx, chunk, t, st); break;
+    default: geom_unit<5>(J, gx, chunk, t, st); break;
     }
 }
 
-template <typename T>
-__global__ void geom_setup_kernel(T *__restrict__ G, const double *__restrict__ tabX64,
-                                  const double *__restrict__ tabY64, const double *__restrict__ CP,
-                                  const double *__restrict__ qw, const double *__restrict__ kappa, StripGrid g,
-                                  int *err)
+static void launch_geom(const GeomJob &j, cudaStream_t s)
 {
-    const long long total = geom_points(g);
-    for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < total;
-         t += (long long)gridDim.x * blockDim.x)
-        geom_point(sizeof(T) == 8 ? (double *)(void *)G : nullptr, sizeof(T) == 4 ? (float *)(void *)G : nullptr,
-                   tabX64, tabY64, CP, qw, kappa, g, err, t);
-}
-
-// Every job of a batch's plans in one launch: the CTA finds the job of the
-// first point of its 256-point block once (jobs hold at least 2 x 32 x 9 x
-// 16 points, so a block straddles at most one boundary) and each thread
-// steps to the next job if its point lies past that one's start.
-__global__ void geom_jobs_kernel(const GeomJob *__restrict__ jobs, int njobs, long long total)
-{
-    __shared__ int js;
-    for (long long b0 = (long long)blockIdx.x * blockDim.x; b0 < total; b0 += (long long)gridDim.x * blockDim.x) {
-        if (threadIdx.x == 0) {
-            int lo = 0, hi = njobs - 1;
-            while (lo < hi) {
-                const int mid = (lo + hi + 1) >> 1;
-                if (jobs[mid].t0 <= b0) lo = mid;
-                else hi = mid - 1;
-            }
-            js = lo;
-        }
-        __syncthreads();
-        const long long t = b0 + threadIdx.x;
-        int j = js;
-        __syncthreads();
-        if (t < total) {
-            if (j + 1 < njobs && t >= jobs[j + 1].t0) ++j;
-            const GeomJob &J = jobs[j];
-            geom_point(J.G64, J.G32, J.tx, J.ty, J.cp, J.qw, J.kappa, J.g, J.err, t - J.t0);
-        }
-    }
-}
-
-__device__ double load_f(int fkind, double x, double y)
-{
-    const double pi = 3.141592653589793238462643383279;
-    if (fkind == 0) return x * (1 - x) * y * (1 - y);
-    if (fkind == 1) return 2.0 * pi * pi * sin(pi * x) * sin(pi * y);
-    const double r = sqrt(x * x + y * y), th = atan2(y, x);
-    return (pi * pi * sin(pi * r) - pi * cos(pi * r) / r + 4.0 * sin(pi * r) / (r * r)) * sin(2.0 * th);
-}
-
-// Load vector F = int R f (matrix_free/src/LocalAssemblyMF.cpp:3-29), gathered
-// per control point over its supporting elements in a fixed order (the
-// atomic-free scheme of matrix_free_gpu_dbd/src/mult.cu:233-340), F[Dir] = 0.
-__global__ void rhs_kernel(double *__restrict__ F, const double *__restrict__ tabX64,
-                           const double *__restrict__ tabY64, const double *__restrict__ CP,
-                           const double *__restrict__ qw, int fkind, StripGrid g)
-{
-    const int P = g.P, NB = P + 1, NQ = P + 1;
-    const long long N = (long long)g.m * g.n;
-    for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < N; t += (long long)gridDim.x * blockDim.x) {
-        const int C = (int)(t % g.m), R = (int)(t / g.m);
-        if (R == 0 || C == 0 || R == g.n - 1 || C == g.m - 1) {
-            F[t] = 0.0;
-            continue;
-        }
-        double v = 0.0;
-        for (int ey = max(0, R - P); ey <= min(R, g.ney - 1); ++ey)
-            for (int ex = max(0, C - P); ex <= min(C, g.nex - 1); ++ex) {
-                const int il0 = C - ex, jl0 = R - ey;
-                for (int qy = 0; qy < NQ; ++qy)
-                    for (int qx = 0; qx < NQ; ++qx) {
-                        double xq = 0, yq = 0, x_xi = 0, x_eta = 0, y_xi = 0, y_eta = 0;
-                        for (int jl = 0; jl < NB; ++jl) {
-                            const double n2 = tabY64[((size_t)(ey * 2 + 0) * NQ + qy) * NB + jl];
-                            const double d2 = tabY64[((size_t)(ey * 2 + 1) * NQ + qy) * NB + jl];
-                            for (int il = 0; il < NB; ++il) {
-                                const double n1 = tabX64[((size_t)(ex * 2 + 0) * NQ + qx) * NB + il];
-                                const double d1 = tabX64[((size_t)(ex * 2 + 1) * NQ + qx) * NB + il];
-                                const size_t A = (size_t)(ey + jl) * g.m + (ex + il);
-                                const double cx = CP[2 * A], cy = CP[2 * A + 1];
-                                xq += cx * n1 * n2;
-                                yq += cy * n1 * n2;
-                                x_xi += cx * d1 * n2;
-                                x_eta += cx * n1 * d2;
-                                y_xi += cy * d1 * n2;
-                                y_eta += cy * n1 * d2;
-                            }
-                        }
-                        const double det = x_xi * y_eta - x_eta * y_xi;
-                        const double Ra = tabX64[((size_t)(ex * 2) * NQ + qx) * NB + il0] *
-                                          tabY64[((size_t)(ey * 2) * NQ + qy) * NB + jl0];
-                        v += Ra * load_f(fkind, xq, yq) * qw[qx] * qw[qy] * det;
-                    }
-            }
-        F[t] = v;
+    const unsigned grid = (unsigned)geom_units(j);   // at most a sixteenth of the elements: one dimension holds it
+    switch (j.g.P) {
+    case 1: geom_kernel<1><<<grid, kSW * 2, 0, s>>>(j); break;
+    case 2: geom_kernel<2><<<grid, kSW * 3, 0, s>>>(j); break;
+    case 3: geom_kernel<3><<<grid, kSW * 4, 0, s>>>(j); break;
+    case 4: geom_kernel<4><<<grid, kSW * 5, 0, s>>>(j); break;
+    default: geom_kernel<5><<<grid, kSW * 6, 0, s>>>(j); break;
     }
 }
 
@@ -443,24 +299,9 @@ void PlanArena::stage(void *dst, const void *src, size_t bytes)
     if (c->sealed && c->staged == c->used) cv.notify_all();
 }
 
-static bool same_grid(const StripGrid &a, const StripGrid &b)
-{
-    return a.m == b.m && a.n == b.n && a.nex == b.nex && a.ney == b.ney && a.TY == b.TY && a.NSX == b.NSX &&
-           a.NSY == b.NSY && a.P == b.P;
-}
-
 void PlanArena::defer_geom(const GeomJob &j)
 {
     std::lock_guard<std::mutex> lock(mu);
-    for (size_t k = geom.size(); k-- > 0;) {   // the plan's other precision, added just before by the same thread
-        GeomJob &o = geom[k];
-        if (o.cp == j.cp && o.tx == j.tx && o.kappa == j.kappa && same_grid(o.g, j.g) && !(o.G64 && j.G64) &&
-            !(o.G32 && j.G32)) {
-            if (j.G64) o.G64 = j.G64;
-            if (j.G32) o.G32 = j.G32;
-            return;
-        }
-    }
     geom.push_back(j);
 }
 
@@ -494,18 +335,13 @@ cudaError_t PlanArena::flush()
         long long t = 0;
         for (GeomJob &j : geom) {
             j.t0 = t;
-            t += geom_points(j.g);
+            t += geom_units(j);
         }
         GeomJob *dj = nullptr;
         cudaError_t e = alloc((void **)&dj, geom.size() * sizeof(GeomJob));
         if (e == cudaSuccess) e = cudaMemcpy(dj, geom.data(), geom.size() * sizeof(GeomJob), cudaMemcpyHostToDevice);
         if (e != cudaSuccess) return e;
-        int nsm = 148, dev = 0;
-        if (cudaGetDevice(&dev) != cudaSuccess ||
-            cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
-            nsm = 148;
-        const long long blocks = std::min<long long>((t + 255) / 256, 8LL * nsm);
-        geom_jobs_kernel<<<(unsigned)blocks, 256>>>(dj, (int)geom.size(), t);
+        geom_jobs_kernel<<<(unsigned)t, 96>>>(dj, (int)geom.size());
         geom.clear();
     }
     return cudaGetLastError();
@@ -737,32 +573,37 @@ static int build_operator(iga_plan *pl, OperatorData &op, const Patch &P, const 
         const size_t gelems = (size_t)g.NSX * g.NSY * g.TY * NQ2 * 3 * kSW;
         op.geom_bytes = gelems * sizeof(T);
         if ((st = upload((T **)&op.G, nullptr, op.geom_bytes))) return st;
-        if (pl->arena && pl->arena->defer) {   // after the arena's flush has sent the tables
-            GeomJob j;
-            if (sizeof(T) == 8) j.G64 = (double *)op.G;
-            else j.G32 = (float *)op.G;
-            j.tx = pl->tabX64;
-            j.ty = pl->tabY64;
-            j.cp = pl->CP;
-            j.qw = pl->qw;
-            j.kappa = pl->kappa_dev;
-            j.g = g;
-            j.err = pl->d_err;
-            pl->arena->defer_geom(j);
-            op.ready = true;
-            return IGA_OK;
-        }
-        geom_setup_kernel<T><<<1184, 256>>>((T *)op.G, pl->tabX64, pl->tabY64, pl->CP, pl->qw, pl->kappa_dev, g,
-                                            pl->d_err);
-        // in an arena (a batch's set-up) the caller synchronises once for all plans
-        cudaError_t e = pl->arena ? cudaPeekAtLastError() : cudaDeviceSynchronize();
-        if (e != cudaSuccess) {
-            set_error(std::string("geometry setup: ") + cudaGetErrorString(e));
-            return IGA_ERR_CUDA;
-        }
     }
     op.ready = true;
     return IGA_OK;
+}
+
+// The precomputed geometry of every operator of the plan, from kappa (null:
+// 1); kappa_out: a copy of it, written in the same pass.
+static GeomJob geom_job(const iga_plan *pl, const double *kappa, double *kappa_out)
+{
+    GeomJob j;
+    j.tx = pl->tabX64;
+    j.ty = pl->tabY64;
+    j.cp = pl->CP;
+    j.qw = pl->qw;
+    j.kappa = kappa;
+    j.kappa_out = kappa_out;
+    j.err = pl->d_err;
+    j.g = pl->grid;
+    // a batch's plans run together: every unit count is enough there
+    j.rows = pl->arena ? 8 : column_rows(pl->grid.NSX, pl->ney, pl->nsm);
+    if (pl->op64.ready) {
+        j.G64 = (double *)pl->op64.G;
+        j.TY64 = pl->op64.grid.TY;
+        j.NSY64 = pl->op64.grid.NSY;
+    }
+    if (pl->op32.ready) {
+        j.G32 = (float *)pl->op32.G;
+        j.TY32 = pl->op32.grid.TY;
+        j.NSY32 = pl->op32.grid.NSY;
+    }
+    return j;
 }
 
 // Win: a window of strip rows (gyn >= 0: strip rows gy0 .. gy0 + gyn - 1, and
@@ -1093,6 +934,20 @@ int iga_plan_create(const iga_mesh_desc *d, const iga_opts *opts_in, iga_plan **
         pl->op32.warps = warps_for(P.p, IGA_FP32, opts.geometry);
         if ((st = build_operator<float>(pl, pl->op32, P, tx, ty))) return fail(st);
     }
+    if (pl->geometry == IGA_GEOM_PRECOMPUTED) {
+        const GeomJob j = geom_job(pl, pl->kappa_dev, nullptr);
+        if (pl->arena && pl->arena->defer) {
+            pl->arena->defer_geom(j);   // after the arena's flush has sent the tables
+        } else {
+            launch_geom(j, 0);
+            // in an arena (a batch's set-up) the caller synchronises once for all plans
+            const cudaError_t e = pl->arena ? cudaPeekAtLastError() : cudaDeviceSynchronize();
+            if (e != cudaSuccess) {
+                set_error(std::string("geometry setup: ") + cudaGetErrorString(e));
+                return fail(IGA_ERR_CUDA);
+            }
+        }
+    }
     int herr = 0;
     if (!pl->arena) cudaMemcpy(&herr, pl->d_err, sizeof(int), cudaMemcpyDeviceToHost);
     if (herr) {
@@ -1155,20 +1010,15 @@ int iga_plan_set_kappa(iga_plan *pl, const double *kappa, void *stream)
     cudaStream_t s = (cudaStream_t)stream;
     const long long nq = (long long)pl->nex * pl->ney * (pl->p + 1) * (pl->p + 1);
     if (!pl->kappa_dev) IGA_CUDA_TRY(cudaMalloc((void **)&pl->kappa_dev, nq * sizeof(double)));
-    IGA_CUDA_TRY(cudaMemcpyAsync(pl->kappa_dev, kappa, nq * sizeof(double), cudaMemcpyDeviceToDevice, s));
     ++pl->kappa_version;
-    OperatorData *ops[2] = {&pl->op64, &pl->op32};
-    for (int k = 0; k < 2; ++k) {
-        OperatorData &op = *ops[k];
-        if (!op.ready) continue;
-        if (pl->geometry == IGA_GEOM_PRECOMPUTED) {
-            if (k == 0)
-                geom_setup_kernel<double><<<1184, 256, 0, s>>>((double *)op.G, pl->tabX64, pl->tabY64, pl->CP, pl->qw,
-                                                              pl->kappa_dev, op.grid, pl->d_err);
-            else
-                geom_setup_kernel<float><<<1184, 256, 0, s>>>((float *)op.G, pl->tabX64, pl->tabY64, pl->CP, pl->qw,
-                                                             pl->kappa_dev, op.grid, pl->d_err);
-        } else {
+    if (pl->geometry == IGA_GEOM_PRECOMPUTED) {   // the pass over the points also takes the copy
+        launch_geom(geom_job(pl, kappa, kappa == pl->kappa_dev ? nullptr : pl->kappa_dev), s);
+    } else {
+        IGA_CUDA_TRY(cudaMemcpyAsync(pl->kappa_dev, kappa, nq * sizeof(double), cudaMemcpyDeviceToDevice, s));
+        OperatorData *ops[2] = {&pl->op64, &pl->op32};
+        for (int k = 0; k < 2; ++k) {
+            OperatorData &op = *ops[k];
+            if (!op.ready) continue;
             const size_t es = k == 0 ? sizeof(double) : sizeof(float);
             if (!op.kappa) IGA_CUDA_TRY(cudaMalloc(&op.kappa, nq * es));
             if (k == 0) kappa_convert_kernel<double><<<296, 256, 0, s>>>((double *)op.kappa, pl->kappa_dev, nq);
@@ -1291,8 +1141,21 @@ int iga_apply_host(iga_plan *pl, const double *xh, double *yh)
 int iga_rhs(iga_plan *pl, int fkind, double *F, void *stream)
 {
     if (!pl || !F || fkind < 0 || fkind > 2) return IGA_ERR_ARG;
-    rhs_kernel<<<2 * 148, 256, 0, (cudaStream_t)stream>>>(F, pl->tabX64, pl->tabY64, pl->CP, pl->qw, fkind,
-                                                         pl->grid);
+    // control-point rows per CTA: as few as one wave of CTAs allows (each
+    // evaluates its halo of P element rows again)
+    const StripGrid &g = pl->grid;
+    const int cols = (g.m + kRhsCols - 1) / kRhsCols;
+    const int want = std::max(1, rhs_ctas(pl->p) * pl->nsm / cols);   // CTAs along y
+    const int rows = std::max(2, (g.n + want - 1) / want);
+    const unsigned grid = (unsigned)((long long)cols * ((g.n + rows - 1) / rows));
+    const cudaStream_t s = (cudaStream_t)stream;
+    switch (pl->p) {
+    case 1: rhs_kernel<1><<<grid, rhs_threads(1), 0, s>>>(F, pl->tabX64, pl->tabY64, pl->CP, pl->qw, fkind, g, rows); break;
+    case 2: rhs_kernel<2><<<grid, rhs_threads(2), 0, s>>>(F, pl->tabX64, pl->tabY64, pl->CP, pl->qw, fkind, g, rows); break;
+    case 3: rhs_kernel<3><<<grid, rhs_threads(3), 0, s>>>(F, pl->tabX64, pl->tabY64, pl->CP, pl->qw, fkind, g, rows); break;
+    case 4: rhs_kernel<4><<<grid, rhs_threads(4), 0, s>>>(F, pl->tabX64, pl->tabY64, pl->CP, pl->qw, fkind, g, rows); break;
+    default: rhs_kernel<5><<<grid, rhs_threads(5), 0, s>>>(F, pl->tabX64, pl->tabY64, pl->CP, pl->qw, fkind, g, rows); break;
+    }
     IGA_CUDA_TRY(cudaGetLastError());
     return IGA_OK;
 }

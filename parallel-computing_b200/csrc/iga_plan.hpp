@@ -34,13 +34,17 @@ struct OperatorData {
 
 struct SolverState;   // defined by the solver translation unit
 
-// One plan's precomputed-geometry set-up inside a batch's single launch:
-// G in FP64 and / or FP32 (null: not wanted) on strip grid g from the plan's
-// FP64 tables and control points; t0 = the job's first point in the launch.
+// One plan's precomputed geometry (iga_column.cuh): G in FP64 and / or FP32
+// (null: not wanted), each on its own strips (TY rows each, NSY of them; g
+// gives the patch), from the plan's FP64 tables and control points; kappa_out:
+// where to copy kappa (or null); t0 = the job's first unit in a batch's launch.
 struct GeomJob {
     double *G64 = nullptr;
     float *G32 = nullptr;
+    int TY64 = 1, NSY64 = 0, TY32 = 1, NSY32 = 0;
+    int rows = 8;   // element rows per unit
     const double *tx = nullptr, *ty = nullptr, *cp = nullptr, *qw = nullptr, *kappa = nullptr;
+    double *kappa_out = nullptr;
     StripGrid g;
     int *err = nullptr;
     long long t0 = 0;
@@ -101,8 +105,7 @@ struct PlanArena {
     void copy_loop(int device);
     void stop_copier();
     ~PlanArena() { stop_copier(); }
-    // deferred geometry set-up: one job per plan (a MIXED plan's two
-    // precisions on the same strips share one), all run by one launch in flush()
+    // deferred geometry set-up: one job per plan, all run by one launch in flush()
     std::vector<GeomJob> geom;
     cudaError_t alloc_data(void **p, size_t bytes);
     void stage(void *dst, const void *src, size_t bytes);
@@ -172,6 +175,4 @@ int iga_apply_internal(iga_plan *pl, int prec, const void *x, void *y, cudaStrea
 // Operator with explicit sign / boundary rule (the solver applies +K with identity rows).
 int iga_apply_internal_sb(iga_plan *pl, int prec, const void *x, void *y, cudaStream_t s, int sign, int bc);
 int iga_check_error_flag(iga_plan *pl);
-// Computes G of one operator precision from the plan's tables and kappa (device).
-int iga_rebuild_geometry(iga_plan *pl, cudaStream_t s);
 void iga_solver_release(iga_plan *pl);

@@ -851,25 +851,46 @@ __global__ void boundary_copy_kernel(T *__restrict__ z, const T *__restrict__ r,
 // s_i = 1 / sqrt(mean of kappa over the quadrature points of the elements
 // supporting control point i); the preconditioner becomes S M^-1 S, which
 // keeps the FEM matrix's shape and adds the coefficient's local magnitude.
-__global__ void kappa_scale_kernel(const double *__restrict__ kappa, double *__restrict__ s64, float *__restrict__ s32,
-                                   StripGrid g)
+// A CTA sums kappa over each element of its tile's supports once (kKsX x kKsY
+// control points and a halo of P elements; one thread per element and
+// quadrature row, then the rows) and the control points sum those. Bound: the
+// bytes of kappa (p=3 512^2: 17 us; every control point summing all points of
+// its elements: 262 us).
+constexpr int kKsX = 32, kKsY = 8;
+
+__global__ void __launch_bounds__(kKsX *kKsY) kappa_scale_kernel(const double *__restrict__ kappa, double *__restrict__ s64,
+                                                                 float *__restrict__ s32, StripGrid g)
 {
-    const int P = g.P, NQ2 = (P + 1) * (P + 1);
-    const long long N = (long long)g.m * g.n;
-    for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < N; t += (long long)gridDim.x * blockDim.x) {
-        const int C = (int)(t % g.m), R = (int)(t / g.m);
-        double sum = 0.0;
-        int cnt = 0;
-        for (int ey = max(0, R - P); ey <= min(R, g.ney - 1); ++ey)
-            for (int ex = max(0, C - P); ex <= min(C, g.nex - 1); ++ex) {
-                const double *k = kappa + ((size_t)ey * g.nex + ex) * NQ2;
-                for (int q = 0; q < NQ2; ++q) sum += k[q];
-                cnt += NQ2;
-            }
-        const double v = (cnt > 0 && sum > 0.0) ? 1.0 / sqrt(sum / cnt) : 1.0;
-        s64[t] = v;
-        s32[t] = (float)v;
+    __shared__ double part[(kKsX + 5) * (kKsY + 5) * 6];
+    __shared__ double sum[(kKsX + 5) * (kKsY + 5)];
+    const int P = g.P, NQ = P + 1, EX = kKsX + P, EY = kKsY + P;
+    const int cols = (g.m + kKsX - 1) / kKsX, by = blockIdx.x / cols;
+    const int C0 = kKsX * (blockIdx.x - by * cols), R0 = kKsY * by;
+    for (int u = threadIdx.x; u < EX * EY * NQ; u += blockDim.x) {
+        const int qy = u % NQ, k = u / NQ, ex = C0 - P + k % EX, ey = R0 - P + k / EX;
+        double v = 0.0;
+        if (ex >= 0 && ex < g.nex && ey >= 0 && ey < g.ney) {
+            const double *q = kappa + (((size_t)ey * g.nex + ex) * NQ + qy) * NQ;
+            for (int a = 0; a < NQ; ++a) v += q[a];
+        }
+        part[u] = v;
     }
+    __syncthreads();
+    for (int k = threadIdx.x; k < EX * EY; k += blockDim.x) {
+        double v = 0.0;
+        for (int a = 0; a < NQ; ++a) v += part[k * NQ + a];
+        sum[k] = v;
+    }
+    __syncthreads();
+    const int cl = threadIdx.x % kKsX, rl = threadIdx.x / kKsX, C = C0 + cl, R = R0 + rl;
+    if (C >= g.m || R >= g.n) return;
+    double v = 0.0;
+    for (int b = 0; b <= P; ++b)
+        for (int a = 0; a <= P; ++a) v += sum[(rl + b) * EX + cl + a];
+    const int nx = min(C, g.nex - 1) - max(0, C - P) + 1, ny = min(R, g.ney - 1) - max(0, R - P) + 1;
+    v = v > 0.0 ? 1.0 / sqrt(v / ((double)nx * ny * NQ * NQ)) : 1.0;
+    s64[(size_t)R * g.m + C] = v;
+    s32[(size_t)R * g.m + C] = (float)v;
 }
 
 template <typename T>
@@ -1475,7 +1496,9 @@ static int update_kscale(const iga_plan *pl, SolverState *S)
         SOLVE_TRY(cudaMalloc((void **)&S->ks64, sizeof(double) * pl->nfunc));
         SOLVE_TRY(cudaMalloc((void **)&S->ks32, sizeof(float) * pl->nfunc));
     }
-    kappa_scale_kernel<<<kRedBlocks, kThreads, 0, S->stream>>>(pl->kappa_dev, S->ks64, S->ks32, pl->grid);
+    const StripGrid &g = pl->grid;
+    const long long tiles = (long long)((g.m + kKsX - 1) / kKsX) * ((g.n + kKsY - 1) / kKsY);
+    kappa_scale_kernel<<<(unsigned)tiles, kKsX * kKsY, 0, S->stream>>>(pl->kappa_dev, S->ks64, S->ks32, g);
     S->kappa_version = pl->kappa_version;
     SOLVE_TRY(cudaGetLastError());
     return IGA_OK;

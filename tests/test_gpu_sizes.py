@@ -93,3 +93,36 @@ def test_fem_cg_breakdown_and_zero(torch_cuda, ib):
     plan.pc_apply(r, z, pc=ib.PC_FEM_CG)
     assert float(z.abs().max()) == 0.0
     plan.close()
+
+
+# Quadrature-point fields: one element, fewer columns or rows than a strip or
+# a chunk, remainders of 16 columns, 8 rows, 32 x 8 and 32-column tiles, every
+# degree (its own kernel and G layout), both precisions' G on strips of
+# their own heights.
+FIELD_SHAPES = [(1, 1, 1), (1, 33, 40), (2, 16, 8), (2, 50, 37), (3, 15, 9), (3, 64, 65), (4, 17, 31), (4, 70, 20),
+                (5, 33, 18), (5, 7, 90)]
+
+
+@pytest.mark.parametrize("p,nex,ney", FIELD_SHAPES)
+def test_set_kappa_adjoint_gradient_and_load(torch_cuda, ib, orc, p, nex, ney):
+    M = distorted(ib.unit_square(p, nex, ney))
+    plan = ib.Plan(M, precision=ib.MIXED)
+    n = plan.nfunc
+    kq = np.exp(splitmix_uniform(5, -1.0, 1.0, nex * ney * (p + 1) ** 2))
+    x = splitmix_uniform(6, -1.0, 1.0, n)
+    lam = splitmix_uniform(7, -1.0, 1.0, n)
+    plan.set_kappa(torch_cuda.from_numpy(kq).cuda())
+    ref = orc.apply_mf(dict(M, kappa=kq), x)
+    for prec, dt, tol in ((ib.FP64, torch_cuda.float64, 1e-12), (ib.FP32, torch_cuda.float32, 2e-5)):
+        xd = torch_cuda.from_numpy(x).to("cuda", dt)
+        yd = torch_cuda.full_like(xd, float("nan"))
+        plan.apply(xd, yd, precision=prec)
+        assert rel(yd.double().cpu().numpy(), ref) < tol
+    g = torch_cuda.full((kq.size,), float("nan"), dtype=torch_cuda.float64, device="cuda")
+    plan.adjoint_grad(torch_cuda.from_numpy(x).cuda(), torch_cuda.from_numpy(lam).cuda(), g)
+    assert rel(g.cpu().numpy(), orc.adjoint_grad(M, x, lam)) < 1e-12
+    F = torch_cuda.full((n,), float("nan"), dtype=torch_cuda.float64, device="cuda")
+    for kind in (ib.F_REFERENCE, ib.F_SINSIN):
+        plan.rhs(F, kind)
+        assert np.abs(F.cpu().numpy() - orc.rhs(M, kind)).max() <= 1e-12 * max(np.abs(orc.rhs(M, kind)).max(), 1e-300)
+    plan.close()
