@@ -209,10 +209,9 @@ int launch(int dev, int nsm, unsigned char *base, const Layout &Ly, int TY, int 
                block(32, W);
     kern<<<grid, block, apply_smem_bytes<P, double, 1, 2>(W, !percol && g.NSY % W ? 2 : 1), s>>>(a);
     cudaError_t e = cudaPeekAtLastError();
-    const long long nseam = (long long)(g.NSX - 1) * P * g.n + (long long)(g.NSY - 1) * P * g.m;
-    if (e == cudaSuccess && nseam > 0) {
-        seam_fixup_kernel<P, double><<<(int)std::min<long long>((nseam + 255) / 256, 592), 256, 0, s>>>(
-            a.frame, d_in, d_out, g, -1.0, a.bc, d_ID);
+    const int blocks = seam_range(g).total;
+    if (e == cudaSuccess && blocks > 0) {
+        seam_fixup_kernel<P, double><<<blocks, kSeamBlock, 0, s>>>(a.frame, d_in, d_out, g, -1.0, a.bc, 0, g.n, d_ID);
         e = cudaPeekAtLastError();
     }
     if (e != cudaSuccess) {

@@ -661,23 +661,23 @@ static int launch_apply_t(iga_plan *pl, const OperatorData &op, const T *x, T *y
     const long long nstrips = (long long)g.NSX * rows;
     const dim3 grid = percol ? dim3(g.NSX, (rows + W - 1) / W) : dim3((unsigned)((nstrips + W - 1) / W));
     dim3 block(32, W);
-    if (rows > 0) IGA_CUDA_TRY(launch_k(kern, grid, block, smem, s, a));
-    if (win.gyn < 0) {
-        const long long nseam = (long long)(g.NSX - 1) * P * g.n + (long long)(g.NSY - 1) * P * g.m;
-        if (nseam > 0) {
-            // about one seam point per thread, so that the points' frame loads
-            // (L2 hits) are all in flight at once (p=3 2048^2 FP64 MatMult:
-            // 309.5 us with 7 points per thread, 306 us with one)
-            const int blocks = (int)std::min<long long>((nseam + 255) / 256, 32 * 148);
-            IGA_CUDA_TRY(launch_k(seam_fixup_kernel<P, T>, dim3(blocks), dim3(256), 0, s, (const T *)op.frame, x, y,
-                                  g, (T)sign, bc, win.ID));
-        }
-    } else if (win.R1 > win.R0) {
-        const long long nseam = (long long)(g.NSX - 1) * P * (win.R1 - win.R0) + (long long)2 * P * g.m * (rows + 1);
-        const int blocks = (int)std::max<long long>(1, std::min<long long>((nseam + 255) / 256, 4 * 148));
-        seam_fixup_rows_kernel<P, T><<<blocks, 256, 0, s>>>((const T *)op.frame, x, y, g, (T)sign, bc, win.R0,
-                                                             win.R1, win.ID);
+    if (rows > 0) {
+        // In the solver's loop: a programmatic dependent of the direction
+        // update only while its CTAs fit one wave. Past that its first CTAs
+        // start one by one as that kernel's blocks leave the SMs, and the
+        // later waves stay as ragged (mixed solve 2048^2 p=3: 355 us an
+        // iteration, 339 with an ordinary edge; 64^2: 42.6 against 44.3).
+        const bool pdl = pdl_capture();
+        if ((long long)grid.x * grid.y > pl->nsm) pdl_capture() = false;
+        const cudaError_t e = launch_k(kern, grid, block, smem, s, a);
+        pdl_capture() = pdl;
+        IGA_CUDA_TRY(e);
     }
+    const int R0 = win.gyn < 0 ? 0 : win.R0, R1 = win.gyn < 0 ? g.n : win.R1;
+    const int blocks = R1 > R0 ? seam_range(g, R0, R1).total : 0;
+    if (blocks > 0)
+        IGA_CUDA_TRY(launch_after(seam_fixup_kernel<P, T>, dim3(blocks), dim3(kSeamBlock), s, (const T *)op.frame, x, y,
+                                  g, (T)sign, bc, R0, R1, win.ID));
     IGA_CUDA_TRY(cudaGetLastError());
     return IGA_OK;
 }

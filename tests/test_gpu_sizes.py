@@ -126,3 +126,37 @@ def test_set_kappa_adjoint_gradient_and_load(torch_cuda, ib, orc, p, nex, ney):
         plan.rhs(F, kind)
         assert np.abs(F.cpu().numpy() - orc.rhs(M, kind)).max() <= 1e-12 * max(np.abs(orc.rhs(M, kind)).max(), 1e-300)
     plan.close()
+
+
+# Seams: a strip height that leaves one row (or fewer than P) in the last
+# strip row, one strip row or column only, more than one block of points per
+# seam in either direction.
+@pytest.mark.parametrize("p,nex,ney,ty", [(3, 33, 9, 4), (3, 17, 5, 4), (2, 16, 30, 7), (4, 40, 4, 5), (5, 49, 11, 5),
+                                          (1, 600, 3, 2), (3, 32, 200, 199), (2, 130, 300, 16)])
+@pytest.mark.parametrize("bc", [0, 1, 2])
+def test_seams(torch_cuda, ib, orc, p, nex, ney, ty, bc):
+    M = distorted(ib.unit_square(p, nex, ney))
+    plan = ib.Plan(M, bc=bc, sign=1, rows_per_strip=ty)
+    x = splitmix_uniform(p + nex, -1.0, 1.0, plan.nfunc)
+    xd = torch_cuda.from_numpy(x).cuda()
+    yd = torch_cuda.full_like(xd, float("nan"))
+    plan.apply(xd, yd)
+    ref = orc.apply_mf(M, x, sign=1.0, bc=0 if bc == 2 else bc)
+    y, m, n = yd.cpu().numpy(), nex + p, ney + p
+    if bc == 2:   # full sums on the ring too: compare the interior, the ring with tall strips
+        one = ib.Plan(M, bc=bc, sign=1, rows_per_strip=max(ney, p))
+        y2 = torch_cuda.full_like(xd, float("nan"))
+        one.apply(xd, y2)
+        assert rel(y, y2.cpu().numpy()) < 1e-12
+        inner = np.s_[1:-1, 1:-1]
+        y, ref = y.reshape(n, m)[inner], ref.reshape(n, m)[inner]
+    assert rel(y, ref) < 1e-12
+    # a caller's own capture, replayed
+    g = torch_cuda.cuda.CUDAGraph()
+    s = torch_cuda.cuda.Stream()
+    y3 = torch_cuda.full_like(xd, float("nan"))
+    with torch_cuda.cuda.graph(g, stream=s):
+        plan.apply(xd, y3, stream=s)
+    g.replay()
+    torch_cuda.cuda.synchronize()
+    assert torch_cuda.equal(y3, yd)
