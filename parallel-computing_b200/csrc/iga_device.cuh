@@ -61,12 +61,34 @@ inline cudaError_t launch_k(void (*kern)(KArgs...), dim3 grid, dim3 block, size_
     return cudaLaunchKernelEx(&cfg, kern, std::forward<Args>(args)...);
 }
 
+// launch_k() with an ordinary edge for grids of more CTAs than SMs: as
+// programmatic dependents their CTAs start where the preceding grid's leave
+// first, and those SMs fill up while others stay empty (FP64 preconditioner
+// p=3 1024^2, GEMMs of 289 CTAs, up to three an SM: 173 us against 108; FP64
+// PCG 296 -> 233 us an iteration). Kernels bound by latency or bandwidth lose
+// less than the launch gap is worth (TF32 GEMMs at 1024^2: 37.6 us as
+// dependents, 42.2 with ordinary edges).
+template <typename... KArgs, typename... Args>
+inline cudaError_t launch_even(void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t s,
+                               Args &&...args)
+{
+    const bool was = pdl_capture();
+    int nsm = 148, dev = 0;
+    if (was && (cudaGetDevice(&dev) != cudaSuccess ||
+                cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess))
+        nsm = 148;
+    if ((long long)grid.x * grid.y * grid.z > nsm) pdl_capture() = false;
+    const cudaError_t e = launch_k(kern, grid, block, smem, s, std::forward<Args>(args)...);
+    pdl_capture() = was;
+    return e;
+}
+
 // Launches a kernel that follows this call's own preceding kernel on s and
 // begins with pdl_begin(): as a programmatic dependent, so that its CTAs are
 // set up while that one drains (with the seams' own change: MatMult p=2 64^2
 // 10.2 -> 8.2 us, p=3 1024^2 86.6 -> 83.7 us, 2048^2 297.5 -> 292.3 us, where the
-// ordinary edge gives 295.1). Outside the solver's capture only on streams that are not being captured: a caller's
-// graph keeps ordinary edges.
+// ordinary edge gives 295.1). Outside the solver's capture only on streams
+// that are not being captured: a caller's graph keeps ordinary edges.
 template <typename... KArgs, typename... Args>
 inline cudaError_t launch_after(void (*kern)(KArgs...), dim3 grid, dim3 block, cudaStream_t s, Args &&...args)
 {

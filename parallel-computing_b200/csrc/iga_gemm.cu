@@ -593,7 +593,7 @@ int launch_f64(GemmOperand A, GemmOperand B, double *C, int ldc, int M, int N, i
         attr = true;
     }
     const dim3 grid(tiles_along(Mst, TM, split.on_n ? 0 : split.kb), tiles_along(Nst, TN, split.on_n ? split.kb : 0));
-    return launch_k(gemm_f64_kernel<CFG, AMN, BMN, SCATTER>, grid, dim3(NT), smem, s,
+    return launch_even(gemm_f64_kernel<CFG, AMN, BMN, SCATTER>, grid, dim3(NT), smem, s,
                     static_cast<const double *>(A.ptr), A.ld, static_cast<const double *>(B.ptr), B.ld, C, ldc, M, N, K,
                     Mst, Nst, sc, split) == cudaSuccess
                ? IGA_OK

@@ -661,18 +661,10 @@ static int launch_apply_t(iga_plan *pl, const OperatorData &op, const T *x, T *y
     const long long nstrips = (long long)g.NSX * rows;
     const dim3 grid = percol ? dim3(g.NSX, (rows + W - 1) / W) : dim3((unsigned)((nstrips + W - 1) / W));
     dim3 block(32, W);
-    if (rows > 0) {
-        // In the solver's loop: a programmatic dependent of the direction
-        // update only while its CTAs fit one wave. Past that its first CTAs
-        // start one by one as that kernel's blocks leave the SMs, and the
-        // later waves stay as ragged (mixed solve 2048^2 p=3: 355 us an
-        // iteration, 339 with an ordinary edge; 64^2: 42.6 against 44.3).
-        const bool pdl = pdl_capture();
-        if ((long long)grid.x * grid.y > pl->nsm) pdl_capture() = false;
-        const cudaError_t e = launch_k(kern, grid, block, smem, s, a);
-        pdl_capture() = pdl;
-        IGA_CUDA_TRY(e);
-    }
+    // In the solver's loop: a programmatic dependent of the direction update
+    // only while its CTAs fit one wave (mixed solve 2048^2 p=3: 355 us an
+    // iteration, 339 with an ordinary edge; 64^2: 42.6 against 44.3).
+    if (rows > 0) IGA_CUDA_TRY(launch_even(kern, grid, block, smem, s, a));
     const int R0 = win.gyn < 0 ? 0 : win.R0, R1 = win.gyn < 0 ? g.n : win.R1;
     const int blocks = R1 > R0 ? seam_range(g, R0, R1).total : 0;
     if (blocks > 0)

@@ -38,6 +38,7 @@ struct DevScalars {
     int err;                                        // a bounded wait in a kernel gave up
     int it, maxit;                                  // outer PCG in a device-side loop
     long long ipc;                                  // inner iterations of one call's cluster FEM-CG solves
+    double rzv[2];                                  // r.z of the device-side loop's even / odd iterations
 };
 
 }  // namespace iga
@@ -96,6 +97,48 @@ __device__ bool reduce_last(double (&v)[K], double *partials, unsigned *counter,
         *counter = 0u;
     }
     return true;
+}
+
+// Blocks of a loop kernel over N entries: 16 bytes a thread, at most
+// kRedBlocks (a 64^2 patch's 592 mostly empty blocks cost 0.5 us a launch and
+// 0.9 us a reduction more than its 9).
+template <typename T>
+static int vec_blocks(long long N)
+{
+    const long long per = (long long)kThreads * (16 / (long long)sizeof(T));
+    return (int)std::max(1LL, std::min<long long>(kRedBlocks, (N + per - 1) / per));
+}
+
+// One partial sum per block, v summed over the block in a fixed order.
+__device__ __forceinline__ void put_partial(double v, double *part)
+{
+    __shared__ double sh[kThreads / 32];
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
+    if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = v;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        double s = 0.0;
+        for (int w = 0; w < kThreads / 32; ++w) s += sh[w];
+        part[blockIdx.x] = s;
+    }
+}
+
+// The sum of an earlier kernel's np block partials, in every thread of every
+// block, in the same order. The kernel that needs a dot product sums its
+// partials itself instead of the producer's last block (whose fence, counter
+// and second pass are serial: a producer and consumer 4.0 us apart with 592
+// blocks against 5.3, 2.8 against 3.8 with 16).
+__device__ __forceinline__ double sum_partials(const double *part, int np)
+{
+    __shared__ double sh[kThreads / 32];
+    double v = 0.0;
+    for (int b = threadIdx.x; b < np; b += kThreads) v += __ldcg(part + b);
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = v;
+    __syncthreads();
+    v = 0.0;
+    for (int w = 0; w < kThreads / 32; ++w) v += sh[w];
+    return v;
 }
 
 __device__ __forceinline__ bool bnd(int i, int j, int m, int n) { return i == 0 || j == 0 || i == m - 1 || j == n - 1; }
@@ -350,6 +393,7 @@ __global__ void dot_kernel(const T *__restrict__ a, const T *__restrict__ b, lon
     if (reduce_last<1>(v, partials, counter, tot) && threadIdx.x == 0) *out = tot[0];
 }
 
+// ---- the host-driven loop's kernels (each dot product's total in S)
 // alpha = rz / (p.q) from the device scalars
 template <typename T>
 __global__ void pcg_pq_kernel(const T *__restrict__ p, const T *__restrict__ q, long long N, DevScalars *s,
@@ -379,10 +423,9 @@ __global__ void pcg_pq_kernel(const T *__restrict__ p, const T *__restrict__ q, 
 // so that z need not be kept). Returns the totals to the last block.
 template <typename T>
 __device__ __forceinline__ bool xr_update(T *__restrict__ x, T *__restrict__ r, const T *__restrict__ p,
-                                          const T *__restrict__ q, const T *__restrict__ z, long long N,
-                                          const DevScalars *s, double *partials, unsigned *counter, double (&tot)[2])
+                                          const T *__restrict__ q, const T *__restrict__ z, long long N, T al,
+                                          double *partials, unsigned *counter, double (&tot)[2])
 {
-    const T al = (T)s->alpha;
     double v[2] = {0.0, 0.0};
     vloop<T>(N, al16(x) && al16(r) && al16(p) && al16(q) && al16(z), [&](long long i, int c) {
         Pk<T> xv = ldc(x, i, c), rv = ldc(r, i, c);
@@ -407,26 +450,75 @@ __global__ void pcg_xr_kernel(T *__restrict__ x, T *__restrict__ r, const T *__r
                               const T *__restrict__ z, long long N, DevScalars *s, double *partials, unsigned *counter)
 {
     double tot[2];
-    if (xr_update(x, r, p, q, z, N, s, partials, counter, tot) && threadIdx.x == 0) {
+    if (xr_update(x, r, p, q, z, N, (T)s->alpha, partials, counter, tot) && threadIdx.x == 0) {
         s->rr = tot[0];
         s->rzo = tot[1];
     }
 }
 
-// Same update inside the device-side loop: counts the iteration and sets the
-// loop's condition (continue while rr > tol2, it < maxit, no breakdown, finite).
+// ---- the device-side loop's kernels: dot products as block partials, summed
+// by the kernel that uses them (sum_partials); r.z of iteration `it` in
+// rzv[it & 1], so that no block reads a scalar another block has replaced
 template <typename T>
-__global__ void pcg_xr_cond_kernel(T *__restrict__ x, T *__restrict__ r, const T *__restrict__ p,
-                                   const T *__restrict__ q, const T *__restrict__ z, long long N, DevScalars *s,
-                                   double *partials, unsigned *counter, cudaGraphConditionalHandle h)
+__global__ void __launch_bounds__(kThreads) loop_dot_kernel(const T *__restrict__ a, const T *__restrict__ b, long long N,
+                                                            double *part)
 {
     pdl_begin();
+    double v = 0.0;
+    vloop<T>(N, al16(a) && al16(b), [&](long long i, int c) {
+        const Pk<T> x = ldc(a, i, c), y = ldc(b, i, c);
+#pragma unroll
+        for (int k = 0; k < Pk<T>::n; ++k)
+            if (k < c) v += (double)x.v[k] * (double)y.v[k];
+    });
+    put_partial(v, part);
+}
+
+// Flexible (Polak-Ribiere) beta = r.(z - z_old) / rz_old with r.z_old = rzo
+// from the last update, zero in the first iteration; p = z + beta p.
+template <typename T>
+__global__ void __launch_bounds__(kThreads) loop_p_kernel(T *__restrict__ p, const T *__restrict__ z, long long N,
+                                                          DevScalars *s, const double *part, int np)
+{
+    pdl_begin();
+    const double rz = sum_partials(part, np);
+    const int it = s->it;
+    const T be = it == 0 ? T(0) : (T)((rz - s->rzo) / s->rzv[(it & 1) ^ 1]);
+    if (blockIdx.x == 0 && threadIdx.x == 0) s->rzv[it & 1] = rz;
+    vloop<T>(N, al16(p) && al16(z), [&](long long i, int c) {
+        const Pk<T> zv = ldc(z, i, c);
+        if (it == 0) {   // the first direction never reads stale p
+            stc(p, i, c, zv);
+            return;
+        }
+        Pk<T> pv = ldc(p, i, c);
+#pragma unroll
+        for (int k = 0; k < Pk<T>::n; ++k) pv.v[k] = zv.v[k] + be * pv.v[k];
+        stc(p, i, c, pv);
+    });
+}
+
+// alpha = rz / p.q (zero, and a breakdown, unless p.q > 0); the update; counts
+// the iteration and sets the loop's condition (continue while rr > tol2, it <
+// maxit, no breakdown, finite).
+template <typename T>
+__global__ void __launch_bounds__(kThreads)
+    loop_xr_kernel(T *__restrict__ x, T *__restrict__ r, const T *__restrict__ p, const T *__restrict__ q,
+                   const T *__restrict__ z, long long N, DevScalars *s, const double *part, int np, double *partials,
+                   unsigned *counter, cudaGraphConditionalHandle h)
+{
+    pdl_begin();
+    const double pq = sum_partials(part, np);
+    const bool bad = !(pq > 0.0) || s->breakdown;   // breakdown already set: by the preconditioner
+    const double alpha = bad ? 0.0 : s->rzv[s->it & 1] / pq;
     double tot[2];
-    if (xr_update(x, r, p, q, z, N, s, partials, counter, tot) && threadIdx.x == 0) {
+    if (xr_update(x, r, p, q, z, N, (T)alpha, partials, counter, tot) && threadIdx.x == 0) {
+        s->alpha = alpha;
+        if (bad) s->breakdown = 1;
         s->rr = tot[0];
         s->rzo = tot[1];
         s->it += 1;
-        const bool go = tot[0] > s->tol2 && s->it < s->maxit && !s->breakdown && tot[0] == tot[0];
+        const bool go = tot[0] > s->tol2 && s->it < s->maxit && !bad && tot[0] == tot[0];
         cudaGraphSetConditional(h, go ? 1u : 0u);
     }
 }
@@ -440,11 +532,10 @@ __global__ void loop_init_kernel(DevScalars *s, double tol2, int maxit)
 }
 
 // Flexible (Polak-Ribiere) beta = r.(z - z_old) / rz_old with r.z_old = rzo
-// from the update kernel; rz = r.z. loop: in the device-side loop, whose first
-// pass has no old direction (beta = 0).
+// from the update kernel; rz = r.z.
 template <typename T>
 __global__ void pcg_beta_kernel(const T *__restrict__ r, const T *__restrict__ z, long long N, DevScalars *s,
-                                double *partials, unsigned *counter, int loop)
+                                double *partials, unsigned *counter)
 {
     pdl_begin();
     double v[1] = {0.0};
@@ -456,18 +547,15 @@ __global__ void pcg_beta_kernel(const T *__restrict__ r, const T *__restrict__ z
     });
     double tot[1];
     if (reduce_last<1>(v, partials, counter, tot) && threadIdx.x == 0) {
-        s->beta = loop && s->it == 0 ? 0.0 : (tot[0] - s->rzo) / s->rz;
+        s->beta = (tot[0] - s->rzo) / s->rz;
         s->rz = tot[0];
     }
 }
 
-// first: 1 the first direction (p = z), 0 a later one, -1 by the device-side
-// loop's iteration count.
 template <typename T>
 __global__ void pcg_p_kernel(T *__restrict__ p, const T *__restrict__ z, long long N, const DevScalars *s, int first)
 {
     pdl_begin();
-    if (first < 0) first = s->it == 0;
     const T be = first ? T(0) : (T)s->beta;
     vloop<T>(N, al16(p) && al16(z), [&](long long i, int c) {
         const Pk<T> zv = ldc(z, i, c);
@@ -739,42 +827,47 @@ static int tri_warps(int nyp, size_t esz, size_t &smem)
 // blockIdx.y strides over the columns b, so no index division is needed. With
 // sc (FP64 vectors, FP32 transform) the gather divides by pc_scale and the
 // scatter multiplies by it.
-// z = r on the boundary ring of the m x n grid (identity rows of K_fem),
-// ring entries t0, t0 + stride, ...
+// Entry t of the boundary ring of the m x n grid (2 m + 2 (n - 2) entries).
+__device__ __forceinline__ long long ring_index(long long t, int m, int n)
+{
+    if (t < m) return t;
+    if (t < 2LL * m) return (long long)(n - 1) * m + (t - m);
+    const long long u = t - 2LL * m;
+    return (1 + u / 2) * m + ((u % 2) ? (m - 1) : 0);
+}
+
+// z = r on the boundary ring (identity rows of K_fem; ks r ks with a scaling
+// ks), ring entries t0, t0 + stride, ...
 template <typename T>
-__device__ __forceinline__ void ring_copy(T *__restrict__ z, const T *__restrict__ r, int m, int n, long long t0,
-                                          long long stride)
+__device__ __forceinline__ void ring_copy(T *__restrict__ z, const T *__restrict__ r, const T *__restrict__ ks, int m,
+                                          int n, long long t0, long long stride)
 {
     const long long nb = 2LL * m + 2LL * (n - 2);
     for (long long t = t0; t < nb; t += stride) {
-        long long idx;
-        if (t < m) idx = t;
-        else if (t < 2LL * m) idx = (long long)(n - 1) * m + (t - m);
-        else {
-            const long long u = t - 2LL * m;
-            const long long j = 1 + u / 2;
-            idx = j * m + ((u % 2) ? (m - 1) : 0);
-        }
-        z[idx] = r[idx];
+        const long long i = ring_index(t, m, n);
+        z[i] = ks ? ks[i] * r[i] * ks[i] : r[i];
     }
 }
 
-// The gather also copies the boundary ring of r into z (one launch fewer).
+// The gather also copies the boundary ring of r into z (one launch fewer) and
+// applies the kappa scaling ks (or null) on the way in.
 // With the parity split (kb > 0) column c of U is, for c < kb, the even fold
 // r[c] + r[nx-1-c] (c < fo; the middle entry r[fo] alone when nx is odd) and,
 // for c >= kb, the odd fold r[j] - r[nx-1-j] with j = c - kb < fo.
 template <typename T, typename V>
-__global__ void fd_gather_kernel(const V *__restrict__ r, T *__restrict__ U, V *__restrict__ z, int m, int n, int nx,
-                                 int ny, int nxp, int nyp, int kb, int fo, const DevScalars *sc)
+__global__ void fd_gather_kernel(const V *__restrict__ r, const V *__restrict__ ks, T *__restrict__ U, V *__restrict__ z,
+                                 int m, int n, int nx, int ny, int nxp, int nyp, int kb, int fo, const DevScalars *sc)
 {
     pdl_begin();
-    ring_copy(z, r, m, n, ((long long)blockIdx.y * gridDim.x + blockIdx.x) * blockDim.x + threadIdx.x,
+    ring_copy(z, r, ks, m, n, ((long long)blockIdx.y * gridDim.x + blockIdx.x) * blockDim.x + threadIdx.x,
               (long long)gridDim.x * gridDim.y * blockDim.x);
     constexpr int VN = Pk<T>::n;
     const double inv = sc ? 1.0 / pc_scale(sc) : 1.0;
     const int nv = nxp / VN;
     for (int b = blockIdx.y; b < nyp; b += gridDim.y) {
         const V *rb = r + (size_t)(b + 1) * m + 1;
+        const V *kr = ks ? ks + (size_t)(b + 1) * m + 1 : nullptr;
+        auto at = [&](int i) { return kr ? (double)(V)(rb[i] * kr[i]) : (double)rb[i]; };
         for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < nv; k += gridDim.x * blockDim.x) {
             Pk<T> o;
 #pragma unroll
@@ -783,12 +876,12 @@ __global__ void fd_gather_kernel(const V *__restrict__ r, T *__restrict__ U, V *
                 double v = 0.0;
                 if (b < ny) {
                     if (kb == 0) {
-                        if (a < nx) v = (double)rb[a];
+                        if (a < nx) v = at(a);
                     } else if (a < kb) {
-                        if (a < fo) v = (double)rb[a] + (double)rb[nx - 1 - a];
-                        else if (a == fo && (nx & 1)) v = (double)rb[a];
+                        if (a < fo) v = at(a) + at(nx - 1 - a);
+                        else if (a == fo && (nx & 1)) v = at(a);
                     } else if (a - kb < fo) {
-                        v = (double)rb[a - kb] - (double)rb[nx - 1 - (a - kb)];
+                        v = at(a - kb) - at(nx - 1 - (a - kb));
                     }
                 }
                 o.v[c] = (T)(v * inv);
@@ -801,10 +894,15 @@ __global__ void fd_gather_kernel(const V *__restrict__ r, T *__restrict__ U, V *
 // z's interior from the parity-split transform W [nyp][nxp] (even block
 // Ze = columns 0 .. fe-1, odd block Zo = columns kb .. kb+fo-1):
 // z[j] = Ze[j] + Zo[j], z[nx-1-j] = Ze[j] - Zo[j] (j < fo), and the middle
-// entry z[fo] = Ze[fo] when nx is odd; times sqrt(*rr) when rr is set.
+// entry z[fo] = Ze[fo] when nx is odd; times sqrt(*rr) when rr is set and times
+// the kappa scaling ks (or null). With part it also takes the solver's next
+// dot product, r . z over the whole grid, as block partials while z is in
+// registers (one launch and two passes fewer an iteration). A warp takes 32
+// columns of one row at a time.
 template <typename T, typename V>
-__global__ void fd_unfold_kernel(const T *__restrict__ W, V *__restrict__ z, int m, int nx, int ny, int nxp, int kb,
-                                 int fe, int fo, const double *rr)
+__global__ void __launch_bounds__(kThreads)
+    fd_unfold_kernel(const T *__restrict__ W, const V *__restrict__ r, const V *__restrict__ ks, V *__restrict__ z, int m,
+                     int n, int nx, int ny, int nxp, int kb, int fe, int fo, const double *rr, double *part)
 {
     pdl_begin();
     double f = 1.0;
@@ -812,26 +910,43 @@ __global__ void fd_unfold_kernel(const T *__restrict__ W, V *__restrict__ z, int
         const double v = *rr;
         f = (v > 0.0 && v < 1e300) ? sqrt(v) : 1.0;
     }
-    for (int b = blockIdx.y; b < ny; b += gridDim.y) {
+    const int lane = threadIdx.x & 31, cb = (fe + 31) / 32;
+    const int w0 = blockIdx.x * (kThreads / 32) + (threadIdx.x >> 5), ws = gridDim.x * (kThreads / 32);
+    double dot = 0.0;
+    for (long long u = w0; u < (long long)cb * ny; u += ws) {
+        const int b = (int)(u / cb), j = (int)(u - (long long)b * cb) * 32 + lane;
+        if (j >= fe) continue;
         const T *wb = W + (size_t)b * nxp;
-        V *zb = z + (size_t)(b + 1) * m + 1;
-        for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < fe; j += gridDim.x * blockDim.x) {
-            const double e = (double)wb[j];
-            if (j < fo) {
-                const double o = (double)wb[kb + j];
-                zb[j] = (V)(f * (e + o));
-                zb[nx - 1 - j] = (V)(f * (e - o));
-            } else {
-                zb[j] = (V)(f * e);
-            }
+        const size_t o = (size_t)(b + 1) * m + 1, i0 = o + j, i1 = o + (nx - 1 - j);
+        const double e = (double)wb[j];
+        V z0 = (V)(f * e), z1 = V(0);
+        if (j < fo) {
+            const double d = (double)wb[kb + j];
+            z0 = (V)(f * (e + d));
+            z1 = (V)(f * (e - d));
+            if (ks) z1 *= ks[i1];
+            z[i1] = z1;
+        }
+        if (ks) z0 *= ks[i0];
+        z[i0] = z0;
+        if (part) {
+            dot += (double)r[i0] * (double)z0;
+            if (j < fo) dot += (double)r[i1] * (double)z1;
         }
     }
+    if (!part) return;
+    for (long long t = blockIdx.x * (long long)kThreads + threadIdx.x; t < 2LL * m + 2LL * (n - 2);
+         t += (long long)gridDim.x * kThreads) {
+        const long long i = ring_index(t, m, n);
+        const V rv = r[i], zv = ks ? ks[i] * rv * ks[i] : rv;
+        dot += (double)rv * (double)zv;
+    }
+    put_partial(dot, part);
 }
 
-// 2-D launch of the gather / unfold: 128-thread blocks over the groups of a
+// 2-D launch of the gather: 128-thread blocks over the groups of a
 // row, block rows striding over the rows. About one wave of blocks (16 per
-// SM): one block per row made these kernels block-launch bound (the FP32
-// unfold of a 2049 x 1025 half took 21 us in 18.4 K blocks of one row each).
+// SM): one block per row made it block-launch bound.
 static dim3 grid2d(int ngroups, int nrows, int nsm)
 {
     const int gx = std::max(1, (ngroups + 127) / 128);
@@ -841,10 +956,10 @@ static dim3 grid2d(int ngroups, int nrows, int nsm)
 
 // z = r on the boundary ring (identity rows of K_fem).
 template <typename T>
-__global__ void boundary_copy_kernel(T *__restrict__ z, const T *__restrict__ r, int m, int n)
+__global__ void boundary_copy_kernel(T *__restrict__ z, const T *__restrict__ r, const T *__restrict__ ks, int m, int n)
 {
     pdl_begin();
-    ring_copy(z, r, m, n, blockIdx.x * (long long)blockDim.x + threadIdx.x, (long long)gridDim.x * blockDim.x);
+    ring_copy(z, r, ks, m, n, blockIdx.x * (long long)blockDim.x + threadIdx.x, (long long)gridDim.x * blockDim.x);
 }
 
 // ------------------------------------------------------------ kappa scaling of the preconditioner
@@ -893,12 +1008,18 @@ __global__ void __launch_bounds__(kKsX *kKsY) kappa_scale_kernel(const double *_
     s32[(size_t)R * g.m + C] = (float)v;
 }
 
+// out = a b on `rows` rows of `cols` entries, ld apart; ld > 0: the interior of
+// an m = ld wide grid (the boundary ring is left alone).
 template <typename T>
-__global__ void mul_kernel(T *__restrict__ out, const T *__restrict__ a, const T *__restrict__ b, long long N)
+__global__ void mul_kernel(T *__restrict__ out, const T *__restrict__ a, const T *__restrict__ b, int rows, int cols,
+                           int ld)
 {
     pdl_begin();
-    for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < N; t += (long long)gridDim.x * blockDim.x)
-        out[t] = a[t] * b[t];
+    const long long N = (long long)rows * cols;
+    for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < N; t += (long long)gridDim.x * blockDim.x) {
+        const long long i = ld > 0 ? (t / cols + 1) * ld + 1 + t % cols : t;
+        out[i] = a[i] * b[i];
+    }
 }
 
 // ------------------------------------------------------------ host state
@@ -945,6 +1066,8 @@ struct PrecState {
 struct SolverState {
     int device = 0;
     cudaStream_t stream = nullptr;
+    cudaEvent_t ev = nullptr;   // orders a call's work on `stream` after and before the caller's stream
+    bool pc_chain = false;  // a call outside any capture: the exact preconditioner's kernels as programmatic dependents
     bool pc_sync = false;   // IGA_PC_FEM_CG: the call wants the inner solve's status at once
     bool fd_host = false;
     // host x eigenpairs (built once). Split by parity (fold): even modes
@@ -959,7 +1082,9 @@ struct SolverState {
     int kappa_version = 0;
     DevScalars *s = nullptr;
     DevScalars *h = nullptr;   // pinned mirror
-    double *partials = nullptr;
+    double *partials = nullptr;   // of reduce_last; then the loop's p.q and r.z partials (kRedBlocks each)
+    double *part_pq() const { return partials + 4 * kRedBlocks; }
+    double *part_rz() const { return partials + 5 * kRedBlocks; }
     unsigned *counter = nullptr;
     double *r64 = nullptr, *q64 = nullptr;   // refinement residual / operator output
     PrecState<double> d;
@@ -1119,8 +1244,9 @@ static int ensure_state(iga_plan *pl, SolverState **out)
     SOLVE_TRY(cudaStreamCreateWithFlags(&S->stream, cudaStreamNonBlocking));
     SOLVE_TRY(cudaMalloc((void **)&S->s, sizeof(DevScalars)));
     SOLVE_TRY(cudaMemset(S->s, 0, sizeof(DevScalars)));
+    SOLVE_TRY(cudaEventCreateWithFlags(&S->ev, cudaEventDisableTiming));
     SOLVE_TRY(cudaMallocHost((void **)&S->h, sizeof(DevScalars)));
-    SOLVE_TRY(cudaMalloc((void **)&S->partials, sizeof(double) * kRedBlocks * 4));
+    SOLVE_TRY(cudaMalloc((void **)&S->partials, sizeof(double) * kRedBlocks * 6));
     SOLVE_TRY(cudaMalloc((void **)&S->counter, sizeof(unsigned)));
     SOLVE_TRY(cudaMemset(S->counter, 0, sizeof(unsigned)));
     SOLVE_TRY(cudaMalloc((void **)&S->r64, sizeof(double) * pl->nfunc));
@@ -1156,6 +1282,7 @@ void iga_solver_release(iga_plan *pl)
                     (void *)S->ks64, (void *)S->ks32})
         if (v) cudaFree(v);
     if (S->h) cudaFreeHost(S->h);
+    if (S->ev) cudaEventDestroy(S->ev);
     if (S->stream) cudaStreamDestroy(S->stream);
     delete S;
     pl->solver = nullptr;
@@ -1416,22 +1543,37 @@ static int transform_gemm(PrecState<float> &ps, const iga_plan *pl, int which, c
 // tridiagonal solves (the fast diagonalisation in both directions would take
 // four GEMMs). With the parity split the gather folds r (r[i] +- r[nx-1-i]),
 // the GEMMs work on the two half blocks, and the unfold kernel forms z.
+// ks: the kappa scaling of r and z, or null. rz (or null): where the r . z
+// partials go; its n stays 0 when this path does not take them.
 // V is the vectors' type; an FP32 transform of FP64 vectors (T = float,
 // V = double) passes sc, the device scalars whose rr scales the data.
+struct DotPart {
+    double *part = nullptr;
+    int n = 0;
+};
+
 template <typename T, typename V>
-static int fd_apply(PrecState<T> &ps, const iga_plan *pl, SolverState *S, const V *r, V *z, const DevScalars *sc)
+static int fd_apply(PrecState<T> &ps, const iga_plan *pl, SolverState *S, const V *r, V *z, const DevScalars *sc,
+                    const V *ks, DotPart *rz)
 {
     const int m = pl->m, n = pl->n, nx = m - 2, ny = n - 2;
     if (nx <= 0 || ny <= 0) {   // no free nodes: the ring is everything
-        SOLVE_TRY(launch_k(boundary_copy_kernel<V>, dim3(kRedBlocks), dim3(kThreads), 0, S->stream, z, r, m, n));
+        SOLVE_TRY(launch_k(boundary_copy_kernel<V>, dim3(kRedBlocks), dim3(kThreads), 0, S->stream, z, r, ks, m, n));
         return IGA_OK;
     }
     const int nxp = ps.nxp, nyp = ps.nyp;
     int seg = (ny + 31) / 32;
     seg |= 1;   // odd: conflict-free shared-memory rows
     constexpr int VN = Pk<T>::n;
-    SOLVE_TRY(launch_k(fd_gather_kernel<T, V>, grid2d(nxp / VN, nyp, ps.nsm), dim3(128), 0, S->stream, r, ps.W2, z, m, n, nx, ny,
+    SOLVE_TRY(launch_k(fd_gather_kernel<T, V>, grid2d(nxp / VN, nyp, ps.nsm), dim3(128), 0, S->stream, r, ks, ps.W2, z, m, n, nx, ny,
                        nxp, nyp, ps.kb, ps.fo, sc));
+    // the gather follows whatever the stream holds (a wait for the caller's
+    // stream, say); its successors follow this call's own kernels
+    struct Chain {
+        bool was = pdl_capture();
+        ~Chain() { pdl_capture() = was; }
+    } chain;
+    if (S->pc_chain) pdl_capture() = true;
     int e = transform_gemm(ps, pl, 1, S->stream);
     if (e == IGA_OK) {
         if (ps.tri_w) {
@@ -1451,10 +1593,14 @@ static int fd_apply(PrecState<T> &ps, const iga_plan *pl, SolverState *S, const 
             // parity split: the second GEMM writes both halves' products, the
             // unfold kernel combines them into z's interior
             e = transform_gemm(ps, pl, 2, S->stream);
-            if (e == IGA_OK)
-                SOLVE_TRY(launch_k(fd_unfold_kernel<T, V>, grid2d(ps.fe, ny, ps.nsm), dim3(128), 0, S->stream,
-                                   (const T *)ps.W2, z, m, nx, ny, nxp, ps.kb, ps.fe, ps.fo,
-                                   sc ? &sc->rr : (const double *)nullptr));
+            if (e == IGA_OK) {
+                const long long items = (long long)((ps.fe + 31) / 32) * ny;
+                const int blocks = (int)std::max(1LL, std::min<long long>(kRedBlocks, (items + 7) / 8));
+                SOLVE_TRY(launch_k(fd_unfold_kernel<T, V>, dim3(blocks), dim3(kThreads), 0, S->stream,
+                                   (const T *)ps.W2, r, ks, z, m, n, nx, ny, nxp, ps.kb, ps.fe, ps.fo,
+                                   sc ? &sc->rr : (const double *)nullptr, rz ? rz->part : (double *)nullptr));
+                if (rz) rz->n = blocks;
+            }
         } else {
             // the second GEMM's epilogue writes z's interior itself
             GemmScatter gs;
@@ -1465,6 +1611,9 @@ static int fd_apply(PrecState<T> &ps, const iga_plan *pl, SolverState *S, const 
             gs.cols = nx;
             gs.rr = sc ? &sc->rr : nullptr;
             e = transform_gemm(ps, pl, 2, S->stream, gs);
+            if (e == IGA_OK && ks)
+                SOLVE_TRY(launch_k(mul_kernel<V>, dim3(kRedBlocks), dim3(kThreads), 0, S->stream, z, (const V *)z, ks, ny, nx,
+                                   m));
         }
     }
     if (e != IGA_OK) {
@@ -1483,7 +1632,7 @@ static int sync_scalars(SolverState *S)
 
 template <typename T>
 static int pc_apply_core(PrecState<T> &ps, const iga_plan *pl, SolverState *S, const iga_solve_opts &o, const T *r,
-                         T *z, double pc_rtol, int64_t &pc_iters);
+                         T *z, double pc_rtol, int64_t &pc_iters, const T *ks = nullptr, DotPart *rz = nullptr);
 
 static const double *kscale(SolverState *S, double *) { return S->ks64; }
 static const float *kscale(SolverState *S, float *) { return S->ks32; }
@@ -1510,30 +1659,32 @@ static int update_kscale(const iga_plan *pl, SolverState *S)
 // output multiplied back into FP64. The outer flexible PCG absorbs the FP32
 // (TF32 GEMM) rounding of the preconditioner.
 static int pc_apply_fp32(const iga_plan *pl, SolverState *S, const iga_solve_opts &o, const double *r, double *z,
-                         double pc_rtol, int64_t &pc_iters)
+                         double pc_rtol, int64_t &pc_iters, DotPart *rz)
 {
     const long long N = pl->nfunc;
     PrecState<float> &f = S->f;
     int st;
-    const double *rin = r;
-    if (pl->kappa_dev) {
-        if ((st = update_kscale(pl, S))) return st;
-        mul_kernel<double><<<kRedBlocks, kThreads, 0, S->stream>>>(S->d.sc, r, S->ks64, N);
-        rin = S->d.sc;
-    }
+    if (pl->kappa_dev && (st = update_kscale(pl, S))) return st;
+    const double *ks = pl->kappa_dev ? S->ks64 : nullptr;
     if (o.pc == IGA_PC_FEM_EXACT) {
         if ((st = fd_upload(f, pl, S))) return st;
-        if ((st = fd_apply<float, double>(f, pl, S, rin, z, S->s))) return st;
-    } else {
+        return fd_apply<float, double>(f, pl, S, r, z, S->s, ks, rz);
+    }
+    const double *rin = r;
+    if (ks) {
+        SOLVE_TRY(launch_k(mul_kernel<double>, dim3(kRedBlocks), dim3(kThreads), 0, S->stream, S->d.sc, r, ks, 1, (int)N, 0));
+        rin = S->d.sc;
+    }
+    {
         SOLVE_TRY(launch_k(to_fp32_kernel, dim3(kRedBlocks), dim3(kThreads), 0, S->stream, rin, f.sc, N,
                            (const DevScalars *)S->s));
         if ((st = pc_apply_core<float>(f, pl, S, o, f.sc, f.tz, pc_rtol, pc_iters))) return st;
         SOLVE_TRY(launch_k(from_fp32_kernel, dim3(kRedBlocks), dim3(kThreads), 0, S->stream, (const float *)f.tz, z, N,
                            (const DevScalars *)S->s));
     }
-    if (pl->kappa_dev)
-        SOLVE_TRY(launch_k(mul_kernel<double>, dim3(kRedBlocks), dim3(kThreads), 0, S->stream, z, (const double *)z,
-                           (const double *)S->ks64, N));
+    if (ks)
+        SOLVE_TRY(launch_k(mul_kernel<double>, dim3(kRedBlocks), dim3(kThreads), 0, S->stream, z, (const double *)z, ks, 1,
+                           (int)N, 0));
     return IGA_OK;
 }
 
@@ -1541,25 +1692,28 @@ static int pc_apply_fp32(const iga_plan *pl, SolverState *S, const iga_solve_opt
 // z = S M^-1 (S r) with the local scaling S.
 template <typename T>
 static int pc_apply(PrecState<T> &ps, const iga_plan *pl, SolverState *S, const iga_solve_opts &o, const T *r, T *z,
-                    double pc_rtol, int64_t &pc_iters)
+                    double pc_rtol, int64_t &pc_iters, DotPart *rz = nullptr)
 {
-    const long long N = pl->nfunc;
+    const int N = (int)pl->nfunc;
     if constexpr (std::is_same<T, double>::value) {
-        if (o.precision == IGA_MIXED_PC && o.pc != IGA_PC_NONE) return pc_apply_fp32(pl, S, o, r, z, pc_rtol, pc_iters);
+        if (o.precision == IGA_MIXED_PC && o.pc != IGA_PC_NONE)
+            return pc_apply_fp32(pl, S, o, r, z, pc_rtol, pc_iters, rz);
     }
-    if (o.pc == IGA_PC_NONE || !pl->kappa_dev) return pc_apply_core(ps, pl, S, o, r, z, pc_rtol, pc_iters);
+    if (o.pc == IGA_PC_NONE || !pl->kappa_dev)
+        return pc_apply_core(ps, pl, S, o, r, z, pc_rtol, pc_iters, (const T *)nullptr, rz);
     int st;
     if ((st = update_kscale(pl, S))) return st;
     const T *sv = kscale(S, (T *)nullptr);
-    SOLVE_TRY(launch_k(mul_kernel<T>, dim3(kRedBlocks), dim3(kThreads), 0, S->stream, ps.sc, r, sv, N));
+    if (o.pc == IGA_PC_FEM_EXACT) return pc_apply_core(ps, pl, S, o, r, z, pc_rtol, pc_iters, sv, rz);
+    SOLVE_TRY(launch_k(mul_kernel<T>, dim3(kRedBlocks), dim3(kThreads), 0, S->stream, ps.sc, r, sv, 1, N, 0));
     if ((st = pc_apply_core(ps, pl, S, o, ps.sc, z, pc_rtol, pc_iters))) return st;
-    SOLVE_TRY(launch_k(mul_kernel<T>, dim3(kRedBlocks), dim3(kThreads), 0, S->stream, z, (const T *)z, sv, N));
+    SOLVE_TRY(launch_k(mul_kernel<T>, dim3(kRedBlocks), dim3(kThreads), 0, S->stream, z, (const T *)z, sv, 1, N, 0));
     return IGA_OK;
 }
 
 template <typename T>
 static int pc_apply_core(PrecState<T> &ps, const iga_plan *pl, SolverState *S, const iga_solve_opts &o, const T *r,
-                         T *z, double pc_rtol, int64_t &pc_iters)
+                         T *z, double pc_rtol, int64_t &pc_iters, const T *ks, DotPart *rz)
 {
     const long long N = pl->nfunc;
     if (o.pc == IGA_PC_NONE) {
@@ -1569,7 +1723,7 @@ static int pc_apply_core(PrecState<T> &ps, const iga_plan *pl, SolverState *S, c
     int st;
     if (o.pc == IGA_PC_FEM_EXACT) {
         if ((st = fd_upload(ps, pl, S))) return st;
-        return fd_apply<T, T>(ps, pl, S, r, z, nullptr);
+        return fd_apply<T, T>(ps, pl, S, r, z, nullptr, ks, rz);
     }
     if (ps.icg.C) {   // one cluster runs the whole inner solve
         IcgArgs<T> a;
@@ -1668,7 +1822,7 @@ static int pcg(iga_plan *pl, SolverState *S, PrecState<T> &ps, const iga_solve_o
         if (!std::isfinite(S->h->rr)) return IGA_ERR_NONFINITE;
         if (std::sqrt(S->h->rr) <= rtol * bnorm) return IGA_OK;
         if ((st = pc_apply(ps, pl, S, o, ps.r, ps.z, pc_rtol, pc_iters))) return st;
-        pcg_beta_kernel<T><<<kRedBlocks, kThreads, 0, s>>>(ps.r, ps.z, N, S->s, S->partials, S->counter, 0);
+        pcg_beta_kernel<T><<<kRedBlocks, kThreads, 0, s>>>(ps.r, ps.z, N, S->s, S->partials, S->counter);
         pcg_p_kernel<T><<<kRedBlocks, kThreads, 0, s>>>(ps.p, ps.z, N, S->s, 0);
     }
     return IGA_ERR_NOT_CONVERGED;
@@ -1709,7 +1863,19 @@ static int build_loop(iga_plan *pl, SolverState *S, PrecState<T> &ps, const iga_
     int64_t dummy = 0;
     // Programmatic dependencies between the body's kernels.
     pdl_capture() = true;
-    int st = pc_apply(ps, pl, S, o, ps.r, ps.z, o.pc_rtol, dummy);
+    DotPart rz;
+    rz.part = S->part_rz();
+    int st = pc_apply(ps, pl, S, o, ps.r, ps.z, o.pc_rtol, dummy, &rz);
+    const int nb = vec_blocks<T>(N);
+    // the vector kernels of vectors of 4 MB or more get ordinary edges: their
+    // blocks run long enough for an uneven start to cost more than a launch
+    // gap (1024^2 mixed 118.8 -> 117 us an iteration, 2048^2 FP64 1111 -> 1100;
+    // 512^2 FP64 97.7 -> 99.5)
+    const bool even = N * (long long)sizeof(T) >= (4LL << 20);
+    auto launch_vec = [&](auto kern, auto... args) {
+        return even ? launch_even(kern, dim3(nb), dim3(kThreads), 0, s, args...)
+                    : launch_k(kern, dim3(nb), dim3(kThreads), 0, s, args...);
+    };
     auto launched = [&](cudaError_t e) {
         if (e != cudaSuccess && !st) {
             set_error(std::string("PCG loop launch: ") + cudaGetErrorString(e));
@@ -1717,17 +1883,17 @@ static int build_loop(iga_plan *pl, SolverState *S, PrecState<T> &ps, const iga_
         }
     };
     if (!st) {
-        launched(launch_k(pcg_beta_kernel<T>, dim3(kRedBlocks), dim3(kThreads), 0, s, (const T *)ps.r,
-                          (const T *)ps.z, N, S->s, S->partials, S->counter, 1));
-        launched(launch_k(pcg_p_kernel<T>, dim3(kRedBlocks), dim3(kThreads), 0, s, ps.p, (const T *)ps.z, N,
-                          (const DevScalars *)S->s, -1));
+        if (rz.n == 0) {   // no preconditioner that took r . z itself
+            launched(launch_vec(loop_dot_kernel<T>, (const T *)ps.r, (const T *)ps.z, N, rz.part));
+            rz.n = nb;
+        }
+        launched(launch_vec(loop_p_kernel<T>, ps.p, (const T *)ps.z, N, S->s, (const double *)rz.part, rz.n));
         if (!st) st = iga_apply_internal_sb(pl, prec, ps.p, ps.q, s, IGA_SIGN_SPD, IGA_BC_IDENTITY);
     }
     if (!st) {
-        launched(launch_k(pcg_pq_kernel<T>, dim3(kRedBlocks), dim3(kThreads), 0, s, (const T *)ps.p, (const T *)ps.q,
-                          N, S->s, S->partials, S->counter));
-        launched(launch_k(pcg_xr_cond_kernel<T>, dim3(kRedBlocks), dim3(kThreads), 0, s, ps.x, ps.r, (const T *)ps.p,
-                          (const T *)ps.q, (const T *)ps.z, N, S->s, S->partials, S->counter, h));
+        launched(launch_vec(loop_dot_kernel<T>, (const T *)ps.p, (const T *)ps.q, N, S->part_pq()));
+        launched(launch_vec(loop_xr_kernel<T>, ps.x, ps.r, (const T *)ps.p, (const T *)ps.q, (const T *)ps.z, N, S->s,
+                            (const double *)S->part_pq(), nb, S->partials, S->counter, h));
     }
     pdl_capture() = false;
     cudaGraph_t captured = body;
@@ -1864,10 +2030,11 @@ int iga_pc_apply(iga_plan *pl, int pc, int prec, const void *r, void *z, double 
     SolverState *S;
     int st;
     if ((st = ensure_state(pl, &S))) return st;
-    cudaEvent_t ev;
-    SOLVE_TRY(cudaEventCreateWithFlags(&ev, cudaEventDisableTiming));
-    SOLVE_TRY(cudaEventRecord(ev, (cudaStream_t)stream));
-    SOLVE_TRY(cudaStreamWaitEvent(S->stream, ev, 0));
+    SOLVE_TRY(cudaEventRecord(S->ev, (cudaStream_t)stream));
+    SOLVE_TRY(cudaStreamWaitEvent(S->stream, S->ev, 0));
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    SOLVE_TRY(cudaStreamIsCapturing(S->stream, &cap));
+    S->pc_chain = cap == cudaStreamCaptureStatusNone;
     iga_solve_opts o;
     iga_solve_opts_default(&o);
     o.pc = pc;
@@ -1881,10 +2048,9 @@ int iga_pc_apply(iga_plan *pl, int pc, int prec, const void *r, void *z, double 
         if (!(st = alloc_prec(S->f, pl, *S)))
             st = pc_apply<float>(S->f, pl, S, o, (const float *)r, (float *)z, pc_rtol, its);
     }
-    S->pc_sync = false;
-    SOLVE_TRY(cudaEventRecord(ev, S->stream));
-    SOLVE_TRY(cudaStreamWaitEvent((cudaStream_t)stream, ev, 0));
-    cudaEventDestroy(ev);
+    S->pc_sync = S->pc_chain = false;
+    SOLVE_TRY(cudaEventRecord(S->ev, S->stream));
+    SOLVE_TRY(cudaStreamWaitEvent((cudaStream_t)stream, S->ev, 0));
     return st;
 }
 
