@@ -395,16 +395,16 @@ int gemm_tf32_launch(const GemmTF32 &g, cudaStream_t s, int *err, const GemmScat
 }
 
 // ------------------------------------------------------------ FP64 on DMMA
-// A CTA of WMW x WNW warps computes a (16 WI WMW) x (32 WNW) tile of C; a
-// warp tile is WI x 4 blocks of the 16 x 8 x 8 FP64 MMA. K slices of 16 are
+// A CTA of WMW x WNW warps computes a (16 WI WMW) x (8 NJ WNW) tile of C; a
+// warp tile is WI x NJ blocks of the 16 x 8 x 8 FP64 MMA. K slices of 16 are
 // staged by 16-byte cp.async into a 3-deep ring: K-major operands as
 // [row][k] with 20 doubles per row, MN-major ones as [k][row] with ROWS + 4
 // per k, both of which make a warp's fragment loads conflict-free. Rows and k
 // past an operand's extent are zero-filled (the matrices are zero-padded, so
-// a 16-byte chunk never straddles the end of the data). Three shapes:
-//   0: 128 x 128, 8 warps of 64 x 32 (one CTA per SM);
-//   1: 128 x 64, 8 warps of 32 x 32 (two CTAs per SM);
-//   2: 64 x 64, 4 warps of 32 x 32 (three CTAs per SM), the default.
+// a 16-byte chunk never straddles the end of the data). Two shapes:
+//   0: 64 x 64, 4 warps of 32 x 32 (three CTAs per SM);
+//   1: 32 x 32, 4 warps of 16 x 16 (six CTAs per SM).
+// (128-wide tiles with one or two CTAs per SM were slower at every size.)
 constexpr int kDK = 16, kDS = 3;
 constexpr int kDLK = 20;
 
@@ -454,15 +454,11 @@ template <int CFG>
 struct DCfg;
 template <>
 struct DCfg<0> {
-    static constexpr int WI = 4, WMW = 2, WNW = 4, MINB = 1;
+    static constexpr int WI = 2, NJ = 4, WMW = 2, WNW = 2, MINB = 3;
 };
 template <>
 struct DCfg<1> {
-    static constexpr int WI = 2, WMW = 4, WNW = 2, MINB = 2;
-};
-template <>
-struct DCfg<2> {
-    static constexpr int WI = 2, WMW = 2, WNW = 2, MINB = 3;
+    static constexpr int WI = 1, NJ = 2, WMW = 2, WNW = 2, MINB = 6;
 };
 
 template <int CFG, bool AMN, bool BMN, bool SCATTER>
@@ -472,8 +468,8 @@ __global__ void __launch_bounds__(32 * DCfg<CFG>::WMW * DCfg<CFG>::WNW, DCfg<CFG
                     GemmSplit split)
 {
     using Cf = DCfg<CFG>;
-    constexpr int WI = Cf::WI, NT = 32 * Cf::WMW * Cf::WNW;
-    constexpr int TM = 16 * WI * Cf::WMW, TN = 32 * Cf::WNW;
+    constexpr int WI = Cf::WI, NJ = Cf::NJ, NT = 32 * Cf::WMW * Cf::WNW;
+    constexpr int TM = 16 * WI * Cf::WMW, TN = 8 * NJ * Cf::WNW;
     using TA = DTile<AMN, TM>;
     using TB = DTile<BMN, TN>;
     pdl_begin();
@@ -481,15 +477,15 @@ __global__ void __launch_bounds__(32 * DCfg<CFG>::WMW * DCfg<CFG>::WNW, DCfg<CFG
     double *As = dsm, *Bs = dsm + kDS * TA::elems;
     const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
     const int g = lane >> 2, t4 = lane & 3;
-    const int wm = (w % Cf::WMW) * 16 * WI, wn = (w / Cf::WMW) * 32;
+    const int wm = (w % Cf::WMW) * 16 * WI, wn = (w / Cf::WMW) * 8 * NJ;
     const TileRange tr = tile_range(split, blockIdx.x, blockIdx.y, TM, TN, K, Mst, Nst);
     const int m0 = tr.m0, n0 = tr.n0, klo = tr.klo;
     const int nk = (tr.khi - klo + kDK - 1) / kDK;
-    double acc[WI][4][4];
+    double acc[WI][NJ][4];
 #pragma unroll
     for (int i = 0; i < WI; ++i)
 #pragma unroll
-        for (int j = 0; j < 4; ++j)
+        for (int j = 0; j < NJ; ++j)
 #pragma unroll
             for (int c = 0; c < 4; ++c) acc[i][j][c] = 0.0;
     for (int s = 0; s < kDS - 1; ++s) {
@@ -513,7 +509,7 @@ __global__ void __launch_bounds__(32 * DCfg<CFG>::WMW * DCfg<CFG>::WNW, DCfg<CFG
         const double *a = As + (kt % kDS) * TA::elems, *b = Bs + (kt % kDS) * TB::elems;
 #pragma unroll
         for (int kk = 0; kk < kDK; kk += 8) {
-            double av[WI][4], bv[4][2];
+            double av[WI][4], bv[NJ][2];
 #pragma unroll
             for (int i = 0; i < WI; ++i) {
                 const int r = wm + 16 * i + g;
@@ -523,14 +519,14 @@ __global__ void __launch_bounds__(32 * DCfg<CFG>::WMW * DCfg<CFG>::WNW, DCfg<CFG
                 av[i][3] = a[TA::at(r + 8, kk + t4 + 4)];
             }
 #pragma unroll
-            for (int j = 0; j < 4; ++j) {
+            for (int j = 0; j < NJ; ++j) {
                 bv[j][0] = b[TB::at(wn + 8 * j + g, kk + t4)];
                 bv[j][1] = b[TB::at(wn + 8 * j + g, kk + t4 + 4)];
             }
 #pragma unroll
             for (int i = 0; i < WI; ++i)
 #pragma unroll
-                for (int j = 0; j < 4; ++j) dmma(acc[i][j], av[i], bv[j]);
+                for (int j = 0; j < NJ; ++j) dmma(acc[i][j], av[i], bv[j]);
         }
     }
     cp_async_wait<0>();
@@ -549,7 +545,7 @@ __global__ void __launch_bounds__(32 * DCfg<CFG>::WMW * DCfg<CFG>::WNW, DCfg<CFG
                 const int row = m0 + wm + 16 * i + g + 8 * h;
                 if (row >= sc.rows || row >= tr.mlim) continue;
 #pragma unroll
-                for (int j = 0; j < 4; ++j)
+                for (int j = 0; j < NJ; ++j)
 #pragma unroll
                     for (int c = 0; c < 2; ++c) {
                         const int col = n0 + wn + 8 * j + 2 * t4 + c;
@@ -564,7 +560,7 @@ __global__ void __launch_bounds__(32 * DCfg<CFG>::WMW * DCfg<CFG>::WNW, DCfg<CFG
                 const int row = m0 + wm + 16 * i + g + 8 * h;
                 if (row >= tr.mlim) continue;
 #pragma unroll
-                for (int j = 0; j < 4; ++j) {
+                for (int j = 0; j < NJ; ++j) {
                     const int col = n0 + wn + 8 * j + 2 * t4;
                     double *dst = C + (size_t)row * ldc + col;
                     if (col + 1 < tr.nlim)
@@ -576,14 +572,12 @@ __global__ void __launch_bounds__(32 * DCfg<CFG>::WMW * DCfg<CFG>::WNW, DCfg<CFG
 }
 
 namespace {
-int g_f64_shape = -1;   // forced CTA shape (timing runs); -1: the default 64 x 64 shape
-
 template <int CFG, bool AMN, bool BMN, bool SCATTER>
 int launch_f64(GemmOperand A, GemmOperand B, double *C, int ldc, int M, int N, int K, int Mst, int Nst, cudaStream_t s,
                const GemmScatter &sc, GemmSplit split)
 {
     using Cf = DCfg<CFG>;
-    constexpr int TM = 16 * Cf::WI * Cf::WMW, TN = 32 * Cf::WNW, NT = 32 * Cf::WMW * Cf::WNW;
+    constexpr int TM = 16 * Cf::WI * Cf::WMW, TN = 8 * Cf::NJ * Cf::WNW, NT = 32 * Cf::WMW * Cf::WNW;
     const size_t smem = (size_t)kDS * (DTile<AMN, TM>::elems + DTile<BMN, TN>::elems) * sizeof(double);
     static bool attr = false;
     if (!attr) {
@@ -616,8 +610,6 @@ int launch_f64_layout(GemmOperand A, GemmOperand B, double *C, int ldc, int M, i
 }
 }  // namespace
 
-void gemm_f64_force_shape(int shape) { g_f64_shape = shape; }
-
 int gemm_f64_launch(GemmOperand A, GemmOperand B, double *C, int ldc, int M, int N, int K, int Mst, int Nst,
                     cudaStream_t s, const GemmScatter &sc, GemmSplit split)
 {
@@ -627,15 +619,23 @@ int gemm_f64_launch(GemmOperand A, GemmOperand B, double *C, int ldc, int M, int
         set_error("FP64 GEMM operands need 16-byte aligned rows (and an FP64 scatter target)");
         return IGA_ERR_ARG;
     }
-    // 64 x 64 tiles, three CTAs per SM, measured fastest at every size the
-    // preconditioner meets (2064^2: 586 us = 30.0 TFLOP/s against 614 us with
-    // 128 x 128; 1040^2: 78 us against 158 us; 528^2: 27 against 84 us)
-    const int shape = g_f64_shape >= 0 ? g_f64_shape : 2;
-    switch (shape) {
-    case 0: return launch_f64_layout<0>(A, B, C, ldc, M, N, K, Mst, Nst, s, sc, split);
-    case 1: return launch_f64_layout<1>(A, B, C, ldc, M, N, K, Mst, Nst, s, sc, split);
-    default: return launch_f64_layout<2>(A, B, C, ldc, M, N, K, Mst, Nst, s, sc, split);
-    }
+    // A GEMM lasts as long as the SM with the most tiles. A 64 x 64 tile takes
+    // about a tenth less time than four of 32 x 32 (fewer fragment loads per
+    // MMA), so the small ones are used where they give the fullest SM that
+    // much less: the preconditioner's two half-size transforms at p=3 512^2 (81
+    // tiles of 64 x 64 for 148 SMs) 50.2 -> 31.9 us in all, 700^2 105 -> 53,
+    // 1200^2 182 -> 165, 2048^2 709 -> 702; at 1024^2 (exactly two of 64 x 64
+    // an SM) 64 x 64 stays, 108 against 117.
+    int nsm = 148, dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
+        nsm = 148;
+    auto per_sm = [&](int t) {   // the most tiles of t x t an SM gets
+        const long long n = (long long)tiles_along(Mst, t, split.on_n ? 0 : split.kb) *
+                            tiles_along(Nst, t, split.on_n ? split.kb : 0);
+        return (n + nsm - 1) / nsm;
+    };
+    if (11 * per_sm(32) < 40 * per_sm(64)) return launch_f64_layout<1>(A, B, C, ldc, M, N, K, Mst, Nst, s, sc, split);
+    return launch_f64_layout<0>(A, B, C, ldc, M, N, K, Mst, Nst, s, sc, split);
 }
 
 }  // namespace iga

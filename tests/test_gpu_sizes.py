@@ -160,3 +160,51 @@ def test_seams(torch_cuda, ib, orc, p, nex, ney, ty, bc):
     g.replay()
     torch_cuda.cuda.synchronize()
     assert torch_cuda.equal(y3, yd)
+
+
+# The exact preconditioner's FP64 GEMM tiles: 32 x 32 (small and ragged sizes,
+# 700^2) and 64 x 64 (1022^2, whose half transforms give every SM two), one
+# tile and less, with and without the parity split; and the solver's loop on
+# it with and without a kappa scaling (r.z taken in the unfold or not).
+# K_fem z = r to 1e-10 as for every exact inverse.
+@pytest.mark.parametrize("p,nex,ney", [(2, 5, 9), (2, 31, 33), (3, 65, 200), (3, 700, 690), (3, 1021, 1021)])
+@pytest.mark.parametrize("split", [0, 1])
+def test_exact_preconditioner_tiles(torch_cuda, ib, orc, p, nex, ney, split):
+    plan = ib.Plan(ib.unit_square(p, nex, ney))
+    plan.set_pc_split(split)
+    gx, gy = plan.fem_nodes()
+    r = splitmix_uniform(p + nex, -1.0, 1.0, plan.nfunc)
+    rd = torch_cuda.from_numpy(r).cuda()
+    zd = torch_cuda.full_like(rd, float("nan"))
+    plan.pc_apply(rd, zd)
+    res = orc.fem_matvec(gx, gy, zd.cpu().numpy()) - r
+    assert np.linalg.norm(res) <= 1e-10 * np.linalg.norm(r)
+    if nex > 300:
+        plan.close()
+        return
+    # z = S M^-1 S r with S from kappa, through the same kernels (kappa = 4: S = 1/2)
+    kq = torch_cuda.full((nex * ney * (p + 1) ** 2,), 4.0, dtype=torch_cuda.float64, device="cuda")
+    plan.set_kappa(kq)
+    z2 = torch_cuda.full_like(rd, float("nan"))
+    plan.pc_apply(rd, z2)
+    assert rel(z2.cpu().numpy(), 0.25 * zd.cpu().numpy()) < 1e-12
+    plan.close()
+    plan = ib.Plan(ib.unit_square(p, nex, ney), precision=ib.MIXED)
+    plan.set_pc_split(split)
+    m, n = nex + p, ney + p
+    b = r.reshape(n, m).copy()
+    b[0], b[-1], b[:, 0], b[:, -1] = 0.0, 0.0, 0.0, 0.0
+    bd = torch_cuda.from_numpy(b.ravel()).cuda()
+    ref = None
+    for kappa in (False, True):
+        if kappa:
+            plan.set_kappa(kq)
+        for prec in (ib.FP64, ib.MIXED, ib.MIXED_PC):
+            x = torch_cuda.zeros_like(bd)
+            st = plan.solve(bd, x, precision=prec, pc=ib.PC_FEM_EXACT)
+            assert st.relres <= 1e-10
+            x = x.cpu().numpy() * (4.0 if kappa else 1.0)
+            ref = x if ref is None else ref
+            # K's condition times the residuals' 1e-10 bounds the difference; 1e-7 holds it with room
+            assert rel(x, ref) < 1e-7
+    plan.close()
