@@ -793,7 +793,24 @@ __global__ void __launch_bounds__(apply_max_threads<P, T, 0>(), 1)
         apply_load_tabs<P, T, 0, NST>(params[it.x].tabX, it.y, 1, apply_tab_slots<P, T, 0, NST>());
         __syncthreads();
     }
-    apply_tile<P, T, 0, NST>(params[it.x], xb + o, yb + o, it.y, flat ? it.z : it.z * blockDim.y + threadIdx.y, 0);
+    // The item's parameters where stores to y cannot make the compiler fetch
+    // them from global memory again at every element row: in FP32 registers
+    // (256 problems of p = 2, 3: 285 -> 243 us; in shared memory 288), in FP64
+    // and at p >= 4, whose registers are full, shared memory (FP64 403 -> 367;
+    // in registers 385).
+    const int gy = flat ? it.z : it.z * blockDim.y + threadIdx.y;
+    if constexpr (sizeof(T) == 4 && P <= 3) {
+        const ApplyParams<T> a = params[it.x];
+        apply_tile<P, T, 0, NST>(a, xb + o, yb + o, it.y, gy, 0);
+    } else {
+        constexpr int NI = (int)sizeof(ApplyParams<T>) / 8;
+        static_assert(sizeof(ApplyParams<T>) % 8 == 0, "copied in 8-byte words");
+        __shared__ long long sp[apply_max_threads<P, T, 0>() / 32][NI];
+        const long long *src = reinterpret_cast<const long long *>(params + it.x);
+        for (int i = threadIdx.x; i < NI; i += 32) sp[threadIdx.y][i] = src[i];
+        __syncwarp();
+        apply_tile<P, T, 0, NST>(*reinterpret_cast<const ApplyParams<T> *>(sp[threadIdx.y]), xb + o, yb + o, it.y, gy, 0);
+    }
 }
 
 // ------------------------------------------------------------ seams
@@ -910,7 +927,7 @@ __global__ void __launch_bounds__(kSeamBlock) seam_fixup_batch_kernel(const Appl
 {
     const int pr = blockIdx.y;
     if (!active[pr]) return;
-    const ApplyParams<T> &a = params[pr];
+    const ApplyParams<T> a = params[pr];   // a copy: see apply_batch_kernel
     const long long o = offs[pr];
     switch (a.g.P) {
     case 1: seam_loop<1, T>(a, xb + o, yb + o); break;

@@ -1646,6 +1646,17 @@ int setup_items(iga_batch *B, int pi)
                     for (int gx = 0; gx < g.NSX; ++gx) items.push_back(make_int4(i, gx, gyb, 0));
             }
         }
+        if (flat) {
+            // full strips first, the patches' shorter last ones at the end: the
+            // warps of a CTA walk equally long strips and the launch ends on
+            // short ones (256 problems, FP64 418 -> 403 us, FP32 294 -> 285)
+            auto steps = [&](const int4 &t) {
+                const StripGrid &g = (pi ? B->plans[t.x]->op32 : B->plans[t.x]->op64).grid;
+                return std::min(g.TY, g.ney - g.TY * t.z);
+            };
+            std::stable_sort(items.begin(), items.end(),
+                             [&](const int4 &x, const int4 &y) { return steps(x) > steps(y); });
+        }
         if (flat)
             while (items.size() % W) items.push_back(make_int4(-1, 0, 0, 0));   // whole CTAs
         G.nitems[pi] = (int)(flat ? items.size() / W : items.size());         // CTAs
