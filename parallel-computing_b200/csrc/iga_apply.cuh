@@ -32,6 +32,11 @@
 
 namespace iga {
 
+// Largest geometry streamed with policy_once(): past it there is nothing of the
+// stream to keep, and a MatMult alone was slower with it (p=3 2048^2 FP64, 1.6
+// GB, 298 -> 301 us; FP32, 0.8 GB, 157 -> 156 us).
+constexpr size_t kOnceBytes = size_t(1) << 30;
+
 template <typename T>
 struct ApplyParams {
     const T *x;
@@ -57,6 +62,8 @@ struct ApplyParams {
     const int *ID = nullptr;
     // Polls of each wait for a G stage before it reports IGA_ERR_TIMEOUT.
     long long wait_polls = kWaitLimit;
+    // G streamed with policy_once(): geometry up to kOnceBytes
+    int g_once = 1;
 };
 
 // Stores sign * v for control point i = R m + C under boundary rule bc
@@ -259,6 +266,13 @@ __device__ __forceinline__ void apply_tile(const ApplyParams<T> &a, const T *__r
     const int ex = ex0 + c;
     const T *Gstrip = GEOM == 0 ? a.G + (size_t)(gx * g.NSY + gy) * g.TY * S::GE : nullptr;
 
+    // The policy is held in registers, except where those two make the kernel
+    // spill more (FP32 p = 5, 800^2: 86 -> 93 us): made at each use there.
+    constexpr bool HOLD = !(sizeof(T) == 4 && P == 5);
+    const uint64_t pol = GEOM == 0 && HOLD ? (a.g_once ? policy_once() : policy_normal()) : 0;
+    auto fetch_g = [&](T *dst, const T *src, uint64_t *bar) {
+        bulk_g2s(dst, src, S::GBYTES, bar, HOLD ? pol : policy_once());
+    };
     if (GEOM == 0) {
         if (lane == 0) {
             for (int i = 0; i < NST; ++i) mbar_init(&wbar[i], 1);
@@ -268,7 +282,7 @@ __device__ __forceinline__ void apply_tile(const ApplyParams<T> &a, const T *__r
         if (lane == 0)
             for (int s = 0; s < NST && s < nsteps; ++s) {
                 mbar_arrive_expect_tx(&wbar[s], S::GBYTES);
-                bulk_g2s(Gs + (size_t)s * S::GE, Gstrip + (size_t)s * S::GE, S::GBYTES, &wbar[s]);
+                fetch_g(Gs + (size_t)s * S::GE, Gstrip + (size_t)s * S::GE, &wbar[s]);
             }
     }
 
@@ -714,7 +728,7 @@ __device__ __forceinline__ void apply_tile(const ApplyParams<T> &a, const T *__r
             if (lane == 0 && s + NST < nsteps) {
                 fence_proxy_async_smem();
                 mbar_arrive_expect_tx(&wbar[slot], S::GBYTES);
-                bulk_g2s(Gs + (size_t)slot * S::GE, Gstrip + (size_t)(s + NST) * S::GE, S::GBYTES, &wbar[slot]);
+                fetch_g(Gs + (size_t)slot * S::GE, Gstrip + (size_t)(s + NST) * S::GE, &wbar[slot]);
             }
         }
         write_row(s);
