@@ -821,12 +821,6 @@ static int tri_warps(int nyp, size_t esz, size_t &smem)
     return w;
 }
 
-// Interior block of r (m x n grid, x fastest) into a zero-padded nxp x nyp
-// column-major matrix (rows = x), and back: GEMM-friendly leading dimensions.
-// Each thread moves 16 bytes of the padded matrix (nxp is a multiple of 16);
-// blockIdx.y strides over the columns b, so no index division is needed. With
-// sc (FP64 vectors, FP32 transform) the gather divides by pc_scale and the
-// scatter multiplies by it.
 // Entry t of the boundary ring of the m x n grid (2 m + 2 (n - 2) entries).
 __device__ __forceinline__ long long ring_index(long long t, int m, int n)
 {
@@ -849,44 +843,52 @@ __device__ __forceinline__ void ring_copy(T *__restrict__ z, const T *__restrict
     }
 }
 
-// The gather also copies the boundary ring of r into z (one launch fewer) and
-// applies the kappa scaling ks (or null) on the way in.
-// With the parity split (kb > 0) column c of U is, for c < kb, the even fold
-// r[c] + r[nx-1-c] (c < fo; the middle entry r[fo] alone when nx is odd) and,
-// for c >= kb, the odd fold r[j] - r[nx-1-j] with j = c - kb < fo.
+// The exact inverse's gather and unfold move a row's 32 kFoldN columns per
+// warp and step, lane by lane, so that every access is a whole line although
+// the rows of r and z start anywhere, with kFoldN loads of each array in
+// flight per lane (bound: bytes; 2048^2 FP32: gather 15 -> 11 us against 16-byte
+// stores with scalar loads of their own, unfold 20.5 -> 9.4 us against one column).
+constexpr int kFoldN = 4;
+
+// Interior block of r (m x n grid, x fastest) into the zero-padded GEMM
+// operand U [nyp][nxp], and the boundary ring of r into z (one launch fewer),
+// both times the kappa scaling ks (or null). With sc (FP64 vectors, FP32
+// transform) the values are divided by pc_scale. With the parity split (kb >
+// 0) column c of U is, for c < kb, the even fold r[c] + r[nx-1-c] (c < fo; the
+// middle entry r[fo] alone when nx is odd) and, for c >= kb, the odd fold
+// r[j] - r[nx-1-j] with j = c - kb < fo.
 template <typename T, typename V>
-__global__ void fd_gather_kernel(const V *__restrict__ r, const V *__restrict__ ks, T *__restrict__ U, V *__restrict__ z,
-                                 int m, int n, int nx, int ny, int nxp, int nyp, int kb, int fo, const DevScalars *sc)
+__global__ void __launch_bounds__(kThreads)
+    fd_gather_kernel(const V *__restrict__ r, const V *__restrict__ ks, T *__restrict__ U, V *__restrict__ z, int m, int n,
+                     int nx, int ny, int nxp, int nyp, int kb, int fo, const DevScalars *sc)
 {
     pdl_begin();
-    ring_copy(z, r, ks, m, n, ((long long)blockIdx.y * gridDim.x + blockIdx.x) * blockDim.x + threadIdx.x,
-              (long long)gridDim.x * gridDim.y * blockDim.x);
-    constexpr int VN = Pk<T>::n;
+    ring_copy(z, r, ks, m, n, blockIdx.x * (long long)kThreads + threadIdx.x, (long long)gridDim.x * kThreads);
     const double inv = sc ? 1.0 / pc_scale(sc) : 1.0;
-    const int nv = nxp / VN;
-    for (int b = blockIdx.y; b < nyp; b += gridDim.y) {
-        const V *rb = r + (size_t)(b + 1) * m + 1;
-        const V *kr = ks ? ks + (size_t)(b + 1) * m + 1 : nullptr;
-        auto at = [&](int i) { return kr ? (double)(V)(rb[i] * kr[i]) : (double)rb[i]; };
-        for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < nv; k += gridDim.x * blockDim.x) {
-            Pk<T> o;
+    const int lane = threadIdx.x & 31, half = kb > 0 ? kb : nxp, cb = (half + 32 * kFoldN - 1) / (32 * kFoldN);
+    const int w0 = blockIdx.x * (kThreads / 32) + (threadIdx.x >> 5), ws = gridDim.x * (kThreads / 32);
+    for (long long u = w0; u < (long long)cb * nyp; u += ws) {
+        const int b = (int)(u / cb), a0 = (int)(u - (long long)b * cb) * 32 * kFoldN + lane;
+        const size_t o = (size_t)(b + 1) * m + 1;
+        V f[kFoldN], g[kFoldN];
 #pragma unroll
-            for (int c = 0; c < VN; ++c) {
-                const int a = k * VN + c;
-                double v = 0.0;
-                if (b < ny) {
-                    if (kb == 0) {
-                        if (a < nx) v = at(a);
-                    } else if (a < kb) {
-                        if (a < fo) v = at(a) + at(nx - 1 - a);
-                        else if (a == fo && (nx & 1)) v = at(a);
-                    } else if (a - kb < fo) {
-                        v = at(a - kb) - at(nx - 1 - (a - kb));
-                    }
-                }
-                o.v[c] = (T)(v * inv);
+        for (int k = 0; k < kFoldN; ++k) {
+            const int a = a0 + 32 * k, e = nx - 1 - a;
+            // kb > 0: a pairs with e for a < fo; the middle entry (odd nx) has none
+            f[k] = b < ny && (kb > 0 ? a < nx - fo : a < nx) ? r[o + a] : V(0);
+            g[k] = b < ny && kb > 0 && a < fo ? r[o + e] : V(0);
+            if (ks) {
+                if (b < ny && (kb > 0 ? a < nx - fo : a < nx)) f[k] *= ks[o + a];
+                if (b < ny && kb > 0 && a < fo) g[k] *= ks[o + e];
             }
-            stp(U, (long long)b * nxp + (long long)k * VN, o);
+        }
+        T *ub = U + (size_t)b * nxp;
+#pragma unroll
+        for (int k = 0; k < kFoldN; ++k) {
+            const int a = a0 + 32 * k;
+            if (a >= half) continue;
+            ub[a] = (T)(((double)f[k] + (double)g[k]) * inv);
+            if (kb > 0 && kb + a < nxp) ub[kb + a] = (T)((a < fo ? (double)f[k] - (double)g[k] : 0.0) * inv);
         }
     }
 }
@@ -897,8 +899,7 @@ __global__ void fd_gather_kernel(const V *__restrict__ r, const V *__restrict__ 
 // entry z[fo] = Ze[fo] when nx is odd; times sqrt(*rr) when rr is set and times
 // the kappa scaling ks (or null). With part it also takes the solver's next
 // dot product, r . z over the whole grid, as block partials while z is in
-// registers (one launch and two passes fewer an iteration). A warp takes 32
-// columns of one row at a time.
+// registers (one launch and two passes fewer an iteration).
 template <typename T, typename V>
 __global__ void __launch_bounds__(kThreads)
     fd_unfold_kernel(const T *__restrict__ W, const V *__restrict__ r, const V *__restrict__ ks, V *__restrict__ z, int m,
@@ -910,28 +911,42 @@ __global__ void __launch_bounds__(kThreads)
         const double v = *rr;
         f = (v > 0.0 && v < 1e300) ? sqrt(v) : 1.0;
     }
-    const int lane = threadIdx.x & 31, cb = (fe + 31) / 32;
+    const int lane = threadIdx.x & 31, cb = (fe + 32 * kFoldN - 1) / (32 * kFoldN);
     const int w0 = blockIdx.x * (kThreads / 32) + (threadIdx.x >> 5), ws = gridDim.x * (kThreads / 32);
     double dot = 0.0;
     for (long long u = w0; u < (long long)cb * ny; u += ws) {
-        const int b = (int)(u / cb), j = (int)(u - (long long)b * cb) * 32 + lane;
-        if (j >= fe) continue;
+        const int b = (int)(u / cb), j0 = (int)(u - (long long)b * cb) * 32 * kFoldN + lane;
         const T *wb = W + (size_t)b * nxp;
-        const size_t o = (size_t)(b + 1) * m + 1, i0 = o + j, i1 = o + (nx - 1 - j);
-        const double e = (double)wb[j];
-        V z0 = (V)(f * e), z1 = V(0);
-        if (j < fo) {
-            const double d = (double)wb[kb + j];
-            z0 = (V)(f * (e + d));
-            z1 = (V)(f * (e - d));
-            if (ks) z1 *= ks[i1];
-            z[i1] = z1;
+        const size_t o = (size_t)(b + 1) * m + 1;
+        T e[kFoldN], d[kFoldN];
+        V r0[kFoldN], r1[kFoldN], k0[kFoldN], k1[kFoldN];
+#pragma unroll
+        for (int k = 0; k < kFoldN; ++k) {
+            const int j = j0 + 32 * k, jm = nx - 1 - j;
+            e[k] = j < fe ? wb[j] : T(0);
+            d[k] = j < fo ? wb[kb + j] : T(0);
+            if (part) {
+                r0[k] = j < fe ? r[o + j] : V(0);
+                r1[k] = j < fo ? r[o + jm] : V(0);
+            }
+            if (ks) {
+                k0[k] = j < fe ? ks[o + j] : V(0);
+                k1[k] = j < fo ? ks[o + jm] : V(0);
+            }
         }
-        if (ks) z0 *= ks[i0];
-        z[i0] = z0;
-        if (part) {
-            dot += (double)r[i0] * (double)z0;
-            if (j < fo) dot += (double)r[i1] * (double)z1;
+#pragma unroll
+        for (int k = 0; k < kFoldN; ++k) {
+            const int j = j0 + 32 * k;
+            if (j >= fe) continue;
+            V z0 = (V)(f * ((double)e[k] + (double)d[k]));
+            if (ks) z0 *= k0[k];
+            z[o + j] = z0;
+            if (part) dot += (double)r0[k] * (double)z0;
+            if (j >= fo) continue;   // the middle entry (d = 0)
+            V z1 = (V)(f * ((double)e[k] - (double)d[k]));
+            if (ks) z1 *= k1[k];
+            z[o + nx - 1 - j] = z1;
+            if (part) dot += (double)r1[k] * (double)z1;
         }
     }
     if (!part) return;
@@ -942,16 +957,6 @@ __global__ void __launch_bounds__(kThreads)
         dot += (double)rv * (double)zv;
     }
     put_partial(dot, part);
-}
-
-// 2-D launch of the gather: 128-thread blocks over the groups of a
-// row, block rows striding over the rows. About one wave of blocks (16 per
-// SM): one block per row made it block-launch bound.
-static dim3 grid2d(int ngroups, int nrows, int nsm)
-{
-    const int gx = std::max(1, (ngroups + 127) / 128);
-    const int gy = std::max(1, std::min({nrows, 65535, std::max(1, 16 * nsm / gx)}));
-    return dim3((unsigned)gx, (unsigned)gy);
 }
 
 // z = r on the boundary ring (identity rows of K_fem).
@@ -1564,9 +1569,13 @@ static int fd_apply(PrecState<T> &ps, const iga_plan *pl, SolverState *S, const 
     const int nxp = ps.nxp, nyp = ps.nyp;
     int seg = (ny + 31) / 32;
     seg |= 1;   // odd: conflict-free shared-memory rows
-    constexpr int VN = Pk<T>::n;
-    SOLVE_TRY(launch_k(fd_gather_kernel<T, V>, grid2d(nxp / VN, nyp, ps.nsm), dim3(128), 0, S->stream, r, ks, ps.W2, z, m, n, nx, ny,
-                       nxp, nyp, ps.kb, ps.fo, sc));
+    // warp steps of `cols` columns by `rows` rows, in at most `most` blocks
+    auto blocks = [](int cols, int rows, int most) {
+        const long long steps = (long long)((cols + 32 * kFoldN - 1) / (32 * kFoldN)) * rows;
+        return (int)std::max(1LL, std::min<long long>(most, (steps + kThreads / 32 - 1) / (kThreads / 32)));
+    };
+    SOLVE_TRY(launch_k(fd_gather_kernel<T, V>, dim3(blocks(ps.kb > 0 ? ps.kb : nxp, nyp, 8 * ps.nsm)), dim3(kThreads), 0,
+                       S->stream, r, ks, ps.W2, z, m, n, nx, ny, nxp, nyp, ps.kb, ps.fo, sc));
     // the gather follows whatever the stream holds (a wait for the caller's
     // stream, say); its successors follow this call's own kernels
     struct Chain {
@@ -1594,12 +1603,11 @@ static int fd_apply(PrecState<T> &ps, const iga_plan *pl, SolverState *S, const 
             // unfold kernel combines them into z's interior
             e = transform_gemm(ps, pl, 2, S->stream);
             if (e == IGA_OK) {
-                const long long items = (long long)((ps.fe + 31) / 32) * ny;
-                const int blocks = (int)std::max(1LL, std::min<long long>(kRedBlocks, (items + 7) / 8));
-                SOLVE_TRY(launch_k(fd_unfold_kernel<T, V>, dim3(blocks), dim3(kThreads), 0, S->stream,
+                const int nu = blocks(ps.fe, ny, kRedBlocks);
+                SOLVE_TRY(launch_k(fd_unfold_kernel<T, V>, dim3(nu), dim3(kThreads), 0, S->stream,
                                    (const T *)ps.W2, r, ks, z, m, n, nx, ny, nxp, ps.kb, ps.fe, ps.fo,
                                    sc ? &sc->rr : (const double *)nullptr, rz ? rz->part : (double *)nullptr));
-                if (rz) rz->n = blocks;
+                if (rz) rz->n = nu;
             }
         } else {
             // the second GEMM's epilogue writes z's interior itself
