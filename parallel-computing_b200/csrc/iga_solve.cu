@@ -680,15 +680,19 @@ __global__ void from_fp32_kernel(const float *__restrict__ z32, double *__restri
 // (the unit lower factor's subdiagonal, Lf_0 = 0) and Dv_b = 1 / d_b, so
 //   forward  u_b = w_b - Lf_b u_{b-1},       v_b = Dv_b u_b,
 //   backward x_b = v_b - Lf_{b+1} x_{b+1}    (no term past the last free row).
-// One warp per mode: lane l owns rows [l s, l s + s) with s odd, so that the
-// lanes' shared-memory accesses fall in distinct banks. Each recurrence is
-// composed per lane into an affine map c -> E + P c, the maps are combined by
-// a warp shuffle scan, and each lane then runs its rows from its carry-in.
-// Arithmetic in T. STAGED: the mode's column and factors are brought into
-// shared memory by the bulk-copy engine and the result is written back with
-// 16-byte stores; else (columns too long for shared memory) the kernel works
-// on them in place.
-constexpr int kTriMaxWarps = 16;
+// One CTA of NW warps per mode: thread t owns rows [t s, t s + s) with s odd,
+// so that a warp's shared-memory accesses fall in distinct banks. Each
+// recurrence is composed per thread into an affine map c -> E + P c, the maps
+// are combined by a warp shuffle scan and across the warps through shared
+// memory, and each thread then runs its rows from its carry-in. Arithmetic in
+// T. STAGED: the mode's column and factors are brought into shared memory by
+// the bulk-copy engine and the result is written back with 16-byte stores;
+// else (columns too long for shared memory) the kernel works on them in place.
+// Bound: the recurrences' latency, then bytes. A warp per mode with all of an
+// SM's modes in one CTA had every warp load, then solve, then store at the
+// same time (2048^2: FP32 25 us, FP64 50 us; two buffers per warp, half the
+// warps: 30 and 67 us); CTAs of their own overlap these phases, and four warps
+// shorten the chains: 17 and 31 us.
 
 // inclusive scan of affine maps over lanes, lane order (forward) or reverse lane order
 template <typename R>
@@ -705,120 +709,128 @@ __device__ __forceinline__ void affine_scan(R &E, R &P, int lane, bool reverse)
     }
 }
 
-template <typename T, bool STAGED>
-__global__ void __launch_bounds__(kTriMaxWarps * 32)
-fd_tri_kernel(T *__restrict__ W, const T *__restrict__ Lf, const T *__restrict__ Dv, int nx, int ny, int nyp, int seg,
+template <typename T, bool STAGED, int NW>
+__global__ void __launch_bounds__(NW * 32)
+fd_tri_kernel(T *__restrict__ W, const T *__restrict__ Lf, const T *__restrict__ Dv, int ny, int nyp, int seg,
               DevScalars *sc)
 {
     pdl_launch();
     extern __shared__ __align__(16) unsigned char tri_smem[];
-    __shared__ uint64_t bar[kTriMaxWarps];
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
-    T *wb = nullptr, *lb = nullptr, *db = nullptr;
-    if constexpr (STAGED) {
-        wb = reinterpret_cast<T *>(tri_smem) + (size_t)wid * 3 * nyp;
-        lb = wb + nyp;
-        db = lb + nyp;
-        if (lane == 0) mbar_init(&bar[wid], 1);
-        fence_mbar_init();
-        __syncwarp();
-    }
-    uint32_t phase = 0;
-    const int b0 = lane * seg, b1 = min(b0 + seg, ny);
+    __shared__ uint64_t bar;
+    __shared__ T fE[NW], fP[NW], rE[NW], rP[NW];   // the warps' maps, forward and backward
+    const int t = threadIdx.x, lane = t & 31, wid = t >> 5;
+    const size_t a = blockIdx.x;
+    T *wg = W + a * nyp, *wp = wg;
+    const T *lp = Lf + a * nyp, *dp = Dv + a * nyp;
     const uint32_t bytes = (uint32_t)nyp * (uint32_t)sizeof(T);
-    const int a0 = blockIdx.x * nw + wid;
-    // the first mode's factors (constant) are requested before the wait for
-    // the preceding grid, its column of W after it
-    if (STAGED && lane == 0 && a0 < nx) {
-        mbar_arrive_expect_tx(&bar[wid], 3u * bytes);
-        bulk_g2s(lb, Lf + (size_t)a0 * nyp, bytes, &bar[wid]);
-        bulk_g2s(db, Dv + (size_t)a0 * nyp, bytes, &bar[wid]);
+    if constexpr (STAGED) {
+        T *wb = reinterpret_cast<T *>(tri_smem);
+        if (t == 0) {   // the factors (constant) before the wait for the preceding grid, the column after it
+            mbar_init(&bar, 1);
+            fence_mbar_init();
+            mbar_arrive_expect_tx(&bar, 3u * bytes);
+            bulk_g2s(wb + nyp, lp, bytes, &bar);
+            bulk_g2s(wb + 2 * nyp, dp, bytes, &bar);
+        }
+        wp = wb;
+        lp = wb + nyp;
+        dp = wb + 2 * nyp;
     }
     pdl_wait();
-    for (int a = a0; a < nx; a += gridDim.x * nw) {
-        T *wg = W + (size_t)a * nyp;
-        const T *lg = Lf + (size_t)a * nyp, *dg = Dv + (size_t)a * nyp;
-        T *wp;
-        const T *lp, *dp;
-        if constexpr (STAGED) {
-            if (lane == 0) {
-                if (a != a0) {
-                    mbar_arrive_expect_tx(&bar[wid], 3u * bytes);
-                    bulk_g2s(lb, lg, bytes, &bar[wid]);
-                    bulk_g2s(db, dg, bytes, &bar[wid]);
-                }
-                bulk_g2s(wb, wg, bytes, &bar[wid]);
-            }
-            if (!mbar_wait_bounded(&bar[wid], phase)) {
-                if (lane == 0) sc->err = 1;
-                mbar_wait_bounded(&bar[wid], phase);   // let the copies land before leaving
-                return;
-            }
-            phase ^= 1u;
-            wp = wb;
-            lp = lb;
-            dp = db;
-        } else {
-            wp = wg;
-            lp = lg;
-            dp = dg;
+    if constexpr (STAGED) {
+        if (t == 0) bulk_g2s(wp, wg, bytes, &bar);
+        __syncthreads();   // the barrier is set up
+        if (!__syncthreads_and(mbar_wait_bounded(&bar, 0))) {
+            if (t == 0) sc->err = 1;
+            mbar_wait_bounded(&bar, 0);   // let the copies land before leaving
+            return;
         }
-        // forward: this lane's map, the scan, then its rows from the carry-in
-        T E = 0, P = 1;
+    }
+    const int b0 = t * seg, b1 = min(b0 + seg, ny);
+    // forward: this thread's map, the scan, then its rows from the carry-in
+    T E = 0, P = 1;
 #pragma unroll 4
-        for (int b = b0; b < b1; ++b) {
-            const T l = lp[b];
-            E = wp[b] - l * E;
-            P = -l * P;
+    for (int b = b0; b < b1; ++b) {
+        const T l = lp[b];
+        E = wp[b] - l * E;
+        P = -l * P;
+    }
+    affine_scan(E, P, lane, false);
+    T c = 0;   // the carry into this warp
+    if constexpr (NW > 1) {
+        if (lane == 31) {
+            fE[wid] = E;
+            fP[wid] = P;
         }
-        affine_scan(E, P, lane, false);
-        T u = __shfl_up_sync(0xffffffffu, E, 1);
-        if (lane == 0) u = 0;
+        __syncthreads();
+        for (int w = 0; w < wid; ++w) c = fE[w] + fP[w] * c;
+    }
+    const T pe = __shfl_up_sync(0xffffffffu, E, 1), pp = __shfl_up_sync(0xffffffffu, P, 1);
+    T u = lane == 0 ? c : pe + pp * c;
 #pragma unroll 4
-        for (int b = b0; b < b1; ++b) {
-            u = wp[b] - lp[b] * u;
-            wp[b] = u * dp[b];
-        }
-        __syncwarp();
-        // backward over the same rows, lanes in reverse order
-        E = 0;
-        P = 1;
+    for (int b = b0; b < b1; ++b) {
+        u = wp[b] - lp[b] * u;
+        wp[b] = u * dp[b];
+    }
+    // backward over the same rows, threads in reverse order
+    E = 0;
+    P = 1;
 #pragma unroll 4
-        for (int b = b1 - 1; b >= b0; --b) {
-            const T l = b + 1 < ny ? lp[b + 1] : T(0);
-            E = wp[b] - l * E;
-            P = -l * P;
+    for (int b = b1 - 1; b >= b0; --b) {
+        const T l = b + 1 < ny ? lp[b + 1] : T(0);
+        E = wp[b] - l * E;
+        P = -l * P;
+    }
+    affine_scan(E, P, lane, true);
+    c = 0;
+    if constexpr (NW > 1) {
+        if (lane == 0) {
+            rE[wid] = E;
+            rP[wid] = P;
         }
-        affine_scan(E, P, lane, true);
-        T x = __shfl_down_sync(0xffffffffu, E, 1);
-        if (lane == 31) x = 0;
+        __syncthreads();
+        for (int w = NW - 1; w > wid; --w) c = rE[w] + rP[w] * c;
+    }
+    const T ne = __shfl_down_sync(0xffffffffu, E, 1), np = __shfl_down_sync(0xffffffffu, P, 1);
+    T x = lane == 31 ? c : ne + np * c;
 #pragma unroll 4
-        for (int b = b1 - 1; b >= b0; --b) {
-            const T l = b + 1 < ny ? lp[b + 1] : T(0);
-            x = wp[b] - l * x;
-            wp[b] = x;
-        }
-        if constexpr (STAGED) {
-            __syncwarp();
-            const int nv = (int)((size_t)nyp * sizeof(T) / 16);
-            const uint4 *src = reinterpret_cast<const uint4 *>(wb);
-            uint4 *dst = reinterpret_cast<uint4 *>(wg);
-            for (int i = lane; i < nv; i += 32) dst[i] = src[i];
-            fence_proxy_async_smem();   // order these generic accesses before the next bulk copy
-            __syncwarp();
-        }
+    for (int b = b1 - 1; b >= b0; --b) {
+        const T l = b + 1 < ny ? lp[b + 1] : T(0);
+        x = wp[b] - l * x;
+        wp[b] = x;
+    }
+    if constexpr (STAGED) {
+        __syncthreads();
+        const int nv = (int)((size_t)nyp * sizeof(T) / 16);
+        const uint4 *src = reinterpret_cast<const uint4 *>(wp);
+        uint4 *dst = reinterpret_cast<uint4 *>(wg);
+        for (int i = t; i < nv; i += NW * 32) dst[i] = src[i];
     }
 }
 
-// Launch shape of fd_tri_kernel for columns of nyp entries of T: warps per
-// CTA of the staged kernel (0 when a column and its factors do not fit in
-// shared memory) and its dynamic shared memory.
-static int tri_warps(int nyp, size_t esz, size_t &smem)
+// Warps per mode: enough that a thread has few rows, no more than keep most
+// threads busy.
+constexpr int tri_warps(int ny) { return ny <= 96 ? 1 : ny <= 384 ? 2 : 4; }
+constexpr size_t kTriSmem = 226 * 1024;   // most shared memory of a staged mode (leaves room for the static part)
+
+template <typename T, int NW>
+static cudaError_t launch_tri(T *W, const T *Lf, const T *Dv, int nmodes, int ny, int nyp, cudaStream_t s, DevScalars *sc)
 {
-    const size_t per_warp = 3 * (size_t)nyp * esz, cap = 226 * 1024;   // leaves room for the static barriers
-    const int w = (int)std::min<size_t>(kTriMaxWarps, cap / per_warp);
-    smem = (size_t)w * per_warp;
-    return w;
+    const size_t smem = 3 * (size_t)nyp * sizeof(T);
+    int seg = (ny + 32 * NW - 1) / (32 * NW);
+    seg |= 1;   // odd: conflict-free shared-memory rows
+    if (smem > kTriSmem)
+        return launch_k(fd_tri_kernel<T, false, NW>, dim3(nmodes), dim3(NW * 32), 0, s, W, Lf, Dv, ny, nyp, seg, sc);
+    return launch_k(fd_tri_kernel<T, true, NW>, dim3(nmodes), dim3(NW * 32), smem, s, W, Lf, Dv, ny, nyp, seg, sc);
+}
+
+template <typename T>
+static cudaError_t tri_prepare()   // the staged kernels' shared-memory limit
+{
+    cudaError_t e = cudaSuccess;
+    for (auto k : {fd_tri_kernel<T, true, 1>, fd_tri_kernel<T, true, 2>, fd_tri_kernel<T, true, 4>})
+        if (e == cudaSuccess) e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTriSmem);
+    return e;
 }
 
 // Entry t of the boundary ring of the m x n grid (2 m + 2 (n - 2) entries).
@@ -1048,8 +1060,6 @@ struct PrecState {
     // nmodes = rows of the mode-major work matrix the y solves walk
     int kb = 0, fe = 0, fo = 0, nmodes = 0;
     GemmTF32 g1, g2;        // FP32: the two transforms' prepared tensor-core GEMMs
-    int tri_w = 0;          // most warps per CTA of the staged tridiagonal kernel (0: in place)
-    size_t tri_smem = 0;    // its shared memory at tri_w warps
     int nsm = 148;          // SMs of the plan's device
     // device-side PCG loop: a CUDA graph whose conditional WHILE node runs one
     // iteration per pass (built for one preconditioner / kappa-scaling choice)
@@ -1500,11 +1510,8 @@ static int fd_upload(PrecState<T> &ps, const iga_plan *pl, SolverState *S)
     if ((st = up_mat(&ps.Vx)) || (st = up_vec(&ps.lx, S->lamx, nxp)) || (st = up_fac(&ps.Dv, S->Dv)) ||
         (st = up_fac(&ps.Lf, S->Lf)))
         return st;
-    ps.tri_w = tri_warps(nyp, sizeof(T), ps.tri_smem);
     SOLVE_TRY(cudaDeviceGetAttribute(&ps.nsm, cudaDevAttrMultiProcessorCount, pl->device));
-    if (ps.tri_w)
-        SOLVE_TRY(cudaFuncSetAttribute(fd_tri_kernel<T, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       (int)ps.tri_smem));
+    SOLVE_TRY(tri_prepare<T>());
     SOLVE_TRY(cudaMalloc((void **)&ps.W1, sizeof(T) * (size_t)nxp * nyp));
     SOLVE_TRY(cudaMalloc((void **)&ps.W2, sizeof(T) * (size_t)nxp * nyp));
     return prepare_gemms(ps);
@@ -1567,8 +1574,6 @@ static int fd_apply(PrecState<T> &ps, const iga_plan *pl, SolverState *S, const 
         return IGA_OK;
     }
     const int nxp = ps.nxp, nyp = ps.nyp;
-    int seg = (ny + 31) / 32;
-    seg |= 1;   // odd: conflict-free shared-memory rows
     // warp steps of `cols` columns by `rows` rows, in at most `most` blocks
     auto blocks = [](int cols, int rows, int most) {
         const long long steps = (long long)((cols + 32 * kFoldN - 1) / (32 * kFoldN)) * rows;
@@ -1585,18 +1590,11 @@ static int fd_apply(PrecState<T> &ps, const iga_plan *pl, SolverState *S, const 
     if (S->pc_chain) pdl_capture() = true;
     int e = transform_gemm(ps, pl, 1, S->stream);
     if (e == IGA_OK) {
-        if (ps.tri_w) {
-            // one mode per warp as long as the modes reach every SM, else the most
-            // warps per CTA that shared memory allows (warps then loop over modes)
-            const int nm = ps.nmodes;
-            const int w = std::max(1, std::min(ps.tri_w, (nm + ps.nsm - 1) / ps.nsm));
-            const int grid = std::min((nm + w - 1) / w, ps.nsm);
-            const size_t smem = ps.tri_smem / ps.tri_w * w;
-            SOLVE_TRY(launch_k(fd_tri_kernel<T, true>, dim3(grid), dim3(w * 32), smem, S->stream, ps.W1,
-                               (const T *)ps.Lf, (const T *)ps.Dv, nm, ny, nyp, seg, S->s));
-        } else {
-            SOLVE_TRY(launch_k(fd_tri_kernel<T, false>, dim3((ps.nmodes + 7) / 8), dim3(256), 0, S->stream, ps.W1,
-                               (const T *)ps.Lf, (const T *)ps.Dv, ps.nmodes, ny, nyp, seg, S->s));
+        const T *lf = ps.Lf, *dv = ps.Dv;
+        switch (tri_warps(ny)) {
+        case 1: SOLVE_TRY((launch_tri<T, 1>(ps.W1, lf, dv, ps.nmodes, ny, nyp, S->stream, S->s))); break;
+        case 2: SOLVE_TRY((launch_tri<T, 2>(ps.W1, lf, dv, ps.nmodes, ny, nyp, S->stream, S->s))); break;
+        default: SOLVE_TRY((launch_tri<T, 4>(ps.W1, lf, dv, ps.nmodes, ny, nyp, S->stream, S->s))); break;
         }
         if (ps.kb > 0) {
             // parity split: the second GEMM writes both halves' products, the
