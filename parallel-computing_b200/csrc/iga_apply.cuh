@@ -110,55 +110,67 @@ __host__ __device__ constexpr int apply_stages()
                                                  : (12288 / ApplyShape<P, T>::GBYTES > 8 ? 8 : 12288 / ApplyShape<P, T>::GBYTES);
 }
 
+// Warps that share a strip. One, except for the FP64 on-the-fly kernels of p >=
+// 4, whose state (u's and both coordinates' contracted rows for every
+// quadrature column of a lane, 120 doubles at p = 4) did not fit the 255
+// registers a thread can have and spilled. There each of K = ceil(NQ / 2) = 3
+// warps takes two quadrature columns of the strip, one per lane: a third of
+// the state, and 12 instead of 8 warps per SM. The warps run independently
+// but for one exchange per finished row, where warp 0 adds the others' sums,
+// in order. Measured (MatMult): p=5 800^2 470 -> 240 us, 512^2 227 -> 105, p=4
+// 1024^2 288 -> 266, 512^2 80 -> 74. At p = 2, 3, which do not spill, the rows'
+// work that every warp repeats costs more than the warps gain (p=3 1024^2 127
+// -> 142 us without a spill, p=2 94 -> 96).
+template <int P, typename T, int GEOM>
+__host__ __device__ constexpr int apply_split()
+{
+    return GEOM == 1 && sizeof(T) == 8 && P >= 4 ? (P + 2) / 2 : 1;
+}
+
 // Whether a lane keeps its x-direction tables in registers (16 values at
 // p = 3) or reads them from shared memory: registers except where they are
-// the scarcer resource (FP64 p >= 4, FP64 on-the-fly geometry at p <= 2). In
+// the scarcer resource (FP64 precomputed p >= 4, FP64 on-the-fly p <= 2). In
 // registers they save 32 shared loads per element row of a p=3 FP64 strip
 // (12 instead of 13 warps per SM: 1.12x faster), and the warps of a CTA need
 // not share a column strip, so strips are dealt to warps one by one and every
 // SM gets work. The FP64 on-the-fly kernel at p = 3 keeps them in registers
-// at 8 warps per SM (244 registers, no spills; shared tables: 10 warps with
+// at 8 warps per SM (254 registers, no spills; shared tables: 10 warps with
 // spills): 2048^2 673 -> 536 us, 1024^2 208 -> 149 us. At p = 2 the same
 // change was slower (2048^2 392 -> 435 us).
 template <int P, typename T, int GEOM>
 __host__ __device__ constexpr bool apply_txreg()
 {
-    return sizeof(T) == 4 || (GEOM == 0 ? P <= 3 : P == 3);
+    return sizeof(T) == 4 || apply_split<P, T, GEOM>() > 1 || (GEOM == 0 ? P <= 3 : P == 3);
 }
 
-// Where the tables are not in registers they are either copied to shared
-// memory by a CTA that takes W strips of one column strip, or read by each
-// lane straight from global memory (its own entries, L1-resident: a strip's
-// tables are a few KB reused for every element row), which lets the kernel
-// deal strips to warps one by one and fill the SMs. Measured (B200, warm):
-// FP64 p=4 on-the-fly 1024^2 333 -> 302 us from global memory; FP64 p=4
-// precomputed 152.6 -> 164.8 us and p=5 (both geometry modes) 249 -> 278 /
-// 726 -> 890 us slower that way, so shared memory everywhere else.
+// Where the tables are not in registers they are copied to shared memory by a
+// CTA whose strips lie in at most two column strips. (Read by each lane from
+// global memory instead: FP64 p=4 precomputed 152.6 -> 164.8 us, p=5 249 -> 278
+// us at 1024^2.)
 template <int P, typename T, int GEOM>
 __host__ __device__ constexpr bool apply_txshared()
 {
-    return !apply_txreg<P, T, GEOM>() && !(GEOM == 1 && P == 4);
-}
-
-// The FP64 on-the-fly kernel at p = 5 (255 registers, spilling) keeps one
-// CTA per column strip: dealt from the flat grid its spills grew (608 ->
-// 880 B a thread) and it ran 187 -> 255 us at 512^2.
-template <int P, typename T, int GEOM>
-__host__ __device__ constexpr bool apply_percolumn()
-{
-    return apply_txshared<P, T, GEOM>() && GEOM == 1 && P == 5;
+    return !apply_txreg<P, T, GEOM>();
 }
 
 // Shared memory of a CTA of W warps: barriers, then each warp's G ring, x
-// (and control-point) rows and y-table rows, then (apply_txshared) ntab
+// (and control-point) rows and y-table rows, then (apply_split) the strips'
+// exchange slots, two rows of K - 1 warps' values, then (apply_txshared) ntab
 // slots of column-strip x tables, 128-byte aligned.
+template <int P, typename T, int GEOM>
+__host__ __device__ constexpr size_t apply_exchange(int W)
+{
+    constexpr int K = apply_split<P, T, GEOM>();
+    return (size_t)(W / K) * 2 * (K - 1) * 32 * sizeof(T);
+}
+
 template <int P, typename T, int GEOM, int NST>
 __host__ __device__ constexpr size_t apply_tab_offset(int W)
 {
     using S = ApplyShape<P, T>;
     return (((256 + (size_t)W * NST * 8 + 127) & ~size_t(127)) + (GEOM == 0 ? (size_t)W * NST * S::GBYTES : 0) +
             (size_t)W * S::XR * S::XW * sizeof(T) * (GEOM == 1 ? 3 : 1) + (size_t)W * S::XR * S::TYW * sizeof(T) +
-            127) &
+            apply_exchange<P, T, GEOM>(W) + 127) &
            ~size_t(127);
 }
 
@@ -222,27 +234,30 @@ __device__ __forceinline__ float recip<float>(float v) { return __frcp_rn(v); }
 // Threads per CTA the register budget allows (one CTA per SM): the kernel's
 // per-thread state grows with p and doubles in FP64. FP64 precomputed p >= 4
 // runs 8 warps without register spills (at 10 warps it spilled and ran 1.8x
-// slower at p = 4); the FP64 on-the-fly kernels at p >= 4 need more than the
-// 255 registers a thread can have and spill at any bound.
+// slower at p = 4), and p = 1 on the fly 16 (12: 1024^2 41 -> 37 us).
 template <int P, typename T, int GEOM>
 __host__ __device__ constexpr int apply_max_threads()
 {
     return sizeof(T) == 4 ? (P <= 3 ? 512 : (GEOM ? 384 : 512))
-                          : (P <= 2 ? (GEOM ? 384 : 512) : P == 3 ? (GEOM ? 256 : 384) : 256);
+           : GEOM         ? (P == 1 ? 512 : P == 3 ? 256 : 384)
+                          : (P <= 2 ? 512 : P == 3 ? 384 : 256);
 }
 
-// One warp: strip (gx, gy). tab_slot: the slot of the CTA's shared memory
+// One warp: strip (gx, gy), or its share of it (apply_split: quadrature columns
+// 2 k and 2 k + 1 for warp k = threadIdx.y % K). tab_slot: the slot of the CTA's shared memory
 // holding the column strip's x tables (apply_txshared), loaded by the caller.
 template <int P, typename T, int GEOM, int NST>
 __device__ __forceinline__ void apply_tile(const ApplyParams<T> &a, const T *__restrict__ x, T *__restrict__ y, const int gx,
                                            const int gy, const int tab_slot)
 {
     using S = ApplyShape<P, T>;
-    constexpr int NB = S::NB, NQ = S::NQ, QH = S::QH;
+    constexpr int K = apply_split<P, T, GEOM>();
+    constexpr int NB = S::NB, NQ = S::NQ, QH = K > 1 ? 1 : S::QH;   // QH: quadrature columns of a lane
     constexpr bool TXREG = apply_txreg<P, T, GEOM>();
     const StripGrid &g = a.g;
     const int lane = threadIdx.x, w = threadIdx.y, W = blockDim.y;
     const int c = lane >> 1, h = lane & 1;
+    const int kw = K > 1 ? w % K : 0;
 
     extern __shared__ __align__(128) unsigned char smem[];
     uint64_t *bars = reinterpret_cast<uint64_t *>(smem);
@@ -255,6 +270,8 @@ __device__ __forceinline__ void apply_tile(const ApplyParams<T> &a, const T *__r
     T *cr = reinterpret_cast<T *>(smem + off) + (size_t)w * S::XR * S::XW * 2;   // GEOM 1: CP rows (x, y)
     if (GEOM == 1) off += (size_t)W * S::XR * S::XW * 2 * sizeof(T);
     T *yr = reinterpret_cast<T *>(smem + off) + (size_t)w * S::XR * S::TYW;     // y tables of upcoming rows
+    off += (size_t)W * S::XR * S::TYW * sizeof(T);
+    T *xch = reinterpret_cast<T *>(smem + off) + (size_t)(w / K) * 2 * (K - 1) * 32;   // apply_split: exchange slots
     uint64_t *wbar = bars + w * NST;
     // (addressed from the shared array itself, so that the compiler emits shared loads)
     const T *tabXs = reinterpret_cast<const T *>(smem + apply_tab_offset<P, T, GEOM, NST>(W)) + (size_t)tab_slot * S::TABX;
@@ -332,6 +349,18 @@ __device__ __forceinline__ void apply_tile(const ApplyParams<T> &a, const T *__r
 #pragma unroll
             for (int il = 0; il < NB; ++il)
                 tpr[j][il] = make_float2(src[((QH + j) * NB + il) * 32 + lane], src[(j * NB + il) * 32 + lane]);
+    } else if constexpr (K > 1) {
+        // entry of quadrature column qx in the one-warp layout (lane_qx): its
+        // lane half and slot there
+        constexpr int Q0 = S::QH;
+        const int qx = 2 * kw + h;
+        const bool mid = mid_shared(NQ, (int)sizeof(T)) && qx == Q0 - 1;
+        const int h0 = mid ? 0 : qx / Q0, j0 = mid ? Q0 - 1 : qx - h0 * Q0;
+        const T *src = a.tabX + (size_t)gx * S::TABX + 2 * c + h0;
+#pragma unroll
+        for (int kind = 0; kind < 2; ++kind)
+#pragma unroll
+            for (int il = 0; il < NB; ++il) txr[kind][0][il] = qx < NQ ? src[((kind * Q0 + j0) * NB + il) * 32] : T(0);
     } else if constexpr (TXREG) {
         const T *src = a.tabX + (size_t)gx * S::TABX;
 #pragma unroll
@@ -341,12 +370,10 @@ __device__ __forceinline__ void apply_tile(const ApplyParams<T> &a, const T *__r
 #pragma unroll
                 for (int il = 0; il < NB; ++il) txr[kind][j][il] = src[((kind * QH + j) * NB + il) * 32 + lane];
     }
-    const T *txg = a.tabX + (size_t)gx * S::TABX + lane;
     auto tx = [&](int kind, int j, int il) -> T {
         if constexpr (PAIR) return kind ? tpr[j][il].x : tpr[j][il].y;
         else if constexpr (TXREG) return txr[kind][j][il];
-        else if constexpr (apply_txshared<P, T, GEOM>()) return tabXs[((kind * QH + j) * NB + il) * 32 + lane];
-        else return __ldg(txg + ((kind * QH + j) * NB + il) * 32);
+        else return tabXs[((kind * QH + j) * NB + il) * 32 + lane];
     };
     // Everything above reads only the plan's constant tables and geometry;
     // x (an earlier grid's output) and every write come after the wait.
@@ -465,16 +492,29 @@ __device__ __forceinline__ void apply_tile(const ApplyParams<T> &a, const T *__r
             if (c >= il) tot += v;
             else spill += v;
         }
+        // Always inside the patch (ey0 + nsteps + P <= n), but the exit changes
+        // how the stores below are scheduled: with it p=5 precomputed FP64 141 ->
+        // 138 us at 800^2, on-the-fly p=2 75.0 -> 73.9; without it on-the-fly
+        // FP64 p=3 377 -> 371, p=4 213 -> 207.
         const int R = ey0 + lr;
-        if (R >= g.n) return;
+        if constexpr (!(GEOM == 1 && sizeof(T) == 8 && P >= 3))
+            if (R >= g.n) return;
         // Strips covering row R / column C: the
         // first P rows/columns of a strip are shared with the strip before
         // it (if any), the P rows/columns past its end with the one after it.
         const bool row_single = lr < g.TY ? (lr >= P || gy == 0) : (gy + 1 >= g.NSY);
         const int lc = h ? kSW + c : c;
         const int C = ex0 + lc;
+        T v = h ? spill : tot;
+        if constexpr (K > 1) {   // the other warps' shares, in order (two slots: row lr + 1 may be on its way)
+            T *x0 = xch + (lr & 1) * (K - 1) * 32 + lane;
+            if (kw > 0) x0[(kw - 1) * 32] = v;
+            asm volatile("bar.sync %0, %1;" ::"r"(1 + w / K), "n"(32 * K) : "memory");
+            if (kw > 0) return;
+#pragma unroll
+            for (int k = 0; k < K - 1; ++k) v += x0[k * 32];
+        }
         if ((h == 0 || c < P) && C < g.m) {
-            const T v = h ? spill : tot;
             const bool col_single = h ? (gx + 1 >= g.NSX) : (c >= P || gx == 0);
             if (row_single && col_single) store(R, C, v);
             else frame[frame_index(lr, lc, P, g.TY)] = v;
@@ -543,7 +583,7 @@ __device__ __forceinline__ void apply_tile(const ApplyParams<T> &a, const T *__r
             }
         }
         const T *ty = yr + ((s + P) % S::XR) * S::TYW;   // landed with x row s + P
-        constexpr bool MID = mid_shared(NQ, (int)sizeof(T));
+        constexpr bool MID = K == 1 && mid_shared(NQ, (int)sizeof(T));
         constexpr int QJ = MID ? QH - 1 : QH;   // slots of this lane half's own columns
         // y tables of quadrature row qy: value n2 and derivative d2, or their
         // pairs nd (PAIR)
@@ -710,8 +750,9 @@ __device__ __forceinline__ void apply_tile(const ApplyParams<T> &a, const T *__r
             }
 #pragma unroll
             for (int j = 0; j < QJ; ++j) {
-                const int qx = h * QH + j;   // only h = 1's last slot can lie past NQ
-                qpoint(qy, qx, j, (NQ % 2 == 0 || j + 1 < QH) || qx < NQ, t, gv);
+                // only the last column can lie past NQ (h = 1's last slot, the last warp's h = 1)
+                const int qx = K > 1 ? 2 * kw + h : h * QH + j;
+                qpoint(qy, qx, j, NQ % 2 == 0 || (K == 1 && j + 1 < QH) || qx < NQ, t, gv);
             }
         }
         if constexpr (MID) {   // middle column QH - 1: half h takes rows qy = 2 t + h
@@ -753,7 +794,7 @@ __device__ __forceinline__ void apply_tile(const ApplyParams<T> &a, const T *__r
     cp_async_wait<0>();
 }
 
-// Strips to warps: warp k of the 1-D grid takes strip k in column-major
+// Strips to warps: warp k (apply_split: K warps) of the 1-D grid takes strip k in column-major
 // order (gx outer), so the grid covers NSX * rows strips with no partly idle
 // CTAs and the strip height can make the strip count fill the SMs. With the
 // tables in shared memory (apply_txshared) the CTA copies the tables of the
@@ -765,14 +806,8 @@ __global__ void __launch_bounds__(apply_max_threads<P, T, GEOM>(), 1) apply_kern
 {
     pdl_launch();   // apply_tile waits for the preceding grid once its constant operands are in flight
     const int rows = min(a.gyn, a.g.NSY - a.gy0);   // strip rows of the window
-    if constexpr (apply_percolumn<P, T, GEOM>()) {   // CTA = W strips of column strip blockIdx.x
-        apply_load_tabs<P, T, GEOM, NST>(a.tabX, blockIdx.x, 1, apply_tab_slots<P, T, GEOM, NST>());
-        __syncthreads();
-        const int r = blockIdx.y * blockDim.y + threadIdx.y;
-        apply_tile<P, T, GEOM, NST>(a, a.x, a.y, blockIdx.x, r < rows ? a.gy0 + r : a.g.NSY, 0);
-        return;
-    }
-    const int s0 = blockIdx.x * blockDim.y, sid = s0 + threadIdx.y;   // strips: NSX * NSY < 2^31
+    constexpr int K = apply_split<P, T, GEOM>();
+    const int s0 = blockIdx.x * (blockDim.y / K), sid = s0 + threadIdx.y / K;   // strips: NSX * NSY < 2^31
     const int gx = sid / rows;
     int slot = 0;
     if constexpr (apply_txshared<P, T, GEOM>()) {

@@ -134,23 +134,24 @@ Layout layout_for(int P, int nex, int ney, int TY, bool with_id)
     return L;
 }
 
-// Warps per CTA the register budget and the shared memory allow.
+// Strips per CTA the register budget and the shared memory allow.
 template <int P>
-int max_warps()
+int max_strips()
 {
-    int W = iga::apply_max_threads<P, double, 1>() / 32;
-    while (W > 1 && iga::apply_smem_bytes<P, double, 1, 2>(W, 2) > 220 * 1024) --W;
-    return W;
+    constexpr int K = iga::apply_split<P, double, 1>();
+    int S = iga::apply_max_threads<P, double, 1>() / 32 / K;
+    while (S > 1 && iga::apply_smem_bytes<P, double, 1, 2>(S * K, 2) > 220 * 1024) --S;
+    return S;
 }
 
-int max_warps_for(int p)
+int max_strips_for(int p)
 {
     switch (p) {
-    case 1: return max_warps<1>();
-    case 2: return max_warps<2>();
-    case 3: return max_warps<3>();
-    case 4: return max_warps<4>();
-    default: return max_warps<5>();
+    case 1: return max_strips<1>();
+    case 2: return max_strips<2>();
+    case 3: return max_strips<3>();
+    case 4: return max_strips<4>();
+    default: return max_strips<5>();
     }
 }
 
@@ -159,8 +160,9 @@ int launch(int dev, int nsm, unsigned char *base, const Layout &Ly, int TY, int 
            const int *d_ID, const double *d_in, double *d_out, cudaStream_t s)
 {
     using namespace iga;
-    int W = max_warps<P>();
-    const size_t smem_max = apply_smem_bytes<P, double, 1, 2>(W, 2);
+    constexpr int K = apply_split<P, double, 1>();
+    int S = max_strips<P>();
+    const size_t smem_max = apply_smem_bytes<P, double, 1, 2>(S * K, 2);
     auto kern = apply_kernel<P, double, 1, 2>;
     {
         std::lock_guard<std::mutex> lk(g_mu);
@@ -199,15 +201,13 @@ int launch(int dev, int nsm, unsigned char *base, const Layout &Ly, int TY, int 
     a.bc = d_ID ? IGA_BC_NONE : IGA_BC_REFERENCE;
     a.ID = d_ID;
     a.err = reinterpret_cast<int *>(base + Ly.off_err);
-    // strips dealt to warps one by one; with shared tables the CTA's strips
-    // lie in at most two column strips (W - 1 <= NSY)
-    constexpr bool percol = apply_percolumn<P, double, 1>();
-    W = (int)std::max(1LL, std::min<long long>(W, ((long long)g.NSX * g.NSY + nsm - 1) / nsm));
-    if (apply_txshared<P, double, 1>() && !percol) W = std::max(1, std::min(W, g.NSY + 1));
+    // strips dealt one by one; with shared tables the CTA's strips lie in at
+    // most two column strips (S - 1 <= NSY)
+    S = (int)std::max(1LL, std::min<long long>(S, ((long long)g.NSX * g.NSY + nsm - 1) / nsm));
+    if (apply_txshared<P, double, 1>()) S = std::max(1, std::min(S, g.NSY + 1));
     const long long nstrips = (long long)g.NSX * g.NSY;
-    const dim3 grid = percol ? dim3(g.NSX, (g.NSY + W - 1) / W) : dim3((unsigned)((nstrips + W - 1) / W)),
-               block(32, W);
-    kern<<<grid, block, apply_smem_bytes<P, double, 1, 2>(W, !percol && g.NSY % W ? 2 : 1), s>>>(a);
+    const dim3 grid((unsigned)((nstrips + S - 1) / S)), block(32, S * K);
+    kern<<<grid, block, apply_smem_bytes<P, double, 1, 2>(S * K, g.NSY % S ? 2 : 1), s>>>(a);
     cudaError_t e = cudaPeekAtLastError();
     const int blocks = seam_range(g).total;
     if (e == cudaSuccess && blocks > 0) {
@@ -267,7 +267,7 @@ extern "C" int iga_MatrixFreeMatMultCUDA_noalloc(int p, int q, int nex, int ney,
     // then the smallest of these whose tables and frames fit the scratch.
     int TY = 0;
     Layout Ly{};
-    for (int cand : {iga::one_wave_rows(nex, ney, p, max_warps_for(p), nsm), 32, 64, 128, 256, 512, 1024}) {
+    for (int cand : {iga::one_wave_rows(nex, ney, p, max_strips_for(p), nsm), 32, 64, 128, 256, 512, 1024}) {
         if (cand < p) continue;
         Ly = layout_for(p, nex, ney, cand, d_ID != nullptr);
         if (Ly.total <= kScratchBytes) {

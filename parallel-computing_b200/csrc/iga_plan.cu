@@ -413,9 +413,10 @@ template <int P, typename T, int GEOM>
 static int warps_for_t()
 {
     constexpr int NST = apply_stages<P, T>();
+    // whole strips (apply_split warps each)
     for (int W = apply_max_threads<P, T, GEOM>() / 32; W >= 1; --W)
-        if (apply_smem_bytes<P, T, GEOM, NST>(W, 2) <= kSmemBudget) return W;
-    return 1;
+        if (W % apply_split<P, T, GEOM>() == 0 && apply_smem_bytes<P, T, GEOM, NST>(W, 2) <= kSmemBudget) return W;
+    return apply_split<P, T, GEOM>();
 }
 
 template <typename T, int GEOM>
@@ -436,20 +437,23 @@ int warps_for(int P, int prec, int geom)
     return geom ? warps_for_g<float, 1>(P) : warps_for_g<float, 0>(P);
 }
 
+// Warps per strip of the apply kernel (apply_split).
+static int split_for(int P, int prec, int geom)
+{
+    return geom == IGA_GEOM_ON_THE_FLY && prec == IGA_FP64 && P >= 4 ? (P + 2) / 2 : 1;
+}
+
 // Rows per strip: the candidate whose CTA count fills the SMs best, with a
 // small penalty on short strips (more seam traffic). A MIXED plan launches
 // its FP64 and FP32 operators with different warps per CTA on the same
 // strips: each precision's cost is taken relative to its own best and the
-// candidate with the smallest sum wins. flat: the kernel deals strips to warps
-// one by one (apply_txreg), else a CTA covers W strips of one column.
+// candidate with the smallest sum wins. W: strips a CTA works on.
 struct WarpShape {
     int W;
-    bool flat;
     // also try the strip heights whose CTA count fills whole waves of SMs:
-    // the kernels with shared x tables dealt from a flat grid (FP64
-    // precomputed p >= 4, FP64 on-the-fly p = 1, 2), which are held back by
-    // each SM's own progress rather than by HBM (p=4 1024^2: 57 rows, 144
-    // CTAs, 146.4 -> 140.3 us; p=5: 38 rows, 238 -> 230 us; on-the-fly p=2
+    // the kernels held back by each SM's own progress rather than by HBM (FP64
+    // precomputed p >= 4, FP64 on-the-fly; p=4 1024^2: 57 rows, 144 CTAs,
+    // 146.4 -> 140.3 us; p=5: 38 rows, 238 -> 230 us; on-the-fly p=2
     // 1024^2 105.5 -> 101.4 us, p=1 50.1 -> 48.1 us), where the p=3 headline
     // at 82% of HBM gained nothing from it (40 or 50 rows: 312 / 314 us)
     bool waves = false;
@@ -458,7 +462,7 @@ struct WarpShape {
 static double strip_cost(int NSX, int ney, int TY, WarpShape ws, int nsm)
 {
     const int NSY = (ney + TY - 1) / TY, W = ws.W;
-    const long long ctas = ws.flat ? ((long long)NSX * NSY + W - 1) / W : (long long)NSX * ((NSY + W - 1) / W);
+    const long long ctas = ((long long)NSX * NSY + W - 1) / W;
     const long long waves = (ctas + nsm - 1) / nsm;
     const double work = (double)waves * W * (TY + 2.0);   // per-SM time in strip-row units
     return work * (1.0 + 0.5 * 3.0 / TY);
@@ -490,7 +494,7 @@ static int rows_for(int nex, int ney, int P, const std::vector<WarpShape> &Ws, i
         if (const int TY = one_wave_rows(nex, ney, P, Ws[0].W, nsm)) return TY;
     std::vector<int> cands = {64, 56, 48, 40, 32, 28, 24, 20, 16};
     for (const WarpShape &ws : Ws)
-        if (ws.waves && ws.flat)
+        if (ws.waves)
             for (int k = 1; k <= 16; ++k) {
                 const long long nsy = (long long)k * nsm * ws.W / NSX;   // strip rows of k full waves
                 if (nsy < 1) continue;
@@ -512,11 +516,6 @@ static int rows_for(int nex, int ney, int P, const std::vector<WarpShape> &Ws, i
     }
     return best;
 }
-
-// The single-plan kernel deals strips to warps one by one in every
-// configuration (shared x tables included) but the FP64 on-the-fly p = 5
-// one (apply_percolumn).
-static bool apply_flat(int P, int prec, int geom) { return !(P == 5 && prec == IGA_FP64 && geom == IGA_GEOM_ON_THE_FLY); }
 
 }  // namespace iga
 
@@ -651,17 +650,16 @@ static int launch_apply_t(iga_plan *pl, const OperatorData &op, const T *x, T *y
     // Fewer strips than one wave of full CTAs: as many warps per CTA as spread
     // them over all SMs (p=3 512^2 FP64, 16-row strips: 33.1 us in 86 CTAs of
     // 12 warps, 29.4 us in 147 of 7).
-    constexpr bool percol = apply_percolumn<P, T, GEOM>();
-    int W = (int)std::max(1LL, std::min<long long>(op.warps, ((long long)g.NSX * rows + pl->nsm - 1) / pl->nsm));
-    if (apply_txshared<P, T, GEOM>() && !percol) W = std::max(1, std::min(W, rows + 1));
-    const size_t smem = apply_smem_bytes<P, T, GEOM, NST>(W, !percol && rows % W ? 2 : 1);
+    constexpr int K = apply_split<P, T, GEOM>();   // warps per strip
+    int S = (int)std::max(1LL, std::min<long long>(op.warps / K, ((long long)g.NSX * rows + pl->nsm - 1) / pl->nsm));
+    if (apply_txshared<P, T, GEOM>()) S = std::max(1, std::min(S, rows + 1));
+    const size_t smem = apply_smem_bytes<P, T, GEOM, NST>(S * K, rows % S ? 2 : 1);
     if (win.gyn >= 0) {
         a.gy0 = win.gy0;
         a.gyn = rows;
     }
     const long long nstrips = (long long)g.NSX * rows;
-    const dim3 grid = percol ? dim3(g.NSX, (rows + W - 1) / W) : dim3((unsigned)((nstrips + W - 1) / W));
-    dim3 block(32, W);
+    const dim3 grid((unsigned)((nstrips + S - 1) / S)), block(32, S * K);
     // In the solver's loop: a programmatic dependent of the direction update
     // only while its CTAs fit one wave (mixed solve 2048^2 p=3: 355 us an
     // iteration, 339 with an ordinary edge; 64^2: 42.6 against 44.3).
@@ -851,9 +849,9 @@ int iga_plan_create(const iga_mesh_desc *d, const iga_opts *opts_in, iga_plan **
     // SMs best with its own warps per CTA (or the caller's rows_per_strip).
     auto rows_of = [&](int prec) {
         if (opts.rows_per_strip > 0) return opts.rows_per_strip;
-        const bool shared_flat = prec == IGA_FP64 && (opts.geometry == IGA_GEOM_PRECOMPUTED ? P.p >= 4 : P.p <= 2);
-        return rows_for(P.nex, P.ney, P.p, {{warps_for(P.p, prec, opts.geometry), apply_flat(P.p, prec, opts.geometry),
-                                         shared_flat}},
+        const bool waves = prec == IGA_FP64 && (opts.geometry == IGA_GEOM_ON_THE_FLY || P.p >= 4);
+        return rows_for(P.nex, P.ney, P.p, {{warps_for(P.p, prec, opts.geometry) / split_for(P.p, prec, opts.geometry),
+                                              waves}},
                         nsm);
     };
     auto make_grid = [&](int TY) {
@@ -1097,7 +1095,7 @@ int iga_apply_host(iga_plan *pl, const double *xh, double *yh)
     // slabs of about one wave of strips each (fewer strips leave SMs idle)
     int nsm = 148;
     cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, pl->device);
-    const long long wave = (long long)nsm * pl->op64.warps;
+    const long long wave = (long long)nsm * pl->op64.warps / split_for(g.P, IGA_FP64, pl->geometry);
     const int K = (int)std::max<long long>(1, std::min<long long>({(long long)kHostSlabs, (long long)g.NSY,
                                                                     ((long long)g.NSX * g.NSY + wave / 2) / wave}));
     const int m = g.m, n = g.n, P = g.P;
