@@ -691,8 +691,8 @@ __global__ void from_fp32_kernel(const float *__restrict__ z32, double *__restri
 // Bound: the recurrences' latency, then bytes. A warp per mode with all of an
 // SM's modes in one CTA had every warp load, then solve, then store at the
 // same time (2048^2: FP32 25 us, FP64 50 us; two buffers per warp, half the
-// warps: 30 and 67 us); CTAs of their own overlap these phases, and four warps
-// shorten the chains: 17 and 31 us.
+// warps: 30 and 67 us); CTAs of their own overlap these phases, and up to four
+// warps shorten the chains in FP64: 22.7 and 31 us.
 
 // inclusive scan of affine maps over lanes, lane order (forward) or reverse lane order
 template <typename R>
@@ -808,9 +808,16 @@ fd_tri_kernel(T *__restrict__ W, const T *__restrict__ Lf, const T *__restrict__
     }
 }
 
-// Warps per mode: enough that a thread has few rows, no more than keep most
-// threads busy.
-constexpr int tri_warps(int ny) { return ny <= 96 ? 1 : ny <= 384 ? 2 : 4; }
+// Warps per mode: FP64, enough that a thread has few rows, no more than keep
+// most threads busy. FP32 one: where a recurrence is cut moves its rounding, and
+// in the smoothest modes (condition ~ 1e6) that is worth up to 4e-5 of z, more
+// than FP32 results should depend on a launch shape (2048^2 with four warps: 17
+// us).
+template <typename T>
+constexpr int tri_warps(int ny)
+{
+    return sizeof(T) == 4 || ny <= 96 ? 1 : ny <= 384 ? 2 : 4;
+}
 constexpr size_t kTriSmem = 226 * 1024;   // most shared memory of a staged mode (leaves room for the static part)
 
 template <typename T, int NW>
@@ -827,9 +834,12 @@ static cudaError_t launch_tri(T *W, const T *Lf, const T *Dv, int nmodes, int ny
 template <typename T>
 static cudaError_t tri_prepare()   // the staged kernels' shared-memory limit
 {
-    cudaError_t e = cudaSuccess;
-    for (auto k : {fd_tri_kernel<T, true, 1>, fd_tri_kernel<T, true, 2>, fd_tri_kernel<T, true, 4>})
-        if (e == cudaSuccess) e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTriSmem);
+    auto set = [](auto k) { return cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTriSmem); };
+    cudaError_t e = set(fd_tri_kernel<T, true, 1>);
+    if constexpr (sizeof(T) == 8) {
+        if (e == cudaSuccess) e = set(fd_tri_kernel<T, true, 2>);
+        if (e == cudaSuccess) e = set(fd_tri_kernel<T, true, 4>);
+    }
     return e;
 }
 
@@ -1591,11 +1601,12 @@ static int fd_apply(PrecState<T> &ps, const iga_plan *pl, SolverState *S, const 
     int e = transform_gemm(ps, pl, 1, S->stream);
     if (e == IGA_OK) {
         const T *lf = ps.Lf, *dv = ps.Dv;
-        switch (tri_warps(ny)) {
-        case 1: SOLVE_TRY((launch_tri<T, 1>(ps.W1, lf, dv, ps.nmodes, ny, nyp, S->stream, S->s))); break;
-        case 2: SOLVE_TRY((launch_tri<T, 2>(ps.W1, lf, dv, ps.nmodes, ny, nyp, S->stream, S->s))); break;
-        default: SOLVE_TRY((launch_tri<T, 4>(ps.W1, lf, dv, ps.nmodes, ny, nyp, S->stream, S->s))); break;
+        const int nw = tri_warps<T>(ny);
+        if constexpr (sizeof(T) == 8) {
+            if (nw == 4) SOLVE_TRY((launch_tri<T, 4>(ps.W1, lf, dv, ps.nmodes, ny, nyp, S->stream, S->s)));
+            if (nw == 2) SOLVE_TRY((launch_tri<T, 2>(ps.W1, lf, dv, ps.nmodes, ny, nyp, S->stream, S->s)));
         }
+        if (nw == 1) SOLVE_TRY((launch_tri<T, 1>(ps.W1, lf, dv, ps.nmodes, ny, nyp, S->stream, S->s)));
         if (ps.kb > 0) {
             // parity split: the second GEMM writes both halves' products, the
             // unfold kernel combines them into z's interior
