@@ -394,6 +394,12 @@ struct FdProb {
 // (c -> end + prod c) are composed through shared memory, and each thread
 // adds its carry times the running coefficient product. One read of W, Dv, C
 // and one write of W. rows = (problem, first x mode) per block.
+// Bound: latency (64 registers, 2 blocks per SM in FP32; most stalls wait for
+// the columns' loads). The off-diagonals are converted once per block (read as
+// doubles and converted by every thread at every row they kept the FP64 pipe
+// busy), and lanes past the last mode repeat it, so that the loads need no
+// predicate per row (whose registers spilled): the preconditioner of 256
+// patches FP32 121 -> 109 us, FP64 321 -> 302.
 constexpr int kRowSeg = 16;                // segments per row
 constexpr int kRowLen = 17;                // rows per segment: ny <= kRowSeg * kRowLen (patches up to 272 free nodes)
 
@@ -404,36 +410,43 @@ __global__ void __launch_bounds__(32 * kRowSeg, sizeof(T) == 4 ? 2 : 1) fd_rows_
 {
     using R = T;   // segment arithmetic in the preconditioner's precision (registers: 2 blocks per SM in FP32)
     __shared__ R mE[kRowSeg][32], mP[kRowSeg][32];
+    __shared__ R ko[kRowSeg * kRowLen], mo[kRowSeg * kRowLen];   // the pencil's off-diagonals
     const int2 rw = rows[blockIdx.x];
     if (!act[rw.x]) return;
     const FdProb<T> &f = fps[rw.x];
     const int nx = f.nx, ny = f.ny;
-    const int a = rw.y + threadIdx.x, sg = threadIdx.y;
+    const bool live = rw.y + (int)threadIdx.x < nx;
+    const int a = min(rw.y + (int)threadIdx.x, nx - 1), sg = threadIdx.y;   // the rest repeat the last mode, unstored
     const int seglen = (ny + kRowSeg - 1) / kRowSeg;   // <= kRowLen
-    const int b0 = sg * seglen, len = max(0, min(seglen, ny - b0));
-    const bool live = a < nx;
-    const R lam = live ? f.lx[a] : R(0);
-    const double *yc = f.yc;
-    T *W = f.W1;
-    R w[kRowLen], c[kRowLen];
-#pragma unroll
-    for (int k = 0; k < kRowLen; ++k) {
-        const bool in = live && k < len;
-        w[k] = in ? W[a + (size_t)(b0 + k) * nx] : R(0);
-        c[k] = in ? f.Dv[a + (size_t)(b0 + k) * nx] : R(0);   // Dv now, C later
+    const int b0 = sg * seglen, len = min(seglen, ny - b0);   // (<= 0: no rows)
+    for (int b = sg * 32 + threadIdx.x; b < ny; b += 32 * kRowSeg) {
+        ko[b] = (R)f.yc[ny + b];
+        mo[b] = (R)f.yc[3 * ny + b];
     }
+    const R lam = f.lx[a];
+    T *W = f.W1 + a + b0 * nx;
+    R w[kRowLen], c[kRowLen];
+    {
+        const T *Dv = f.Dv + a + b0 * nx;
+#pragma unroll
+        for (int k = 0; k < kRowLen; ++k) {
+            if (k >= len) break;
+            w[k] = W[k * nx];
+            c[k] = Dv[k * nx];   // Dv now, C later
+        }
+    }
+    __syncthreads();
     // forward, zero carry-in; c[k] becomes beta_k
     R y = 0, pr = 1;
 #pragma unroll
     for (int k = 0; k < kRowLen; ++k) {
-        if (k < len) {
-            const int b = b0 + k;
-            const R beta = b == 0 ? R(0) : -(lam * (R)yc[3 * ny + b - 1] + (R)yc[ny + b - 1]) * c[k];
-            y = c[k] * w[k] + beta * y;
-            pr *= beta;
-            w[k] = y;
-            c[k] = beta;
-        }
+        if (k >= len) break;
+        const int b = b0 + k;
+        const R beta = b == 0 ? R(0) : -(lam * mo[b - 1] + ko[b - 1]) * c[k];
+        y = c[k] * w[k] + beta * y;
+        pr *= beta;
+        w[k] = y;
+        c[k] = beta;
     }
     mE[sg][threadIdx.x] = y;
     mP[sg][threadIdx.x] = pr;
@@ -443,14 +456,19 @@ __global__ void __launch_bounds__(32 * kRowSeg, sizeof(T) == 4 ? 2 : 1) fd_rows_
     R r = 1;
 #pragma unroll
     for (int k = 0; k < kRowLen; ++k) {
-        if (k < len) {
-            r *= c[k];
-            w[k] += r * cin;
-        }
+        if (k >= len) break;
+        r *= c[k];
+        w[k] += r * cin;
     }
     __syncthreads();   // carry maps read; the backward pass reuses them
+    {
+        const T *Cf = f.Cf + a + b0 * nx;
 #pragma unroll
-    for (int k = 0; k < kRowLen; ++k) c[k] = (live && k < len) ? f.Cf[a + (size_t)(b0 + k) * nx] : R(0);
+        for (int k = 0; k < kRowLen; ++k) {
+            if (k >= len) break;
+            c[k] = Cf[k * nx];
+        }
+    }
     R x = 0, q = 1;
 #pragma unroll
     for (int k = kRowLen - 1; k >= 0; --k) {
@@ -470,7 +488,7 @@ __global__ void __launch_bounds__(32 * kRowSeg, sizeof(T) == 4 ? 2 : 1) fd_rows_
     for (int k = kRowLen - 1; k >= 0; --k) {
         if (k < len) {
             r *= -c[k];
-            if (live) W[a + (size_t)(b0 + k) * nx] = (T)(w[k] + r * cin);
+            if (live) W[k * nx] = (T)(w[k] + r * cin);
         }
     }
 }

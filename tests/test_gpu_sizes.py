@@ -208,3 +208,29 @@ def test_exact_preconditioner_tiles(torch_cuda, ib, orc, p, nex, ney, split):
             # K's condition times the residuals' 1e-10 bounds the difference; 1e-7 holds it with room
             assert rel(x, ref) < 1e-7
     plan.close()
+
+
+# The batched exact preconditioner at the edges of its row segments (one row,
+# segments without rows, full ones, 272 rows), of its 32-mode blocks and of
+# its GEMM tiles and k slices (31 to 33, 64, 65, 128, 129 and 257 modes).
+# FP64: K_fem z = r to 1e-10; FP32, on TF32 operands, 1e-2 of the FP64 z.
+def test_batch_preconditioner_edges(torch_cuda, ib, orc):
+    free = [(1, 1), (31, 16), (32, 17), (33, 33), (64, 145), (65, 15), (128, 271), (129, 272), (257, 63), (2, 129)]
+    meshes = [ib.unit_square(p, nx + 2 - p, ny + 2 - p) for i, (nx, ny) in enumerate(free) for p in [1 if min(nx, ny) < 2 else 1 + i % 2]]
+    batch = ib.Batch(meshes, precision=ib.MIXED)
+    r = splitmix_uniform(29, -1.0, 1.0, batch.ntot)
+    rd = torch_cuda.from_numpy(r).cuda()
+    zd = torch_cuda.full_like(rd, float("nan"))
+    batch.pc_apply(rd, zd)
+    z32 = torch_cuda.full_like(rd.float(), float("nan"))
+    batch.pc_apply(rd.float(), z32, precision=ib.FP32)
+    z, z32 = zd.cpu().numpy(), z32.double().cpu().numpy()
+    for i, m in enumerate(meshes):
+        a, b = batch.offsets[i], batch.offsets[i + 1]
+        plan = ib.Plan(m)
+        gx, gy = plan.fem_nodes()
+        plan.close()
+        res = orc.fem_matvec(gx, gy, z[a:b]) - r[a:b]
+        assert np.linalg.norm(res) <= 1e-10 * np.linalg.norm(r[a:b]), free[i]
+        assert rel(z32[a:b], z[a:b]) < 1e-2, free[i]
+    batch.close()
