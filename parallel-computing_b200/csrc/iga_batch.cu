@@ -377,8 +377,7 @@ template <typename T>
 struct FdProb {
     const T *Vx, *lx;      // x eigenvectors (column-major, ld nx) and eigenvalues
     const T *VxT;          // the transpose of Vx (column-major), for the tcgen05 tiles
-    const T *Vxp, *VxTp;   // FP32: Vx and VxT with columns padded to ldv (a multiple of 4): 16-byte rows
-    int ldv;
+    const T *Vxp, *VxTp;   // FP32: Vx and VxT as the A operands of the tcgen05 tiles (umma_a_index)
     const T *Dv, *Cf;      // LDL^T factors of the y systems: 1 / pivot, upper off-diagonal; [b][a], ld nx
     const double *yc;      // free y nodes' pencil Kd | Ko | Md | Mo (ny each)
     T *W1;                 // nx * ny work matrix
@@ -683,43 +682,78 @@ __global__ void __launch_bounds__(128) fd_gemm_kernel(const FdProb<T> *__restric
 }
 
 // FP32 preconditioner tiles on the 5th-generation tensor cores (tcgen05,
-// kind::tf32): C[a + b ldc] = sum_k A[a lda + k] B[b ldb + k] for a 128 x 64
+// kind::tf32): C[a + b ldc] = sum_k A[a][k] B[b ldb + k] for a 128 x 64
 // output tile of one problem, the FP32 accumulator in TMEM.
 //   stage 1: A rows = Vx columns (Vx^T), B rows = R^T (r + m + 1, ld m), C = W1
 //   stage 3: A rows = VxT columns (Vx),   B rows = W1^T (ld nx),        C = z + m + 1 (ld m)
-// All 128 threads stage 32-wide K slices (rounded to TF32) into two shared
-// memory buffers in the no-swizzle K-major layout; thread 0 issues four
-// 128 x 64 x 8 MMAs per slice and commits them to the buffer's mbarrier,
-// which the threads wait on (bounded) before refilling that buffer. The
-// epilogue reads the accumulator with tcgen05.ld (warp w: rows 32w .. 32w+31).
+// A, constant, is laid out at set-up as the shared memory images of its 32-wide
+// K slices, rounded to TF32: thread 0 brings each in with one bulk copy. B's
+// rows are not 16-byte aligned: all 128 threads stage its slices through
+// registers (rounded to TF32). Both in the no-swizzle K-major layout, two
+// buffers each. Thread 0 issues four 128 x 64 x 8 MMAs per slice and commits
+// them to the B buffer's mbarrier, which the threads wait on (bounded) before
+// refilling the buffers. The epilogue reads the accumulator with tcgen05.ld
+// (warp w: rows 32w .. 32w+31).
+// Bound: latency of short contractions (a patch's 3 to 9 slices), so resident
+// CTAs count: 50 KB of buffers and at most 128 registers let four share an SM.
+// A through registers like B (158 registers, three CTAs): 256 patches 109 us
+// for the whole preconditioner, now 94; a third A buffer (three CTAs) 100.
 constexpr int kUM = 128, kUN = 64, kUK = 32;
-constexpr int kALbo = (kUM / 8) * 128 + 16;   // K-chunk stride of an A buffer (+16 B: conflict-free stores)
-constexpr int kBLbo = (kUN / 8) * 128 + 16;
+constexpr int kUA = 2;                        // A buffers
+constexpr int kALbo = (kUM / 8) * 128;        // K-chunk stride of an A buffer
+constexpr int kBLbo = (kUN / 8) * 128 + 16;   // of a B buffer (+16 B: conflict-free stores)
 constexpr int kAStage = 8 * kALbo, kBStage = 8 * kBLbo;   // 8 chunks of 4 values = 32 k
-constexpr int kUmmaSmem = 2 * (kAStage + kBStage) + 64;
+constexpr int kUmmaSmem = kUA * kAStage + 2 * kBStage + 64;
+
+// The A operand as the copies take it: per 128-row tile and 32-wide K slice
+// one block of kAStage bytes, the shared memory image of the slice (chunks of
+// 4 k, 16 bytes a row), zero past n, values rounded to TF32.
+__host__ __device__ constexpr int umma_slices(int n) { return (n + kUK - 1) / kUK; }
+__host__ __device__ constexpr size_t umma_a_size(int n)
+{
+    return (size_t)((n + kUM - 1) / kUM) * umma_slices(n) * (kUM * kUK);
+}
+__host__ __device__ constexpr size_t umma_a_index(int row, int k, int n)
+{
+    return (((size_t)(row / kUM) * umma_slices(n) + k / kUK) * (kUK / 4) + k % kUK / 4) * (kUM * 4) + row % kUM * 4 + k % 4;
+}
 
 template <int STAGE>
-__global__ void __launch_bounds__(128) fd_umma_kernel(const FdProb<float> *__restrict__ fps,
+__global__ void __launch_bounds__(128, 4) fd_umma_kernel(const FdProb<float> *__restrict__ fps,
                                                       const int4 *__restrict__ tiles, const int *__restrict__ act,
                                                       const float *__restrict__ rb, float *__restrict__ zb,
                                                       int *__restrict__ err)
 {
     extern __shared__ __align__(128) unsigned char sm[];
-    uint64_t *bars = reinterpret_cast<uint64_t *>(sm + 2 * (kAStage + kBStage));
-    uint32_t *tbase = reinterpret_cast<uint32_t *>(bars + 2);
+    unsigned char *Bs = sm + kUA * kAStage;
+    uint64_t *bars = reinterpret_cast<uint64_t *>(Bs + 2 * kBStage), *fullA = bars + 2;
+    uint32_t *tbase = reinterpret_cast<uint32_t *>(fullA + kUA);
     const int4 tl = tiles[blockIdx.x];
     if (!act[tl.x]) return;
     const FdProb<float> &f = fps[tl.x];
     const int nx = f.nx, ny = f.ny, m = f.m, K = nx;
     const int a0 = tl.y * kUM, b0 = tl.z * kUN;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const float *A, *Bm;
+    const int nk = umma_slices(K);
+    const float *A = (STAGE == 1 ? f.Vxp : f.VxTp) + (size_t)tl.y * nk * (kUM * kUK);
+    const float *Bm;
     float *C;
-    int lda, ldb, ldc;
+    int ldb, ldc;
     if (STAGE == 1) {
-        A = f.Vxp; lda = f.ldv; Bm = rb + f.off + m + 1; ldb = m; C = f.W1; ldc = nx;
+        Bm = rb + f.off + m + 1; ldb = m; C = f.W1; ldc = nx;
     } else {
-        A = f.VxTp; lda = f.ldv; Bm = f.W1; ldb = nx; C = zb + f.off + m + 1; ldc = m;
+        Bm = f.W1; ldb = nx; C = zb + f.off + m + 1; ldc = m;
+    }
+    auto load_a = [&](int kt) {   // by thread 0
+        mbar_arrive_expect_tx(&fullA[kt % kUA], kAStage);
+        bulk_g2s(sm + kt % kUA * kAStage, A + (size_t)kt * (kUM * kUK), kAStage, &fullA[kt % kUA]);
+    };
+    if (tid == 0) {
+        mbar_init(&bars[0], 1);
+        mbar_init(&bars[1], 1);
+        for (int k = 0; k < kUA; ++k) mbar_init(&fullA[k], 1);
+        fence_mbar_init();
+        for (int k = 0; k < min(nk, kUA); ++k) load_a(k);
     }
     if (STAGE == 1 && tl.y == 0 && tl.z == 0) {   // boundary ring: identity rows of K_fem
         const float *r = rb + f.off;
@@ -740,92 +774,69 @@ __global__ void __launch_bounds__(128) fd_umma_kernel(const FdProb<float> *__res
         umma::alloc(tbase, kUN);
         umma::relinquish();
     }
-    if (tid == 0) {
-        mbar_init(&bars[0], 1);
-        mbar_init(&bars[1], 1);
-        fence_mbar_init();
-    }
     umma::fence_before_sync();
     __syncthreads();
     umma::fence_after_sync();
     const uint32_t tmem = *tbase;
 
-    // A (rows padded to lda, a multiple of 4, zero past K): thread t moves the
-    // 16-byte K chunk t % 8 of rows t / 8 + 16 i; B: thread (warp, lane) moves
-    // k = lane of rows warp + 4 i. Two register sets: slice kt + 2 is loaded
-    // while slice kt + 1 goes from the other set into shared memory, so a
-    // slice's global loads have a whole iteration to land.
-    struct Regs {
-        float4 a[kUM / 16];
-        float b[kUN / 4];
-    };
+    // B: thread (warp, lane) moves k = lane of rows warp + 4 i. Two register
+    // sets: slice kt + 2 is loaded while slice kt + 1 goes from the other set
+    // into shared memory, so a slice's loads have a whole iteration to land.
+    using Regs = float[kUN / 4];
     Regs R0, R1;
+    const float *Bt = Bm + (size_t)(b0 + warp) * ldb + lane;
+    const int nb = (ny - b0 - warp + 3) / 4;   // this thread's rows inside the problem
     auto fetch = [&](int kt, Regs &rg) {
-        const int k0 = kt * kUK, k = k0 + lane;
-        const bool kin = k < K;
-        const int kc = k0 + 4 * (tid & 7);
+        const bool kin = kt * kUK + lane < K;
+        const float *src = Bt + kt * kUK;
 #pragma unroll
-        for (int i = 0; i < kUM / 16; ++i) {
-            const int a = a0 + (tid >> 3) + 16 * i;
-            rg.a[i] = (kc < K && a < nx) ? *reinterpret_cast<const float4 *>(A + (size_t)a * lda + kc)
-                                         : make_float4(0.f, 0.f, 0.f, 0.f);
-        }
-#pragma unroll
-        for (int i = 0; i < kUN / 4; ++i) {
-            const int b = b0 + warp + 4 * i;
-            rg.b[i] = (kin && b < ny) ? Bm[(size_t)b * ldb + k] : 0.0f;
-        }
+        for (int i = 0; i < kUN / 4; ++i) rg[i] = (kin && i < nb) ? src[4 * i * ldb] : 0.0f;
     };
     auto stash = [&](int buf, const Regs &rg) {
-        unsigned char *Ab = sm + buf * kAStage, *Bb = sm + 2 * kAStage + buf * kBStage;
-        const int ch = lane >> 2, w4 = (lane & 3) * 4;
-#pragma unroll
-        for (int i = 0; i < kUM / 16; ++i) {
-            const int r = (tid >> 3) + 16 * i;
-            const float4 v = make_float4(to_operand(rg.a[i].x), to_operand(rg.a[i].y), to_operand(rg.a[i].z),
-                                         to_operand(rg.a[i].w));
-            *reinterpret_cast<float4 *>(Ab + (tid & 7) * kALbo + (r >> 3) * 128 + (r & 7) * 16) = v;
-        }
+        unsigned char *Bb = Bs + buf * kBStage + (lane >> 2) * kBLbo + (lane & 3) * 4;
 #pragma unroll
         for (int i = 0; i < kUN / 4; ++i) {
             const int r = warp + 4 * i;
-            *reinterpret_cast<float *>(Bb + ch * kBLbo + (r >> 3) * 128 + (r & 7) * 16 + w4) = to_operand(rg.b[i]);
+            *reinterpret_cast<float *>(Bb + (r >> 3) * 128 + (r & 7) * 16) = to_operand(rg[i]);
         }
     };
     constexpr uint32_t IDESC = umma::idesc_tf32<kUM, kUN>();
-    const int nk = (K + kUK - 1) / kUK;
     fetch(0, R0);
     if (nk > 1) fetch(1, R1);
     stash(0, R0);
     fence_proxy_async_smem();
     __syncthreads();
     bool failed = false;
-    int last = -1;   // last slice whose MMAs were issued
+    int last = -1;    // last slice stepped through
     // one iteration: MMAs of slice kt; loads of slice kt + 2 into the set that
     // held slice kt (`cur`); slice kt + 1 from the other set (`nxt`) into the
-    // buffer freed by slice kt - 1
+    // B buffer that slice kt - 1 has left, and the next A slice into its A buffer
     auto step = [&](int kt, Regs &cur, Regs &nxt) -> bool {
         const int buf = kt & 1;
+        bool ok = true;
         if (tid == 0) {
-            umma::fence_after_sync();
-            const unsigned char *Ab = sm + buf * kAStage, *Bb = sm + 2 * kAStage + buf * kBStage;
+            ok = mbar_wait_bounded(&fullA[kt % kUA], (kt / kUA) & 1);
+            if (ok) {
+                umma::fence_after_sync();
+                const unsigned char *Ab = sm + kt % kUA * kAStage, *Bb = Bs + buf * kBStage;
 #pragma unroll
-            for (int j = 0; j < kUK / 8; ++j)
-                umma::mma_tf32(tmem, umma::smem_desc(Ab + 2 * j * kALbo, kALbo, 128),
-                               umma::smem_desc(Bb + 2 * j * kBLbo, kBLbo, 128), IDESC, (kt > 0 || j > 0) ? 1u : 0u);
+                for (int j = 0; j < kUK / 8; ++j)
+                    umma::mma_tf32(tmem, umma::smem_desc(Ab + 2 * j * kALbo, kALbo, 128),
+                                   umma::smem_desc(Bb + 2 * j * kBLbo, kBLbo, 128), IDESC, (kt > 0 || j > 0) ? 1u : 0u);
+            }
             umma::commit(&bars[buf]);
         }
         last = kt;
         if (kt + 2 < nk) fetch(kt + 2, cur);
         if (kt + 1 < nk) {
-            bool ok = true;
-            if (kt >= 1) ok = mbar_wait_bounded(&bars[(kt - 1) & 1], ((kt - 1) >> 1) & 1);   // buffer reused
-            if (__syncthreads_or(!ok)) return false;
-            stash((kt + 1) & 1, nxt);
+            if (kt >= 1) {   // buffers reused
+                ok = mbar_wait_bounded(&bars[(kt - 1) & 1], ((kt - 1) >> 1) & 1) && ok;
+                if (tid == 0 && ok && kt - 1 + kUA < nk) load_a(kt - 1 + kUA);
+            }
+            if (ok) stash((kt + 1) & 1, nxt);
             fence_proxy_async_smem();
         }
-        __syncthreads();
-        return true;
+        return !__syncthreads_or(!ok);
     };
     for (int kt = 0; kt < nk; ++kt) {
         const bool ok = (kt & 1) ? step(kt, R1, R0) : step(kt, R0, R1);
@@ -838,8 +849,13 @@ __global__ void __launch_bounds__(128) fd_umma_kernel(const FdProb<float> *__res
     const bool ok = mbar_wait_bounded(&bars[last & 1], (last >> 1) & 1);
     failed = __syncthreads_or(failed || !ok);
     if (failed) {
-        if (tid == 0) atomicExch(err, 8 /* IGA_ERR_TIMEOUT */);
+        if (tid == 0) {
+            atomicExch(err, 8 /* IGA_ERR_TIMEOUT */);
+            // the A copies issued and not consumed land before their buffers are released
+            for (int kt = last; kt < min(nk, last + kUA + 1); ++kt) mbar_wait_bounded(&fullA[kt % kUA], (kt / kUA) & 1);
+        }
         mbar_wait_bounded(&bars[last & 1], (last >> 1) & 1);
+        __syncthreads();
     } else {
         umma::fence_after_sync();
         const int a = a0 + 32 * warp + lane;
@@ -1262,14 +1278,14 @@ __global__ void fd_ldl_kernel(const FdProb<double> *__restrict__ f64, const FdPr
 // (U + uo, hn_o long; uo < 0: a pencil that was not split, fe = n), scaled
 // by sc; mirrored entries v[n-1-i] = +-u[i]; lam: the n eigenvalues in the
 // same mode order. Outputs: V (component i of mode a at a n + i) and its
-// transpose VT, FP64 and, when V32 is set, FP32 with 16-byte padded copies
-// (row length ldp).
+// transpose VT in FP64 and, when Vp32 is set, both as tcgen05 A operands
+// (umma_a_index).
 struct BasisDev {
-    int n, fe, hn_e, hn_o, ldp;
+    int n, fe, hn_e, hn_o;
     long long ue, uo, lo;
     double sc;
     double *V, *VT, *L;
-    float *V32, *VT32, *Vp32, *VTp32, *L32;
+    float *Vp32, *VTp32, *L32;
 };
 
 __global__ void basis_build_kernel(const BasisDev *__restrict__ bs, const double *__restrict__ U,
@@ -1294,11 +1310,9 @@ __global__ void basis_build_kernel(const BasisDev *__restrict__ bs, const double
         }
         b.V[t] = v;
         b.VT[(long long)i * n + a] = v;
-        if (b.V32) {
-            b.V32[t] = (float)v;
-            b.VT32[(long long)i * n + a] = (float)v;
-            b.Vp32[(long long)a * b.ldp + i] = (float)v;
-            b.VTp32[(long long)i * b.ldp + a] = (float)v;
+        if (b.Vp32) {
+            b.Vp32[umma_a_index(a, i, n)] = to_operand((float)v);
+            b.VTp32[umma_a_index(i, a, n)] = to_operand((float)v);
         }
         if (i == 0) {
             b.L[a] = lam[b.lo + a];
@@ -1437,14 +1451,14 @@ int setup_fd(iga_batch *B)
         }
     }
     const bool mixed = B->precision == IGA_MIXED;
-    // every sub-array starts on a 16-byte boundary (the FP32 padded copies
-    // move as 16-byte words)
+    // every sub-array starts on a 16-byte boundary (the tcgen05 operands are
+    // read by bulk copies)
     auto al4 = [](size_t x) { return (x + 3) / 4 * 4; };
     size_t tot64 = 0, tot32 = 0;
     for (const Basis &bb : bases) {
-        const size_t n = (size_t)bb.n, ldp = al4(n);
+        const size_t n = (size_t)bb.n;
         tot64 += 2 * al4(n * n) + al4(n);
-        if (mixed) tot32 += 2 * al4(n * n) + 2 * n * ldp + al4(n);
+        if (mixed) tot32 += 2 * umma_a_size(bb.n) + al4(n);
     }
     double *b64 = nullptr;
     float *b32 = nullptr;
@@ -1454,37 +1468,33 @@ int setup_fd(iga_batch *B)
         B->v64.basis.push_back(b64);
         if (mixed) {
             if ((st = bmalloc(&b32, tot32))) return st;
-            BT_TRY(cudaMemset(b32, 0, sizeof(float) * tot32));   // the padding columns
+            BT_TRY(cudaMemset(b32, 0, sizeof(float) * tot32));   // the operands' padding
             B->v32.basis.push_back(b32);
         }
     }
     std::vector<BasisDev> bd(grids.size());
     std::vector<double *> V64(grids.size()), VT64(grids.size()), L64(grids.size());
-    std::vector<float *> V32(grids.size(), nullptr), VT32(grids.size(), nullptr), Vp32(grids.size(), nullptr),
-        VTp32(grids.size(), nullptr), L32(grids.size(), nullptr);
+    std::vector<float *> Vp32(grids.size(), nullptr), VTp32(grids.size(), nullptr), L32(grids.size(), nullptr);
     {
         size_t o64 = 0, o32 = 0;
         for (size_t k = 0; k < grids.size(); ++k) {
             const int n = bases[k].n;
-            const size_t nn = (size_t)n * n, ldp = al4((size_t)n);
+            const size_t nn = (size_t)n * n;
             V64[k] = b64 + o64;
             VT64[k] = V64[k] + al4(nn);
             L64[k] = VT64[k] + al4(nn);
             o64 += 2 * al4(nn) + al4(n);
             if (mixed) {
-                V32[k] = b32 + o32;
-                VT32[k] = V32[k] + al4(nn);
-                Vp32[k] = VT32[k] + al4(nn);
-                VTp32[k] = Vp32[k] + (size_t)n * ldp;
-                L32[k] = VTp32[k] + (size_t)n * ldp;
-                o32 += 2 * al4(nn) + 2 * (size_t)n * ldp + al4(n);
+                Vp32[k] = b32 + o32;
+                VTp32[k] = Vp32[k] + umma_a_size(n);
+                L32[k] = VTp32[k] + umma_a_size(n);
+                o32 += 2 * umma_a_size(n) + al4(n);
             }
             BasisDev &d = bd[k];
             d.n = n;
             d.fe = split[k] ? fe_of[k] : n;
             d.hn_e = hne[k];
             d.hn_o = hno[k];
-            d.ldp = (int)ldp;
             d.ue = ue_of[k] < 0 ? 0 : ue_of[k];
             d.uo = split[k] ? uo_of[k] : -1;
             d.lo = lo_of[k];
@@ -1492,8 +1502,6 @@ int setup_fd(iga_batch *B)
             d.V = V64[k];
             d.VT = VT64[k];
             d.L = L64[k];
-            d.V32 = V32[k];
-            d.VT32 = VT32[k];
             d.Vp32 = Vp32[k];
             d.VTp32 = VTp32[k];
             d.L32 = L32[k];
@@ -1537,11 +1545,10 @@ int setup_fd(iga_batch *B)
         for (int i = 0; i < B->count; ++i) {
             const iga_plan *pl = B->plans[i];
             FdProb<T> &f = fp[i];
-            f.Vx = pick(V64[bx[i]], V32[bx[i]]);
-            f.VxT = pick(VT64[bx[i]], VT32[bx[i]]);
+            f.Vx = pick(V64[bx[i]], nullptr);
+            f.VxT = pick(VT64[bx[i]], nullptr);
             f.Vxp = f64 ? nullptr : pick(nullptr, Vp32[bx[i]]);
             f.VxTp = f64 ? nullptr : pick(nullptr, VTp32[bx[i]]);
-            f.ldv = (bases[bx[i]].n + 3) / 4 * 4;
             f.lx = pick(L64[bx[i]], L32[bx[i]]);
             f.yc = B->ycoef[by[i]];
             f.W1 = v.W1 + wo;
