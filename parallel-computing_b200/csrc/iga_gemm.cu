@@ -624,7 +624,7 @@ int gemm_f64_launch(GemmOperand A, GemmOperand B, double *C, int ldc, int M, int
     // MMA), so the small ones are used where they give the fullest SM that
     // much less: the preconditioner's two half-size transforms at p=3 512^2 (81
     // tiles of 64 x 64 for 148 SMs) 50.2 -> 31.9 us in all, 700^2 105 -> 53,
-    // 1200^2 182 -> 165, 2048^2 709 -> 702; at 1024^2 (exactly two of 64 x 64
+    // 1200^2 182 -> 165, 2048^2 681 -> 673; at 1024^2 (exactly two of 64 x 64
     // an SM) 64 x 64 stays, 108 against 117.
     int nsm = 148, dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
