@@ -234,3 +234,26 @@ def test_batch_preconditioner_edges(torch_cuda, ib, orc):
         assert np.linalg.norm(res) <= 1e-10 * np.linalg.norm(r[a:b]), free[i]
         assert rel(z32[a:b], z[a:b]) < 1e-2, free[i]
     batch.close()
+
+
+# The batched iteration's vector kernels: patches that start at every entry
+# offset of a 16-byte word, shorter than a word's ragged ends, of exactly one
+# chunk of 2048 entries (32 x 64 control points) and one entry more or less of
+# a few. True residuals by the oracle at twice the tolerance asked for.
+@pytest.mark.parametrize("prec", ["FP64", "MIXED"])
+def test_batch_vectors_start_anywhere(torch_cuda, ib, orc, prec):
+    prec = getattr(ib, prec)
+    points = [(3, 3), (3, 5), (32, 64), (5, 7), (683, 3), (7, 11), (6, 3), (4, 4), (23, 89), (61, 67), (9, 9)]
+    meshes = [ib.unit_square(2, m - 2, n - 2) for m, n in points]
+    batch = ib.Batch(meshes, precision=prec)
+    assert {int(o) % 4 for o in batch.offsets[:-1]} == {0, 1, 2, 3}
+    b = splitmix_uniform(31, -1.0, 1.0, batch.ntot)
+    x = torch_cuda.zeros(batch.ntot, dtype=torch_cuda.float64, device="cuda")
+    st, its, _ = batch.solve(torch_cuda.from_numpy(b).cuda(), x, precision=prec, rtol=1e-10)
+    assert st.converged == len(points)
+    x = x.cpu().numpy()
+    for i, m in enumerate(meshes):
+        s, e = batch.offsets[i], batch.offsets[i + 1]
+        r = b[s:e] - orc.apply_mf(m, x[s:e], sign=1.0, bc=1)
+        assert np.linalg.norm(r) <= 2e-10 * np.linalg.norm(b[s:e]), points[i]
+    batch.close()
