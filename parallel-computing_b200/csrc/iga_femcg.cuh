@@ -35,7 +35,8 @@ struct IcgShape {
     size_t smem = 0;
 };
 
-constexpr int kIcgMaxThreads = 512;   // of a CTA (the kernel's launch bounds)
+constexpr int kIcgMaxThreads = 512;         // of a CTA (the kernel's launch bounds)
+constexpr size_t kIcgMaxSmem = 226 * 1024;   // of a CTA (the limit set for every instance of the kernel)
 
 template <typename T>
 inline size_t icg_smem(int m, int rows, int C, int nw)
@@ -65,7 +66,6 @@ inline IcgShape icg_shape(int m, int n, int k)
     const int rows = (n + C - 1) / C;
     const long long threads = (long long)m * ((rows + L - 1) / L);
     if (threads > kIcgMaxThreads) return s;
-    s.C = C;
     s.rows = rows;
     s.L = L == 4 && rows < 4 ? (rows >= 2 ? 2 : 1) : L;
     s.threads = (int)(((long long)m * ((rows + s.L - 1) / s.L) + 31) / 32 * 32);
@@ -74,6 +74,7 @@ inline IcgShape icg_shape(int m, int n, int k)
         s.threads = (int)((threads + 31) / 32 * 32);
     }
     s.smem = icg_smem<T>(m, rows, C, s.threads / 32);
+    s.C = s.smem <= kIcgMaxSmem ? C : 0;
     return s;
 }
 

@@ -1197,7 +1197,9 @@ static void (*icg_kernel(int L))(IcgArgs<T>)
 }
 
 // The cluster shape of the inner FEM-CG for this plan's grid: the first one
-// that fits and that the device can place.
+// that fits and that the device can place. The kernel's shared-memory limit
+// belongs to the function, which all plans launch: it is set to the most any
+// shape may take, never to this plan's own size.
 template <typename T>
 static int icg_prepare(PrecState<T> &ps, const iga_plan *pl)
 {
@@ -1209,7 +1211,7 @@ static int icg_prepare(PrecState<T> &ps, const iga_plan *pl)
             cudaGetLastError();
             continue;
         }
-        SOLVE_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sh.smem));
+        SOLVE_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kIcgMaxSmem));
         cudaLaunchConfig_t cfg = {};
         cfg.gridDim = dim3(sh.C);
         cfg.blockDim = dim3(sh.threads);
