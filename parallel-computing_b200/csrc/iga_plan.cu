@@ -1,4 +1,5 @@
 // Plans and the C ABI of the matrix-free operator (include/iga_mf.h).
+#include <cuda.h>
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -995,17 +996,50 @@ int iga_plan_get_info(const iga_plan *pl, iga_plan_info *info)
     return IGA_OK;
 }
 
+// Whether a kernel on `device` may read bytes p .. p + n - 1 as doubles:
+// aligned, and inside one allocation of that device's own memory. (A copy takes
+// more: pinned host memory, managed memory, another device's, any alignment;
+// and it refuses what lies outside every allocation, where a kernel would
+// fault.)
+static bool kernel_readable(const void *p, size_t n, int device)
+{
+    using Query = CUresult (*)(unsigned, CUpointer_attribute *, void **, CUdeviceptr);
+    static const Query query = [] {
+        void *f = nullptr;
+        cudaDriverEntryPointQueryResult q;
+        if (cudaGetDriverEntryPoint("cuPointerGetAttributes", &f, cudaEnableDefault, &q) != cudaSuccess ||
+            q != cudaDriverEntryPointSuccess)
+            f = nullptr;
+        return reinterpret_cast<Query>(f);
+    }();
+    if (!query || (uintptr_t)p % alignof(double)) return false;
+    unsigned type = 0;
+    int managed = 0, ordinal = -1;
+    CUdeviceptr start = 0;
+    size_t size = 0;
+    CUpointer_attribute what[] = {CU_POINTER_ATTRIBUTE_MEMORY_TYPE, CU_POINTER_ATTRIBUTE_IS_MANAGED,
+                                  CU_POINTER_ATTRIBUTE_DEVICE_ORDINAL, CU_POINTER_ATTRIBUTE_RANGE_START_ADDR,
+                                  CU_POINTER_ATTRIBUTE_RANGE_SIZE};
+    void *out[] = {&type, &managed, &ordinal, &start, &size};
+    const CUdeviceptr a = (CUdeviceptr)(uintptr_t)p;
+    return query(5, what, out, a) == CUDA_SUCCESS && type == CU_MEMORYTYPE_DEVICE && !managed && ordinal == device &&
+           a >= start && a - start <= size && n <= size - (a - start);
+}
+
 int iga_plan_set_kappa(iga_plan *pl, const double *kappa, void *stream)
 {
     if (!pl || !kappa) return IGA_ERR_ARG;
     cudaStream_t s = (cudaStream_t)stream;
     const long long nq = (long long)pl->nex * pl->ney * (pl->p + 1) * (pl->p + 1);
     if (!pl->kappa_dev) IGA_CUDA_TRY(cudaMalloc((void **)&pl->kappa_dev, nq * sizeof(double)));
+    // the geometry's pass over the points also takes the copy, where it may read kappa
+    const bool fused = pl->geometry == IGA_GEOM_PRECOMPUTED && kappa != pl->kappa_dev &&
+                       kernel_readable(kappa, nq * sizeof(double), pl->device);
+    if (!fused) IGA_CUDA_TRY(cudaMemcpyAsync(pl->kappa_dev, kappa, nq * sizeof(double), cudaMemcpyDeviceToDevice, s));
     ++pl->kappa_version;
-    if (pl->geometry == IGA_GEOM_PRECOMPUTED) {   // the pass over the points also takes the copy
-        launch_geom(geom_job(pl, kappa, kappa == pl->kappa_dev ? nullptr : pl->kappa_dev), s);
+    if (pl->geometry == IGA_GEOM_PRECOMPUTED) {
+        launch_geom(geom_job(pl, fused ? kappa : pl->kappa_dev, fused ? pl->kappa_dev : nullptr), s);
     } else {
-        IGA_CUDA_TRY(cudaMemcpyAsync(pl->kappa_dev, kappa, nq * sizeof(double), cudaMemcpyDeviceToDevice, s));
         OperatorData *ops[2] = {&pl->op64, &pl->op32};
         for (int k = 0; k < 2; ++k) {
             OperatorData &op = *ops[k];
