@@ -151,7 +151,8 @@ int iga_apply_host(iga_plan *plan, const double *x_host, double *y_host);
  * counterpart in the reference, which calls exit() on any CUDA error
  * (matrix_free_gpu/include/memory.cuh:9-12). */
 int iga_plan_device_status(iga_plan *plan, void *stream);
-/* Polls each bounded wait of the plan's MatMult kernel makes before it gives
+/* Polls each bounded wait of the plan's MatMult kernel, and of the cluster
+ * kernel of its inner FEM-CG (IGA_PC_FEM_CG), makes before it gives
  * up with IGA_ERR_TIMEOUT: polls >= 0 sets the limit (0: every wait gives up
  * at once, for tests of the timeout path; the kernel still waits, with the
  * full limit, for the copies it issued before returning), polls < 0 restores

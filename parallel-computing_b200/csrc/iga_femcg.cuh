@@ -88,6 +88,7 @@ struct IcgArgs {
     double rtol;
     int maxit;
     int zero_on_break;   // z = 0 on a breakdown (a solver's own buffer), else z is left as it is
+    long long wait_polls;   // LIMITED: polls of each wait before the solve gives up (IGA_ERR_TIMEOUT)
     DevScalars *s;
 };
 
@@ -123,10 +124,10 @@ __device__ __forceinline__ void cluster_store(uint32_t a, double2 v, uint32_t ba
                  : "memory");
 }
 // Bounded wait of a whole warp: the same answer in every lane.
-__device__ __forceinline__ bool cluster_wait(uint64_t *bar, uint32_t parity)
+__device__ __forceinline__ bool cluster_wait(uint64_t *bar, uint32_t parity, long long limit = kWaitLimit)
 {
     bool done = false;
-    for (long long it = 0; it < kWaitLimit; ++it) {
+    for (long long it = 0; it < limit; ++it) {
         uint32_t ok;
         asm volatile(
             "{\n\t.reg .pred p;\n\t"
@@ -150,7 +151,9 @@ __device__ __forceinline__ double warp_sum(double v)
     return v;
 }
 
-template <typename T, int L>
+// LIMITED: with a limit of the caller's on each wait, in place of kWaitLimit (a
+// limit the compiler does not know costs 0.1 us an iteration).
+template <typename T, int L, bool LIMITED>
 __global__ void __launch_bounds__(kIcgMaxThreads, 1) icg_cluster_kernel(IcgArgs<T> a)
 {
     pdl_begin();
@@ -238,19 +241,20 @@ __global__ void __launch_bounds__(kIcgMaxThreads, 1) icg_cluster_kernel(IcgArgs<
         const double2 v = make_double2(warp_sum(va), warp_sum(vb));
         if (lane < C) cluster_store(cluster_addr(red2 + rank * nw + wid, lane), v, cluster_addr(&bar[1], lane));
     };
+    const long long limit = LIMITED ? a.wait_polls : kWaitLimit;
     bool ok = true;
-    auto total1 = [&]() -> double {
-        ok = cluster_wait(&bar[0], ph1);
-        ph1 ^= 1u;
-        if (t == 0) mbar_arrive_expect_tx(&bar[0], tx1);
+    auto sum1 = [&]() -> double {
         double v = 0.0;
         for (int u = lane; u < C * nw; u += 32) v += red1[u];
         return warp_sum(v);
     };
-    auto total2 = [&](double &va, double &vb) {
-        ok = cluster_wait(&bar[1], ph2);
-        ph2 ^= 1u;
-        if (t == 0) mbar_arrive_expect_tx(&bar[1], tx2 + txh);
+    auto total1 = [&]() -> double {
+        ok = cluster_wait(&bar[0], ph1, limit);
+        ph1 ^= 1u;
+        if (t == 0 && ok) mbar_arrive_expect_tx(&bar[0], tx1);
+        return sum1();
+    };
+    auto sum2 = [&](double &va, double &vb) {
         va = vb = 0.0;
         for (int u = lane; u < C * nw; u += 32) {
             const double2 w = red2[u];
@@ -260,13 +264,25 @@ __global__ void __launch_bounds__(kIcgMaxThreads, 1) icg_cluster_kernel(IcgArgs<
         va = warp_sum(va);
         vb = warp_sum(vb);
     };
+    auto total2 = [&](double &va, double &vb) {
+        ok = cluster_wait(&bar[1], ph2, limit);
+        ph2 ^= 1u;
+        if (t == 0 && ok) mbar_arrive_expect_tx(&bar[1], tx2 + txh);
+        sum2(va, vb);
+    };
+    // the CTA's warps meet on an mbarrier too, so that a warp whose wait gave
+    // up cannot leave the others at a barrier
+    auto arrive3 = [&] {
+        __syncwarp();
+        if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(&bar[2])) : "memory");
+    };
 
     cluster_barrier();   // every CTA of the cluster has set up its mbarriers; p is in place
     post2(v0, v1);
     double rz, rr;
     total2(rz, rr);
     const double tol2 = a.rtol * a.rtol * rr;
-    int its = 0, brk = 0;
+    int its = 0, brk = 0, gave = ok ? -1 : 1;   // gave: the mbarrier this warp gave up at
     if (ok && rr != 0.0) {
         double inv_rz = 1.0 / rz;
         for (;;) {
@@ -305,6 +321,7 @@ __global__ void __launch_bounds__(kIcgMaxThreads, 1) icg_cluster_kernel(IcgArgs<
             pq = total1();
             if (!ok || !(pq > 0.0)) {
                 brk = 1;
+                gave = 0;
                 break;
             }
             const T al = (T)(rz / pq);
@@ -329,7 +346,10 @@ __global__ void __launch_bounds__(kIcgMaxThreads, 1) icg_cluster_kernel(IcgArgs<
             const T be = (T)(rz * inv_old);
             inv_rz = 1.0 / rz;   // next iteration's, off the critical path
             ++its;
-            if (!ok || rr <= tol2 || its >= a.maxit || !(rr == rr)) break;
+            if (!ok || rr <= tol2 || its >= a.maxit || !(rr == rr)) {
+                gave = 1;
+                break;
+            }
 #pragma unroll
             for (int l = 0; l < L; ++l) {
                 if (l < cnt) {
@@ -344,14 +364,43 @@ __global__ void __launch_bounds__(kIcgMaxThreads, 1) icg_cluster_kernel(IcgArgs<
                     *pp = fma(be, *pp, hz[u]);
                 }
             }
-            // the CTA's warps meet on an mbarrier too, so that a wait that
-            // gave up in one warp cannot leave the others at a barrier
-            __syncwarp();
-            if (lane == 0)
-                asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(&bar[2])) : "memory");
-            ok = __all_sync(0xffffffffu, mbar_wait_bounded(&bar[2], ph3));
+            arrive3();
+            ok = __all_sync(0xffffffffu, mbar_wait_bounded(&bar[2], ph3, limit));
             ph3 ^= 1u;
-            if (!ok) break;
+            if (!ok) {
+                gave = 2;
+                break;
+            }
+        }
+    }
+    // No CTA may leave while stores are on their way into its shared memory. So
+    // a warp that gave up lets that exchange land, with the full limit, and
+    // unless its totals end the solve anyway sends NaN in the next one and lets
+    // that land too: the NaN ends the solve in every CTA there, with every
+    // exchange complete.
+    if (!ok) {
+        bool landed = gave == 2 ? __all_sync(0xffffffffu, mbar_wait_bounded(&bar[2], ph3 ^ 1u)) != 0
+                                : cluster_wait(&bar[gave], (gave == 0 ? ph1 : ph2) ^ 1u);
+        if (gave == 0 && landed && sum1() > 0.0) {
+#pragma unroll
+            for (int l = 0; l < L; ++l) {
+                if (l >= cnt) continue;
+                const int k = k0 + l;
+                if (k == 0 && rank > 0) cluster_store(cluster_addr(hz + m + i, rank - 1), T(0), cluster_addr(&bar[1], rank - 1));
+                if (k == nr - 1 && j0 + nr < n) cluster_store(cluster_addr(hz + i, rank + 1), T(0), cluster_addr(&bar[1], rank + 1));
+            }
+            post2(nan(""), nan(""));
+            cluster_wait(&bar[1], ph2);
+        }
+        if (gave == 1 && landed) {
+            sum2(rz, rr);
+            if (its == 0) landed = rr != 0.0;
+            else landed = !(rr <= tol2 || its >= a.maxit || !(rr == rr));
+            if (landed && its > 0) arrive3();
+        }
+        if (gave > 0 && landed) {
+            post1(nan(""));
+            cluster_wait(&bar[0], ph1);
         }
     }
     if ((!brk && ok) || a.zero_on_break) {
@@ -359,14 +408,13 @@ __global__ void __launch_bounds__(kIcgMaxThreads, 1) icg_cluster_kernel(IcgArgs<
         for (int l = 0; l < L; ++l)
             if (l < cnt) a.z[(size_t)(j0 + k0 + l) * m + i] = brk || !ok ? T(0) : z[l];
     }
-    if (!ok) a.s->err = a.s->breakdown = 1;   // a bounded wait gave up
+    if (!ok) a.s->err = a.s->breakdown = 1;
     if (rank == 0 && t == 0) {
         a.s->iiters = its;
         a.s->ipc += its;
         if (brk && ok) a.s->ibreak = a.s->breakdown = 1;
     }
-    // no CTA leaves while another may still store into its shared memory (a
-    // CTA whose wait gave up leaves early)
+    // no CTA leaves while another may still store into its shared memory
     cluster_barrier();
 }
 

@@ -1075,6 +1075,7 @@ struct PrecState {
     // iteration per pass (built for one preconditioner / kappa-scaling choice)
     cudaGraphExec_t loop = nullptr;
     int loop_pc = -1, loop_scaled = -1, loop_prec = -1;
+    long long loop_wait_polls = -1;   // the plan's limit on the kernels' waits
     double loop_pc_rtol = 0.0;   // IGA_PC_FEM_CG: the inner solve's parameters in the loop
     int loop_pc_max_it = 0;
     IcgShape icg;                // IGA_PC_FEM_CG in one cluster (C = 0: the grid does not fit)
@@ -1189,11 +1190,20 @@ void net_lengths(const Patch &P, double &Lx, double &Ly)
         }                                                                            \
     } while (0)
 
-template <typename T>
+template <typename T, bool LIMITED>
 static void (*icg_kernel(int L))(IcgArgs<T>)
 {
-    return L == 1 ? icg_cluster_kernel<T, 1> : L == 2 ? icg_cluster_kernel<T, 2> : L == 4 ? icg_cluster_kernel<T, 4>
-                                                                                           : icg_cluster_kernel<T, 8>;
+    return L == 1   ? icg_cluster_kernel<T, 1, LIMITED>
+           : L == 2 ? icg_cluster_kernel<T, 2, LIMITED>
+           : L == 4 ? icg_cluster_kernel<T, 4, LIMITED>
+                    : icg_cluster_kernel<T, 8, LIMITED>;
+}
+
+// The kernel for a plan with or without a limit of its own on the waits.
+template <typename T>
+static auto icg_kernel(int L, bool limited)
+{
+    return limited ? icg_kernel<T, true>(L) : icg_kernel<T, false>(L);
 }
 
 // The cluster shape of the inner FEM-CG for this plan's grid: the first one
@@ -1206,12 +1216,17 @@ static int icg_prepare(PrecState<T> &ps, const iga_plan *pl)
     for (int k = 0; k < 4; ++k) {
         const IcgShape sh = icg_shape<T>(pl->m, pl->n, k);
         if (!sh.C) continue;
-        auto kern = icg_kernel<T>(sh.L);
-        if (sh.C > 8 && cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) {
+        auto kern = icg_kernel<T>(sh.L, false);
+        bool wide = true;
+        for (bool limited : {false, true}) {
+            auto k2 = icg_kernel<T>(sh.L, limited);
+            if (sh.C > 8) wide &= cudaFuncSetAttribute(k2, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess;
+            SOLVE_TRY(cudaFuncSetAttribute(k2, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kIcgMaxSmem));
+        }
+        if (!wide) {
             cudaGetLastError();
             continue;
         }
-        SOLVE_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kIcgMaxSmem));
         cudaLaunchConfig_t cfg = {};
         cfg.gridDim = dim3(sh.C);
         cfg.blockDim = dim3(sh.threads);
@@ -1756,6 +1771,7 @@ static int pc_apply_core(PrecState<T> &ps, const iga_plan *pl, SolverState *S, c
         a.rtol = pc_rtol;
         a.maxit = o.pc_max_it;
         a.zero_on_break = !S->pc_sync;
+        a.wait_polls = pl->wait_polls;
         a.s = S->s;
         cudaLaunchConfig_t cfg = {};
         cfg.gridDim = dim3(ps.icg.C);
@@ -1774,7 +1790,7 @@ static int pc_apply_core(PrecState<T> &ps, const iga_plan *pl, SolverState *S, c
             SOLVE_TRY(cudaMemsetAsync(&S->s->ibreak, 0, sizeof(int), S->stream));
             SOLVE_TRY(cudaMemsetAsync(&S->s->err, 0, sizeof(int), S->stream));
         }
-        SOLVE_TRY(cudaLaunchKernelEx(&cfg, icg_kernel<T>(ps.icg.L), a));
+        SOLVE_TRY(cudaLaunchKernelEx(&cfg, icg_kernel<T>(ps.icg.L, pl->wait_polls >= 0), a));
         if (S->pc_sync) {
             if ((st = sync_scalars(S))) return st;
             if (S->h->err) {
@@ -1858,7 +1874,8 @@ static int build_loop(iga_plan *pl, SolverState *S, PrecState<T> &ps, const iga_
     const int scaled = pl->kappa_dev ? 1 : 0;
     const bool same_pc = ps.loop_pc == o.pc && (o.pc != IGA_PC_FEM_CG || (ps.loop_pc_rtol == o.pc_rtol &&
                                                                          ps.loop_pc_max_it == o.pc_max_it));
-    if (same_pc && ps.loop_scaled == scaled && ps.loop_prec == o.precision && (ps.loop || ps.loop_failed))
+    if (same_pc && ps.loop_scaled == scaled && ps.loop_prec == o.precision && ps.loop_wait_polls == pl->wait_polls &&
+        (ps.loop || ps.loop_failed))
         return ps.loop ? IGA_OK : IGA_ERR_UNSUPPORTED;
     if (ps.loop) {
         cudaGraphExecDestroy(ps.loop);
@@ -1935,6 +1952,7 @@ static int build_loop(iga_plan *pl, SolverState *S, PrecState<T> &ps, const iga_
         ps.loop_pc = o.pc;
         ps.loop_scaled = scaled;
         ps.loop_prec = o.precision;
+        ps.loop_wait_polls = pl->wait_polls;
         ps.loop_pc_rtol = o.pc_rtol;
         ps.loop_pc_max_it = o.pc_max_it;
         ps.loop_failed = true;
@@ -1945,6 +1963,7 @@ static int build_loop(iga_plan *pl, SolverState *S, PrecState<T> &ps, const iga_
     ps.loop_pc = o.pc;
     ps.loop_scaled = scaled;
     ps.loop_prec = o.precision;
+    ps.loop_wait_polls = pl->wait_polls;
     ps.loop_pc_rtol = o.pc_rtol;
     ps.loop_pc_max_it = o.pc_max_it;
     return IGA_OK;
@@ -2300,11 +2319,16 @@ int iga_spectrum_estimate(iga_plan *pl, int pc, int steps, uint64_t seed, double
     int64_t pcits = 0;
     SOLVE_TRY(cudaMemsetAsync(&S->s->breakdown, 0, sizeof(int), s));
     SOLVE_TRY(cudaMemsetAsync(&S->s->ibreak, 0, sizeof(int), s));
+    SOLVE_TRY(cudaMemsetAsync(&S->s->err, 0, sizeof(int), s));
+    auto pc_status = [&] {   // of the preconditioner's kernels up to the last sync_scalars
+        if (S->h->err) set_error("a bounded device wait gave up in the preconditioner");
+        return S->h->err ? IGA_ERR_TIMEOUT : S->h->ibreak ? IGA_ERR_BREAKDOWN : IGA_OK;
+    };
     if ((st = pc_apply(ps, pl, S, o, ps.r, ps.z, o.pc_rtol, pcits))) return st;
     dot_kernel<double><<<kRedBlocks, kThreads, 0, s>>>(ps.r, ps.z, N, &S->s->rz, S->partials, S->counter);
     pcg_p_kernel<double><<<kRedBlocks, kThreads, 0, s>>>(ps.p, ps.z, N, S->s, 1);
     if ((st = sync_scalars(S))) return st;
-    if (S->h->ibreak) return IGA_ERR_BREAKDOWN;
+    if ((st = pc_status())) return st;
     const double rr0 = S->h->rz;
     std::vector<double> alpha, beta;
     for (int k = 0; k < steps; ++k) {
@@ -2316,7 +2340,7 @@ int iga_spectrum_estimate(iga_plan *pl, int pc, int steps, uint64_t seed, double
         if ((st = pc_apply(ps, pl, S, o, ps.r, ps.z, o.pc_rtol, pcits))) return st;
         dot_kernel<double><<<kRedBlocks, kThreads, 0, s>>>(ps.r, ps.z, N, &S->s->rz, S->partials, S->counter);
         if ((st = sync_scalars(S))) return st;
-        if (S->h->ibreak) return IGA_ERR_BREAKDOWN;
+        if ((st = pc_status())) return st;
         if (S->h->breakdown || !(S->h->alpha > 0.0)) break;
         alpha.push_back(S->h->alpha);
         const double rz_new = S->h->rz;

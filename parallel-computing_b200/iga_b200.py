@@ -633,7 +633,7 @@ class Plan:
         _check(_lib().iga_plan_set_solver_graph(self.h, int(enable)), "iga_plan_set_solver_graph")
 
     def set_wait_limit(self, polls):
-        """Test hook: polls per bounded wait of the MatMult kernel (< 0: default)."""
+        """Test hook: polls per bounded wait of the MatMult and inner FEM-CG kernels (< 0: default)."""
         _check(_lib().iga_plan_set_wait_limit(self.h, int(polls)), "iga_plan_set_wait_limit")
 
     def set_pc_split(self, enable):

@@ -57,3 +57,48 @@ def test_plans_of_several_sizes_together(torch_cuda, ib, prec):
         plan.pc_apply(r, z2, pc=ib.PC_FEM_CG, precision=prec, pc_rtol=1e-3)
         assert torch.equal(z, z2)
         plan.close()
+
+
+# Waits that run out at once: IGA_ERR_TIMEOUT, z as it was, and the plan
+# solves on as before, its loop included (sizes of 1, 8 and 16 CTAs).
+@pytest.mark.parametrize("prec", [0, 1])
+@pytest.mark.parametrize("nex,ney", [(40, 33), (20, 1), (255, 62), (3, 1200)])
+def test_waits_that_run_out(torch_cuda, ib, nex, ney, prec):
+    torch = torch_cuda
+    mesh = ib.unit_square(1, nex, ney)
+    plan = ib.Plan(mesh)
+    r = random_vector(torch, plan, nex, torch.float32 if prec else torch.float64)
+    z = torch.full_like(r, float("nan"))
+    tol = 1e-3 if prec else 1e-10
+    plan.pc_apply(r, z, pc=ib.PC_FEM_CG, precision=prec, pc_rtol=tol)
+    plan.set_wait_limit(0)
+    for _ in range(2):
+        z2 = torch.full_like(r, 3.0)
+        with pytest.raises(ib.IgaError) as e:
+            plan.pc_apply(r, z2, pc=ib.PC_FEM_CG, precision=prec, pc_rtol=tol)
+        assert e.value.status == 8   # IGA_ERR_TIMEOUT
+        assert torch.equal(z2, torch.full_like(r, 3.0))
+    for polls in (1, 2, 4, 8, 16, 64):   # some waits end in time, others run out
+        plan.set_wait_limit(polls)
+        for _ in range(5):
+            z2 = torch.full_like(r, 3.0)
+            try:
+                plan.pc_apply(r, z2, pc=ib.PC_FEM_CG, precision=prec, pc_rtol=tol)
+                assert torch.equal(z, z2)
+            except ib.IgaError as e:
+                assert e.status == 8
+    plan.set_wait_limit(0)
+    if not prec:
+        b, x = free_vector(torch, mesh, 2), torch.zeros(plan.nfunc, dtype=torch.float64, device="cuda")
+        if float(b.abs().max()) > 0.0:
+            assert plan.solve(b, x, check=False, pc=ib.PC_FEM_CG, max_it=3).status != 0
+        with pytest.raises(ib.IgaError):
+            plan.spectrum(pc=ib.PC_FEM_CG, steps=3)
+    plan.set_wait_limit(-1)
+    plan.device_status()   # the MatMult's waits ran out too
+    z2 = torch.full_like(r, float("nan"))
+    plan.pc_apply(r, z2, pc=ib.PC_FEM_CG, precision=prec, pc_rtol=tol)
+    assert torch.equal(z, z2)
+    if not prec and float(b.abs().max()) > 0.0:
+        assert plan.solve(b, x, pc=ib.PC_FEM_CG, max_it=50).relres <= 1e-10
+    plan.close()
