@@ -1997,6 +1997,9 @@ static int pcg_graph(iga_plan *pl, SolverState *S, PrecState<T> &ps, const iga_s
         if ((st = sync_scalars(S))) return st;
         if (std::sqrt(S->h->rr) <= rtol * bnorm) return IGA_OK;
     }
+    // the graph's body runs at least once; a solve with the inner FEM-CG that
+    // is asked for no iteration does none, on grids of any size
+    if (o.pc == IGA_PC_FEM_CG && o.max_it <= 0) return IGA_ERR_NOT_CONVERGED;
     st = pl->solver_graph ? build_loop(pl, S, ps, o, prec) : IGA_ERR_UNSUPPORTED;
     if (st == IGA_ERR_UNSUPPORTED) {   // e.g. a library kernel not allowed in a conditional body, or the host loop asked for
         int64_t pcits = 0;   // the cluster FEM-CG counts on the device

@@ -102,3 +102,17 @@ def test_waits_that_run_out(torch_cuda, ib, nex, ney, prec):
     if not prec and float(b.abs().max()) > 0.0:
         assert plan.solve(b, x, pc=ib.PC_FEM_CG, max_it=50).relres <= 1e-10
     plan.close()
+
+
+# No outer iteration asked for: none done, x as it was.
+@pytest.mark.parametrize("prec", ["FP64", "MIXED", "MIXED_PC"])
+def test_no_outer_iteration(torch_cuda, ib, prec):
+    torch = torch_cuda
+    mesh = ib.unit_square(2, 40, 33)
+    plan = ib.Plan(mesh, precision=ib.MIXED)
+    b, x0 = free_vector(torch, mesh, 4), free_vector(torch, mesh, 5)
+    x = x0.clone()
+    st = plan.solve(b, x, check=False, precision=getattr(ib, prec), pc=ib.PC_FEM_CG, max_it=0, x0_nonzero=1)
+    assert st.status == 5 and st.iterations == 0   # IGA_ERR_NOT_CONVERGED
+    assert torch.equal(x, x0)
+    plan.close()
