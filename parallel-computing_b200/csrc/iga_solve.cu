@@ -499,8 +499,8 @@ __global__ void __launch_bounds__(kThreads) loop_p_kernel(T *__restrict__ p, con
 }
 
 // alpha = rz / p.q (zero, and a breakdown, unless p.q > 0); the update; counts
-// the iteration and sets the loop's condition (continue while rr > tol2, it <
-// maxit, no breakdown, finite).
+// the iteration (unless the preconditioner broke down) and sets the loop's
+// condition (continue while rr > tol2, it < maxit, no breakdown, finite).
 template <typename T>
 __global__ void __launch_bounds__(kThreads)
     loop_xr_kernel(T *__restrict__ x, T *__restrict__ r, const T *__restrict__ p, const T *__restrict__ q,
@@ -509,7 +509,8 @@ __global__ void __launch_bounds__(kThreads)
 {
     pdl_begin();
     const double pq = sum_partials(part, np);
-    const bool bad = !(pq > 0.0) || s->breakdown;   // breakdown already set: by the preconditioner
+    const bool pc_bad = s->breakdown;   // set by the preconditioner
+    const bool bad = !(pq > 0.0) || pc_bad;
     const double alpha = bad ? 0.0 : s->rzv[s->it & 1] / pq;
     double tot[2];
     if (xr_update(x, r, p, q, z, N, (T)alpha, partials, counter, tot) && threadIdx.x == 0) {
@@ -517,7 +518,7 @@ __global__ void __launch_bounds__(kThreads)
         if (bad) s->breakdown = 1;
         s->rr = tot[0];
         s->rzo = tot[1];
-        s->it += 1;
+        if (!pc_bad) s->it += 1;
         const bool go = tot[0] > s->tol2 && s->it < s->maxit && !bad && tot[0] == tot[0];
         cudaGraphSetConditional(h, go ? 1u : 0u);
     }

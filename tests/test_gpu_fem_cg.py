@@ -116,3 +116,21 @@ def test_no_outer_iteration(torch_cuda, ib, prec):
     assert st.status == 5 and st.iterations == 0   # IGA_ERR_NOT_CONVERGED
     assert torch.equal(x, x0)
     plan.close()
+
+
+# A right-hand side whose first inner p.Kp underflows to zero (2.3e-162 squared
+# over diag = 8/3 is under half the smallest double): the preconditioner breaks
+# down before any outer iteration.
+def test_inner_breakdown_ends_the_solve(torch_cuda, ib):
+    torch = torch_cuda
+    plan = ib.Plan(ib.unit_square(2, 64, 64))
+    b = torch.zeros(plan.nfunc, dtype=torch.float64, device="cuda")
+    b[33 * 66 + 33] = 2.3e-162
+    x = torch.full_like(b, 1.0)
+    st = plan.solve(b, x, check=False, pc=ib.PC_FEM_CG)
+    assert st.status == 6 and st.iterations == 0   # IGA_ERR_BREAKDOWN
+    assert float(x.abs().max()) == 0.0
+    # and the plan solves on
+    b = free_vector(torch, plan.mesh, 6)
+    assert plan.solve(b, x, pc=ib.PC_FEM_CG).relres <= 1e-10
+    plan.close()
