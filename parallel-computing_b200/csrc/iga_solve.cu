@@ -38,7 +38,7 @@ struct DevScalars {
     int err;                                        // a bounded wait in a kernel gave up
     int it, maxit;                                  // outer PCG in a device-side loop
     long long ipc;                                  // inner iterations of one call's cluster FEM-CG solves
-    double rzv[2];                                  // r.z of the device-side loop's even / odd iterations
+    double rzv[2];                                  // r.z of the PCG loop's even / odd iterations
 };
 
 }  // namespace iga
@@ -393,7 +393,8 @@ __global__ void dot_kernel(const T *__restrict__ a, const T *__restrict__ b, lon
     if (reduce_last<1>(v, partials, counter, tot) && threadIdx.x == 0) *out = tot[0];
 }
 
-// ---- the host-driven loop's kernels (each dot product's total in S)
+// ---- the Lanczos process's kernels (iga_spectrum_estimate: the host reads each
+// dot product's total from S)
 // alpha = rz / (p.q) from the device scalars
 template <typename T>
 __global__ void pcg_pq_kernel(const T *__restrict__ p, const T *__restrict__ q, long long N, DevScalars *s,
@@ -456,7 +457,7 @@ __global__ void pcg_xr_kernel(T *__restrict__ x, T *__restrict__ r, const T *__r
     }
 }
 
-// ---- the device-side loop's kernels: dot products as block partials, summed
+// ---- the PCG loop's kernels: dot products as block partials, summed
 // by the kernel that uses them (sum_partials); r.z of iteration `it` in
 // rzv[it & 1], so that no block reads a scalar another block has replaced
 template <typename T>
@@ -498,14 +499,21 @@ __global__ void __launch_bounds__(kThreads) loop_p_kernel(T *__restrict__ p, con
     });
 }
 
+// The device-side loop's condition (on = 0: the host drives the loop).
+struct LoopCond {
+    cudaGraphConditionalHandle h = 0;
+    int on = 0;
+};
+
 // alpha = rz / p.q (zero, and a breakdown, unless p.q > 0); the update; counts
 // the iteration (unless the preconditioner broke down) and sets the loop's
-// condition (continue while rr > tol2, it < maxit, no breakdown, finite).
+// condition (continue while rr > tol2, it < maxit, no breakdown, finite) where
+// the loop runs on the device.
 template <typename T>
 __global__ void __launch_bounds__(kThreads)
     loop_xr_kernel(T *__restrict__ x, T *__restrict__ r, const T *__restrict__ p, const T *__restrict__ q,
                    const T *__restrict__ z, long long N, DevScalars *s, const double *part, int np, double *partials,
-                   unsigned *counter, cudaGraphConditionalHandle h)
+                   unsigned *counter, LoopCond cond)
 {
     pdl_begin();
     const double pq = sum_partials(part, np);
@@ -520,7 +528,7 @@ __global__ void __launch_bounds__(kThreads)
         s->rzo = tot[1];
         if (!pc_bad) s->it += 1;
         const bool go = tot[0] > s->tol2 && s->it < s->maxit && !bad && tot[0] == tot[0];
-        cudaGraphSetConditional(h, go ? 1u : 0u);
+        if (cond.on) cudaGraphSetConditional(cond.h, go ? 1u : 0u);
     }
 }
 
@@ -532,27 +540,7 @@ __global__ void loop_init_kernel(DevScalars *s, double tol2, int maxit)
     s->breakdown = 0;
 }
 
-// Flexible (Polak-Ribiere) beta = r.(z - z_old) / rz_old with r.z_old = rzo
-// from the update kernel; rz = r.z.
-template <typename T>
-__global__ void pcg_beta_kernel(const T *__restrict__ r, const T *__restrict__ z, long long N, DevScalars *s,
-                                double *partials, unsigned *counter)
-{
-    pdl_begin();
-    double v[1] = {0.0};
-    vloop<T>(N, al16(r) && al16(z), [&](long long i, int c) {
-        const Pk<T> a = ldc(r, i, c), b = ldc(z, i, c);
-#pragma unroll
-        for (int k = 0; k < Pk<T>::n; ++k)
-            if (k < c) v[0] += (double)a.v[k] * (double)b.v[k];
-    });
-    double tot[1];
-    if (reduce_last<1>(v, partials, counter, tot) && threadIdx.x == 0) {
-        s->beta = (tot[0] - s->rzo) / s->rz;
-        s->rz = tot[0];
-    }
-}
-
+// p = z + beta p (first: p = z)
 template <typename T>
 __global__ void pcg_p_kernel(T *__restrict__ p, const T *__restrict__ z, long long N, const DevScalars *s, int first)
 {
@@ -1829,46 +1817,45 @@ static int pc_apply_core(PrecState<T> &ps, const iga_plan *pl, SolverState *S, c
     return IGA_OK;
 }
 
-// Flexible PCG on K x = b in precision T, from the current x; stops when the
-// recurrence residual satisfies ||r|| <= rtol ||b_ref||. Returns iterations.
+// One iteration of the flexible PCG on the fixed buffers of ps: z = M^-1 r;
+// beta; p = z + beta p (p = z in the first); q = K p; alpha; x += alpha p, r -=
+// alpha q, r.z. With the preconditioner first no iteration ends on one whose
+// result nobody reads (a 12-iteration solve of four sweeps otherwise applies it
+// 16 times). Both loops, the device's and the host's, are made of it.
 template <typename T>
-static int pcg(iga_plan *pl, SolverState *S, PrecState<T> &ps, const iga_solve_opts &o, const T *b, T *x, double rtol,
-               double bnorm, double pc_rtol, int prec, int &its, int64_t &pc_iters)
+static int pcg_step(iga_plan *pl, SolverState *S, PrecState<T> &ps, const iga_solve_opts &o, int prec, LoopCond cond,
+                    int64_t &pc_iters)
 {
     const long long N = pl->nfunc;
     const cudaStream_t s = S->stream;
-    int st;
-    // r = b - K x, rr = r.r
-    if ((st = iga_apply_internal_sb(pl, prec, x, ps.q, s, IGA_SIGN_SPD, IGA_BC_IDENTITY))) return st;
-    sub_kernel<T><<<kRedBlocks, kThreads, 0, s>>>(b, ps.q, ps.r, N, S->s, S->partials, S->counter);
-    if ((st = sync_scalars(S))) return st;
-    if (std::sqrt(S->h->rr) <= rtol * bnorm) return IGA_OK;
-    cudaMemsetAsync(&S->s->breakdown, 0, sizeof(int), s);
-    if ((st = pc_apply(ps, pl, S, o, ps.r, ps.z, pc_rtol, pc_iters))) return st;
-    dot_kernel<T><<<kRedBlocks, kThreads, 0, s>>>(ps.r, ps.z, N, &S->s->rz, S->partials, S->counter);
-    pcg_p_kernel<T><<<kRedBlocks, kThreads, 0, s>>>(ps.p, ps.z, N, S->s, 1);
-    for (int it = 0; it < o.max_it; ++it) {
-        if ((st = iga_apply_internal_sb(pl, prec, ps.p, ps.q, s, IGA_SIGN_SPD, IGA_BC_IDENTITY))) return st;
-        pcg_pq_kernel<T><<<kRedBlocks, kThreads, 0, s>>>(ps.p, ps.q, N, S->s, S->partials, S->counter);
-        pcg_xr_kernel<T><<<kRedBlocks, kThreads, 0, s>>>(x, ps.r, ps.p, ps.q, ps.z, N, S->s, S->partials,
-                                                         S->counter);
-        ++its;
-        if ((st = sync_scalars(S))) return st;
-        if (S->h->breakdown) return IGA_ERR_BREAKDOWN;
-        if (!std::isfinite(S->h->rr)) return IGA_ERR_NONFINITE;
-        if (std::sqrt(S->h->rr) <= rtol * bnorm) return IGA_OK;
-        if ((st = pc_apply(ps, pl, S, o, ps.r, ps.z, pc_rtol, pc_iters))) return st;
-        pcg_beta_kernel<T><<<kRedBlocks, kThreads, 0, s>>>(ps.r, ps.z, N, S->s, S->partials, S->counter);
-        pcg_p_kernel<T><<<kRedBlocks, kThreads, 0, s>>>(ps.p, ps.z, N, S->s, 0);
+    DotPart rz;
+    rz.part = S->part_rz();
+    int st = pc_apply(ps, pl, S, o, ps.r, ps.z, o.pc_rtol, pc_iters, &rz);
+    if (st) return st;
+    const int nb = vec_blocks<T>(N);
+    // the vector kernels of vectors of 4 MB or more get ordinary edges: their
+    // blocks run long enough for an uneven start to cost more than a launch
+    // gap (1024^2 mixed 118.8 -> 117 us an iteration, 2048^2 FP64 1111 -> 1100;
+    // 512^2 FP64 97.7 -> 99.5)
+    const bool even = N * (long long)sizeof(T) >= (4LL << 20);
+    auto launch_vec = [&](auto kern, auto... args) {
+        return even ? launch_even(kern, dim3(nb), dim3(kThreads), 0, s, args...)
+                    : launch_k(kern, dim3(nb), dim3(kThreads), 0, s, args...);
+    };
+    if (rz.n == 0) {   // no preconditioner that took r . z itself
+        SOLVE_TRY(launch_vec(loop_dot_kernel<T>, (const T *)ps.r, (const T *)ps.z, N, rz.part));
+        rz.n = nb;
     }
-    return IGA_ERR_NOT_CONVERGED;
+    SOLVE_TRY(launch_vec(loop_p_kernel<T>, ps.p, (const T *)ps.z, N, S->s, (const double *)rz.part, rz.n));
+    if ((st = iga_apply_internal_sb(pl, prec, ps.p, ps.q, s, IGA_SIGN_SPD, IGA_BC_IDENTITY))) return st;
+    SOLVE_TRY(launch_vec(loop_dot_kernel<T>, (const T *)ps.p, (const T *)ps.q, N, S->part_pq()));
+    SOLVE_TRY(launch_vec(loop_xr_kernel<T>, ps.x, ps.r, (const T *)ps.p, (const T *)ps.q, (const T *)ps.z, N, S->s,
+                         (const double *)S->part_pq(), nb, S->partials, S->counter, cond));
+    return IGA_OK;
 }
 
-// Builds the device-side loop for the current preconditioner choice: body =
-// z = M^-1 r; beta; p = z + beta p (p = z in the first pass); q = K p; alpha;
-// x += alpha p, r -= alpha q, r.z (+ loop condition), on the fixed buffers of
-// ps. With the preconditioner first no pass ends on one whose result nobody
-// reads (a 12-iteration solve of four sweeps otherwise applies it 16 times).
+// Builds the device-side loop for the current preconditioner choice: its body
+// is one pcg_step().
 template <typename T>
 static int build_loop(iga_plan *pl, SolverState *S, PrecState<T> &ps, const iga_solve_opts &o, int prec)
 {
@@ -1882,7 +1869,6 @@ static int build_loop(iga_plan *pl, SolverState *S, PrecState<T> &ps, const iga_
         cudaGraphExecDestroy(ps.loop);
         ps.loop = nullptr;
     }
-    const long long N = pl->nfunc;
     const cudaStream_t s = S->stream;
     cudaGraph_t g;
     SOLVE_TRY(cudaGraphCreate(&g, 0));
@@ -1900,38 +1886,10 @@ static int build_loop(iga_plan *pl, SolverState *S, PrecState<T> &ps, const iga_
     int64_t dummy = 0;
     // Programmatic dependencies between the body's kernels.
     pdl_capture() = true;
-    DotPart rz;
-    rz.part = S->part_rz();
-    int st = pc_apply(ps, pl, S, o, ps.r, ps.z, o.pc_rtol, dummy, &rz);
-    const int nb = vec_blocks<T>(N);
-    // the vector kernels of vectors of 4 MB or more get ordinary edges: their
-    // blocks run long enough for an uneven start to cost more than a launch
-    // gap (1024^2 mixed 118.8 -> 117 us an iteration, 2048^2 FP64 1111 -> 1100;
-    // 512^2 FP64 97.7 -> 99.5)
-    const bool even = N * (long long)sizeof(T) >= (4LL << 20);
-    auto launch_vec = [&](auto kern, auto... args) {
-        return even ? launch_even(kern, dim3(nb), dim3(kThreads), 0, s, args...)
-                    : launch_k(kern, dim3(nb), dim3(kThreads), 0, s, args...);
-    };
-    auto launched = [&](cudaError_t e) {
-        if (e != cudaSuccess && !st) {
-            set_error(std::string("PCG loop launch: ") + cudaGetErrorString(e));
-            st = IGA_ERR_CUDA;
-        }
-    };
-    if (!st) {
-        if (rz.n == 0) {   // no preconditioner that took r . z itself
-            launched(launch_vec(loop_dot_kernel<T>, (const T *)ps.r, (const T *)ps.z, N, rz.part));
-            rz.n = nb;
-        }
-        launched(launch_vec(loop_p_kernel<T>, ps.p, (const T *)ps.z, N, S->s, (const double *)rz.part, rz.n));
-        if (!st) st = iga_apply_internal_sb(pl, prec, ps.p, ps.q, s, IGA_SIGN_SPD, IGA_BC_IDENTITY);
-    }
-    if (!st) {
-        launched(launch_vec(loop_dot_kernel<T>, (const T *)ps.p, (const T *)ps.q, N, S->part_pq()));
-        launched(launch_vec(loop_xr_kernel<T>, ps.x, ps.r, (const T *)ps.p, (const T *)ps.q, (const T *)ps.z, N, S->s,
-                            (const double *)S->part_pq(), nb, S->partials, S->counter, h));
-    }
+    LoopCond cond;
+    cond.h = h;
+    cond.on = 1;
+    const int st = pcg_step(pl, S, ps, o, prec, cond, dummy);
     pdl_capture() = false;
     cudaGraph_t captured = body;
     const cudaError_t ce = cudaStreamEndCapture(s, &captured);
@@ -1970,13 +1928,16 @@ static int build_loop(iga_plan *pl, SolverState *S, PrecState<T> &ps, const iga_
     return IGA_OK;
 }
 
-// Flexible PCG whose iterations run on the device: one graph launch per solve.
-// x_zero: x is known to be zero and b nonzero (a refinement sweep on the
+// Flexible PCG on K x = b in precision T, from the current x; stops when the
+// recurrence residual satisfies ||r|| <= rtol bnorm. Its iterations run on the
+// device, in one graph launch, or (host, and where a plan asks for it or the
+// graph cannot be had) one by one from the host, which reads the scalars after
+// each. x_zero: x is known to be zero and b nonzero (a refinement sweep on the
 // normalised residual): r = b without the operator and no host check before
 // the loop.
 template <typename T>
-static int pcg_graph(iga_plan *pl, SolverState *S, PrecState<T> &ps, const iga_solve_opts &o, const T *b, T *x,
-                     double rtol, double bnorm, int prec, int &its, bool x_zero = false)
+static int pcg(iga_plan *pl, SolverState *S, PrecState<T> &ps, const iga_solve_opts &o, const T *b, T *x, double rtol,
+               double bnorm, int prec, int &its, int64_t &pc_iters, bool host, bool x_zero = false)
 {
     const long long N = pl->nfunc;
     const cudaStream_t s = S->stream;
@@ -1998,22 +1959,31 @@ static int pcg_graph(iga_plan *pl, SolverState *S, PrecState<T> &ps, const iga_s
         if ((st = sync_scalars(S))) return st;
         if (std::sqrt(S->h->rr) <= rtol * bnorm) return IGA_OK;
     }
-    // the graph's body runs at least once; a solve with the inner FEM-CG that
-    // is asked for no iteration does none, on grids of any size
-    if (o.pc == IGA_PC_FEM_CG && o.max_it <= 0) return IGA_ERR_NOT_CONVERGED;
-    st = pl->solver_graph ? build_loop(pl, S, ps, o, prec) : IGA_ERR_UNSUPPORTED;
-    if (st == IGA_ERR_UNSUPPORTED) {   // e.g. a library kernel not allowed in a conditional body, or the host loop asked for
-        int64_t pcits = 0;   // the cluster FEM-CG counts on the device
-        st = pcg<T>(pl, S, ps, o, ps.b, ps.x, rtol, bnorm, o.pc_rtol, prec, its, pcits);
-        if (x != ps.x) copy_kernel<T><<<kRedBlocks, kThreads, 0, s>>>(x, ps.x, N);
-        return st;
+    if (!host) {
+        st = pl->solver_graph ? build_loop(pl, S, ps, o, prec) : IGA_ERR_UNSUPPORTED;
+        if (st && st != IGA_ERR_UNSUPPORTED) return st;
+        host = st != IGA_OK;   // e.g. a library kernel not allowed in a conditional body
     }
-    if (st) return st;
+    // the graph's body runs at least once; a solve from the host or with the
+    // inner FEM-CG that is asked for no iteration does none
+    if ((host || o.pc == IGA_PC_FEM_CG) && o.max_it <= 0) return IGA_ERR_NOT_CONVERGED;
     loop_init_kernel<<<1, 1, 0, s>>>(S->s, rtol * rtol * bnorm * bnorm, o.max_it);
-    SOLVE_TRY(cudaGraphLaunch(ps.loop, s));
+    st = IGA_OK;
+    if (host) {
+        const DevScalars &h = *S->h;
+        do {
+            if ((st = pcg_step(pl, S, ps, o, prec, LoopCond(), pc_iters))) break;
+            if ((st = sync_scalars(S))) return st;
+        } while (h.rr > h.tol2 && h.it < h.maxit && !h.breakdown && std::isfinite(h.rr));
+    } else {
+        SOLVE_TRY(cudaGraphLaunch(ps.loop, s));
+    }
     if (x != ps.x) copy_kernel<T><<<kRedBlocks, kThreads, 0, s>>>(x, ps.x, N);
+    if (st && st != IGA_ERR_BREAKDOWN) return st;
+    const int pc_st = st;   // IGA_ERR_BREAKDOWN: of an inner solve that the host drives
     if ((st = sync_scalars(S))) return st;
     its += S->h->it;
+    if (pc_st) return pc_st;
     if (S->h->breakdown) return IGA_ERR_BREAKDOWN;
     if (!std::isfinite(S->h->rr)) return IGA_ERR_NONFINITE;
     return std::sqrt(S->h->rr) <= rtol * bnorm ? IGA_OK : IGA_ERR_NOT_CONVERGED;
@@ -2227,10 +2197,7 @@ int iga_solve(iga_plan *pl, const double *b, double *x, const iga_solve_opts *o_
         for (int restart = 0; restart < 4 && rel > o.rtol; ++restart) {
             // the inner FEM-CG of grids past one cluster is driven by the host
             const bool host = o.pc == IGA_PC_FEM_CG && !(o.precision == IGA_MIXED_PC ? S->f.icg.C : S->d.icg.C);
-            st = host
-                     ? pcg<double>(pl, S, S->d, o, b, x, o.rtol, bnorm, o.pc_rtol, IGA_FP64, stt.iterations,
-                                   stt.pc_iterations)
-                     : pcg_graph<double>(pl, S, S->d, o, b, x, o.rtol, bnorm, IGA_FP64, stt.iterations);
+            st = pcg<double>(pl, S, S->d, o, b, x, o.rtol, bnorm, IGA_FP64, stt.iterations, stt.pc_iterations, host);
             if (st && st != IGA_ERR_NOT_CONVERGED) {
                 result = st;
                 break;
@@ -2254,10 +2221,9 @@ int iga_solve(iga_plan *pl, const double *b, double *x, const iga_solve_opts *o_
             const double srtol = std::max(o.sweep_rtol, std::min(0.2 * need, 0.5));
             scale_down_kernel<<<kRedBlocks, kThreads, 0, S->stream>>>(S->r64, S->f.b, N, S->s);
             zero_kernel<float><<<kRedBlocks, kThreads, 0, S->stream>>>(S->f.x, N);
-            st = o.pc == IGA_PC_FEM_CG && !S->f.icg.C
-                     ? pcg<float>(pl, S, S->f, o, S->f.b, S->f.x, srtol, 1.0, o.pc_rtol, IGA_FP32, stt.iterations,
-                                  stt.pc_iterations)
-                     : pcg_graph<float>(pl, S, S->f, o, S->f.b, S->f.x, srtol, 1.0, IGA_FP32, stt.iterations, true);
+            const bool host = o.pc == IGA_PC_FEM_CG && !S->f.icg.C;
+            st = pcg<float>(pl, S, S->f, o, S->f.b, S->f.x, srtol, 1.0, IGA_FP32, stt.iterations, stt.pc_iterations, host,
+                            true);
             if (st && st != IGA_ERR_NOT_CONVERGED) {
                 result = st;
                 break;

@@ -134,3 +134,32 @@ def test_inner_breakdown_ends_the_solve(torch_cuda, ib):
     b = free_vector(torch, plan.mesh, 6)
     assert plan.solve(b, x, pc=ib.PC_FEM_CG).relres <= 1e-10
     plan.close()
+
+
+# The solver's loop on the device and from the host: the same kernels in the
+# same order, so the same bits, iterations and inner iterations, with every
+# preconditioner and in every precision, with and without a kappa; and a
+# cap that ends both loops early.
+@pytest.mark.parametrize("prec", ["FP64", "MIXED", "MIXED_PC"])
+@pytest.mark.parametrize("pc", ["NONE", "FEM_EXACT", "FEM_CG"])
+@pytest.mark.parametrize("p,nex,ney", [(2, 40, 33), (3, 129, 70)])
+def test_device_and_host_loops_agree(torch_cuda, ib, p, nex, ney, pc, prec):
+    torch = torch_cuda
+    mesh = ib.unit_square(p, nex, ney)
+    plan = ib.Plan(mesh, precision=ib.MIXED)
+    b = free_vector(torch, mesh, p)
+    kappa = torch.from_numpy(splitmix_uniform(8, 0.5, 2.0, nex * ney * (p + 1) ** 2)).cuda()
+    for with_kappa in (False, True):
+        if with_kappa:
+            plan.set_kappa(kappa)
+        for max_it in (3, 40):
+            got = []
+            for graph in (1, 0):
+                plan.set_solver_graph(graph)
+                x = torch.zeros_like(b)
+                st = plan.solve(b, x, check=False, precision=getattr(ib, prec), pc=getattr(ib, "PC_" + pc),
+                                max_it=max_it)
+                got.append((x, st.status, st.iterations, st.pc_iterations, st.sweeps, st.relres))
+            assert got[0][1:] == got[1][1:]
+            assert torch.equal(got[0][0], got[1][0])
+    plan.close()
