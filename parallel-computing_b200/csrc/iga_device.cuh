@@ -61,26 +61,39 @@ inline cudaError_t launch_k(void (*kern)(KArgs...), dim3 grid, dim3 block, size_
     return cudaLaunchKernelEx(&cfg, kern, std::forward<Args>(args)...);
 }
 
-// launch_k() with an ordinary edge for grids of more CTAs than SMs: as
+// SMs of the current device.
+inline int device_sms()
+{
+    int nsm = 148, dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
+        nsm = 148;
+    return nsm;
+}
+
+// launch_k() with an ordinary edge for grids of more than `most` CTAs: as
 // programmatic dependents their CTAs start where the preceding grid's leave
-// first, and those SMs fill up while others stay empty (FP64 preconditioner
-// p=3 1024^2, GEMMs of 289 CTAs, up to three an SM: 173 us against 108; FP64
-// PCG 296 -> 233 us an iteration). Kernels bound by latency or bandwidth lose
-// less than the launch gap is worth (TF32 GEMMs at 1024^2: 37.6 us as
-// dependents, 42.2 with ordinary edges).
+// first, and those SMs fill up while others stay empty.
+template <typename... KArgs, typename... Args>
+inline cudaError_t launch_upto(long long most, void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t s,
+                               Args &&...args)
+{
+    const bool was = pdl_capture();
+    if ((long long)grid.x * grid.y * grid.z > most) pdl_capture() = false;
+    const cudaError_t e = launch_k(kern, grid, block, smem, s, std::forward<Args>(args)...);
+    pdl_capture() = was;
+    return e;
+}
+
+// The line for the solver's other kernels, at one CTA an SM: bound by latency
+// or bandwidth, they lose less to an uneven start than the launch gap is worth
+// (TF32 GEMMs at 1024^2: 37.6 us as dependents, 42.2 with ordinary edges; the
+// operator in an FP64 PCG iteration p=2 256^2 33.2 against 33.9, p=3 512^2, 147
+// CTAs, 67.3 against 67.7).
 template <typename... KArgs, typename... Args>
 inline cudaError_t launch_even(void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t s,
                                Args &&...args)
 {
-    const bool was = pdl_capture();
-    int nsm = 148, dev = 0;
-    if (was && (cudaGetDevice(&dev) != cudaSuccess ||
-                cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess))
-        nsm = 148;
-    if ((long long)grid.x * grid.y * grid.z > nsm) pdl_capture() = false;
-    const cudaError_t e = launch_k(kern, grid, block, smem, s, std::forward<Args>(args)...);
-    pdl_capture() = was;
-    return e;
+    return launch_upto(pdl_capture() ? device_sms() : 0, kern, grid, block, smem, s, std::forward<Args>(args)...);
 }
 
 // Launches a kernel that follows this call's own preceding kernel on s and

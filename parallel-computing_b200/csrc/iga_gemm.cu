@@ -587,9 +587,16 @@ int launch_f64(GemmOperand A, GemmOperand B, double *C, int ldc, int M, int N, i
         attr = true;
     }
     const dim3 grid(tiles_along(Mst, TM, split.on_n ? 0 : split.kb), tiles_along(Nst, TN, split.on_n ? split.kb : 0));
-    return launch_even(gemm_f64_kernel<CFG, AMN, BMN, SCATTER>, grid, dim3(NT), smem, s,
-                    static_cast<const double *>(A.ptr), A.ld, static_cast<const double *>(B.ptr), B.ld, C, ldc, M, N, K,
-                    Mst, Nst, sc, split) == cudaSuccess
+    // Bound by the FP64 tensor cores, of which the CTAs of an SM share one set:
+    // programmatic dependents only up to two thirds of a CTA an SM. Two CTAs on
+    // some SMs and none on others double the time (the preconditioner at p=3
+    // 700 x 650, 132 CTAs: 85 us against 58; 350^2 without the parity split 41.7
+    // against 26.8; 1024^2, GEMMs of 289 CTAs, 173 against 108), unless they
+    // are few and short (300^2 without it, 24.4 against 25.8).
+    const int most = pdl_capture() ? 2 * device_sms() / 3 : 0;
+    return launch_upto(most, gemm_f64_kernel<CFG, AMN, BMN, SCATTER>, grid, dim3(NT), smem, s,
+                       static_cast<const double *>(A.ptr), A.ld, static_cast<const double *>(B.ptr), B.ld, C, ldc, M, N,
+                       K, Mst, Nst, sc, split) == cudaSuccess
                ? IGA_OK
                : IGA_ERR_CUDA;
 }
@@ -626,9 +633,7 @@ int gemm_f64_launch(GemmOperand A, GemmOperand B, double *C, int ldc, int M, int
     // tiles of 64 x 64 for 148 SMs) 50.2 -> 31.9 us in all, 700^2 105 -> 53,
     // 1200^2 182 -> 165, 2048^2 681 -> 673; at 1024^2 (exactly two of 64 x 64
     // an SM) 64 x 64 stays, 108 against 117.
-    int nsm = 148, dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
-        nsm = 148;
+    const int nsm = device_sms();
     auto per_sm = [&](int t) {   // the most tiles of t x t an SM gets
         const long long n = (long long)tiles_along(Mst, t, split.on_n ? 0 : split.kb) *
                             tiles_along(Nst, t, split.on_n ? split.kb : 0);
