@@ -443,9 +443,9 @@ __global__ void __launch_bounds__(kBT) bk_cond(const int *__restrict__ act, int 
 //   stage 3: Z = Vx W1, scattered into z     (GEMM tiles)
 template <typename T>
 struct FdProb {
-    const T *Vx, *lx;      // x eigenvectors (column-major, ld nx) and eigenvalues
-    const T *VxT;          // the transpose of Vx (column-major), for the tcgen05 tiles
-    const T *Vxp, *VxTp;   // FP32: Vx and VxT as the A operands of the tcgen05 tiles (umma_a_index)
+    const T *lx;           // x eigenvalues
+    const T *Vx;           // FP64: the x eigenvectors (column-major, ld nx)
+    const T *Vxp, *VxTp;   // FP32: Vx and its transpose as the A operands of the tcgen05 tiles (umma_a_index)
     const T *Dv, *Cf;      // LDL^T factors of the y systems: 1 / pivot, upper off-diagonal; [b][a], ld nx
     const double *yc;      // free y nodes' pencil Kd | Ko | Md | Mo (ny each)
     T *W1;                 // nx * ny work matrix
@@ -560,14 +560,13 @@ __global__ void __launch_bounds__(32 * kRowSeg, sizeof(T) == 4 ? 2 : 1) fd_rows_
     }
 }
 
-// Tensor-core tiles: FP64 through DMMA (mma.sync m16n8k8, FP64 accumulate),
-// FP32 through TF32 MMA (mma.sync m16n8k8, operands rounded to TF32 once when
-// staged, FP32 accumulate): the FP32 preconditioner only has to be a close
-// SPD approximation of K_fem^-1 (the flexible PCG and the FP64 refinement
-// absorb the difference).
-// FP64: D (16 x 8) += A (16 x 8) B (8 x 8); fragments (g = lane / 4, t = lane % 4)
+// FP64 tiles through DMMA (mma.sync m16n8k8, FP64 accumulate); the FP32
+// preconditioner's are on tcgen05 (fd_umma_kernel): TF32 operands, FP32
+// accumulate, enough for it to be a close SPD approximation of K_fem^-1 (the
+// flexible PCG and the FP64 refinement absorb the difference).
+// D (16 x 8) += A (16 x 8) B (8 x 8); fragments (g = lane / 4, t = lane % 4)
 // a = A[g][t], A[g+8][t], A[g][t+4], A[g+8][t+4]; b = B[t][g], B[t+4][g];
-// d = D[g][2t], D[g][2t+1], D[g+8][2t], D[g+8][2t+1] (the layout of the FP32 tile).
+// d = D[g][2t], D[g][2t+1], D[g+8][2t], D[g+8][2t+1].
 __device__ __forceinline__ void mma_tile(double (&d)[4], const double (&a)[4], const double (&b)[2])
 {
     asm volatile(
@@ -577,17 +576,6 @@ __device__ __forceinline__ void mma_tile(double (&d)[4], const double (&a)[4], c
         : "d"(a[0]), "d"(a[1]), "d"(a[2]), "d"(a[3]), "d"(b[0]), "d"(b[1]));
 }
 
-__device__ __forceinline__ void mma_tile(float (&d)[4], const float (&a)[4], const float (&b)[2])
-{
-    asm volatile(
-        "mma.sync.aligned.m16n8k8.row.col.f32.tf32.tf32.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, "
-        "{%0, %1, %2, %3};"
-        : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
-        : "r"(__float_as_uint(a[0])), "r"(__float_as_uint(a[1])), "r"(__float_as_uint(a[2])),
-          "r"(__float_as_uint(a[3])), "r"(__float_as_uint(b[0])), "r"(__float_as_uint(b[1])));
-}
-
-__device__ __forceinline__ double to_operand(double v) { return v; }
 __device__ __forceinline__ float to_operand(float v)
 {
     uint32_t r;
@@ -595,15 +583,15 @@ __device__ __forceinline__ float to_operand(float v)
     return __uint_as_float(r);
 }
 
-// 64 x 64 output tile of one problem per CTA of 4 warps (2 x 2 warp tiles of
+// FP64 preconditioner tiles: 64 x 64 output tile of one problem per CTA of 4 warps (2 x 2 warp tiles of
 // 32 x 32). Operands contiguous along k in memory are staged as [row][k]
 // (ld 20), the others as [k][row] (ld 72): both make the fragment loads of a
 // warp conflict-free. Row / column blocks entirely outside the problem skip
 // their MMAs.
-template <typename T, int STAGE>
-__global__ void __launch_bounds__(128) fd_gemm_kernel(const FdProb<T> *__restrict__ fps, const int4 *__restrict__ tiles,
-                                                      const int *__restrict__ act, const T *__restrict__ rb,
-                                                      T *__restrict__ zb)
+template <int STAGE>
+__global__ void __launch_bounds__(128) fd_gemm_kernel(const FdProb<double> *__restrict__ fps, const int4 *__restrict__ tiles,
+                                                      const int *__restrict__ act, const double *__restrict__ rb,
+                                                      double *__restrict__ zb)
 {
     static_assert(STAGE == 1 || STAGE == 3, "stages 1 (W1 = Vx^T R) and 3 (Z = Vx W1)");
     constexpr bool A_KF = STAGE == 1;   // A contiguous along k: staged [a][k]
@@ -611,19 +599,19 @@ __global__ void __launch_bounds__(128) fd_gemm_kernel(const FdProb<T> *__restric
     constexpr int LKF = 20, LRF = 72;
     constexpr int SA = A_KF ? kTile * LKF : kTK * LRF;
     constexpr int SB = B_KF ? kTile * LKF : kTK * LRF;
-    __shared__ __align__(16) T As[2][SA];
-    __shared__ __align__(16) T Bs[2][SB];
+    __shared__ __align__(16) double As[2][SA];
+    __shared__ __align__(16) double Bs[2][SB];
     const int4 tl = tiles[blockIdx.x];
     if (!act[tl.x]) return;
-    const FdProb<T> &f = fps[tl.x];
+    const FdProb<double> &f = fps[tl.x];
     const int nx = f.nx, ny = f.ny, m = f.m;
     const int K = nx;
     const int a0 = tl.y * kTile, b0 = tl.z * kTile;
     const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
     const int g = lane >> 2, t4 = lane & 3;
     const int wm = (w & 1) * 32, wn = (w >> 1) * 32;
-    const T *r = rb + f.off;
-    T *z = zb + f.off;
+    const double *r = rb + f.off;
+    double *z = zb + f.off;
 
     if (STAGE == 1 && tl.y == 0 && tl.z == 0) {   // boundary ring: identity rows of K_fem
         const int n = f.n;
@@ -640,13 +628,13 @@ __global__ void __launch_bounds__(128) fd_gemm_kernel(const FdProb<T> *__restric
         }
     }
 
-    auto ldA = [&](int a, int k) -> T {
-        if (a >= nx || k >= K) return T(0);
+    auto ldA = [&](int a, int k) -> double {
+        if (a >= nx || k >= K) return 0.0;
         if (STAGE == 1) return f.Vx[(size_t)a * nx + k];          // Vx^T
         return f.Vx[(size_t)k * nx + a];                          // Vx (stage 3)
     };
-    auto ldB = [&](int k, int b) -> T {
-        if (k >= K || b >= ny) return T(0);
+    auto ldB = [&](int k, int b) -> double {
+        if (k >= K || b >= ny) return 0.0;
         if (STAGE == 1) return r[(size_t)(b + 1) * m + (k + 1)];   // R
         return f.W1[(size_t)b * nx + k];                          // W1 after the row solves (stage 3)
     };
@@ -660,7 +648,7 @@ __global__ void __launch_bounds__(128) fd_gemm_kernel(const FdProb<T> *__restric
             k = (tid >> 6) + 2 * i;
         }
     };
-    T ra[8], rbv[8];
+    double ra[8], rbv[8];
     auto fetch = [&](int k0) {
 #pragma unroll
         for (int i = 0; i < 8; ++i) {
@@ -676,24 +664,24 @@ __global__ void __launch_bounds__(128) fd_gemm_kernel(const FdProb<T> *__restric
         for (int i = 0; i < 8; ++i) {
             int row, k;
             coord(A_KF, i, row, k);
-            As[buf][A_KF ? row * LKF + k : k * LRF + row] = to_operand(ra[i]);
+            As[buf][A_KF ? row * LKF + k : k * LRF + row] = ra[i];
             coord(B_KF, i, row, k);
-            Bs[buf][B_KF ? row * LKF + k : k * LRF + row] = to_operand(rbv[i]);
+            Bs[buf][B_KF ? row * LKF + k : k * LRF + row] = rbv[i];
         }
     };
-    auto Aat = [&](int buf, int row, int k) -> T { return As[buf][A_KF ? row * LKF + k : k * LRF + row]; };
-    auto Bat = [&](int buf, int k, int col) -> T { return Bs[buf][B_KF ? col * LKF + k : k * LRF + col]; };
+    auto Aat = [&](int buf, int row, int k) -> double { return As[buf][A_KF ? row * LKF + k : k * LRF + row]; };
+    auto Bat = [&](int buf, int k, int col) -> double { return Bs[buf][B_KF ? col * LKF + k : k * LRF + col]; };
 
-    constexpr int MB = 2;      // row blocks of 16 rows in the warp tile (m16n8k8 in both precisions)
+    constexpr int MB = 2;      // row blocks of 16 rows in the warp tile (m16n8k8)
     constexpr int RB = 16;
     constexpr int NACC = 4;
-    T acc[MB][4][NACC];
+    double acc[MB][4][NACC];
 #pragma unroll
     for (int i = 0; i < MB; ++i)
 #pragma unroll
         for (int j = 0; j < 4; ++j)
 #pragma unroll
-            for (int c = 0; c < NACC; ++c) acc[i][j][c] = T(0);
+            for (int c = 0; c < NACC; ++c) acc[i][j][c] = 0.0;
     bool rv[MB], cv[4];
 #pragma unroll
     for (int i = 0; i < MB; ++i) rv[i] = a0 + wm + i * RB < nx;
@@ -708,8 +696,8 @@ __global__ void __launch_bounds__(128) fd_gemm_kernel(const FdProb<T> *__restric
         const int buf = kt & 1;
         if (kt + 1 < nk) fetch((kt + 1) * kTK);
 #pragma unroll
-        for (int kk = 0; kk < kTK; kk += 8) {   // m16n8k8: FP64 DMMA or TF32
-                T av[2][4], bv[4][2];
+        for (int kk = 0; kk < kTK; kk += 8) {   // m16n8k8
+                double av[2][4], bv[4][2];
 #pragma unroll
                 for (int i = 0; i < 2; ++i) {
                     const int r0 = wm + i * 16 + g;
@@ -743,7 +731,7 @@ __global__ void __launch_bounds__(128) fd_gemm_kernel(const FdProb<T> *__restric
                 const int a = a0 + wm + i * RB + g + (c >> 1) * 8;
                 const int b = b0 + wn + j * 8 + 2 * t4 + (c & 1);
                 if (a >= nx || b >= ny) continue;
-                const T v = acc[i][j][c];
+                const double v = acc[i][j][c];
                 if (STAGE == 1) f.W1[(size_t)b * nx + a] = v;
                 else z[(size_t)(b + 1) * m + (a + 1)] = v;
             }
@@ -753,7 +741,7 @@ __global__ void __launch_bounds__(128) fd_gemm_kernel(const FdProb<T> *__restric
 // kind::tf32): C[a + b ldc] = sum_k A[a][k] B[b ldb + k] for a 128 x 64
 // output tile of one problem, the FP32 accumulator in TMEM.
 //   stage 1: A rows = Vx columns (Vx^T), B rows = R^T (r + m + 1, ld m), C = W1
-//   stage 3: A rows = VxT columns (Vx),   B rows = W1^T (ld nx),        C = z + m + 1 (ld m)
+//   stage 3: A rows = Vx rows (Vx),        B rows = W1^T (ld nx),        C = z + m + 1 (ld m)
 // A, constant, is laid out at set-up as the shared memory images of its 32-wide
 // K slices, rounded to TF32: thread 0 brings each in with one bulk copy. B's
 // rows are not 16-byte aligned: all 128 threads stage its slices through
@@ -1142,9 +1130,9 @@ int batch_pc(iga_batch *B, int pc, const T *r, T *z, const int *act, cudaStream_
             fd_rows_kernel<T><<<B->nrows, dim3(32, kRowSeg), 0, s>>>(fd, B->rows, act);
             fd_umma_kernel<3><<<B->ntiles_tc, 128, kUmmaSmem, s>>>(fd, B->tiles_tc, act, r, z, B->d_err);
         } else {                          // FP64 tiles on DMMA
-            fd_gemm_kernel<T, 1><<<B->ntiles, 128, 0, s>>>(fd, B->tiles, act, r, z);
+            fd_gemm_kernel<1><<<B->ntiles, 128, 0, s>>>(fd, B->tiles, act, r, z);
             fd_rows_kernel<T><<<B->nrows, dim3(32, kRowSeg), 0, s>>>(fd, B->rows, act);
-            fd_gemm_kernel<T, 3><<<B->ntiles, 128, 0, s>>>(fd, B->tiles, act, r, z);
+            fd_gemm_kernel<3><<<B->ntiles, 128, 0, s>>>(fd, B->tiles, act, r, z);
         }
     }
     BT_TRY(cudaGetLastError());
@@ -1356,14 +1344,13 @@ __global__ void fd_ldl_kernel(const FdProb<double> *__restrict__ f64, const FdPr
 // half (half vectors at U + ue, hn_e long), the others from the odd half
 // (U + uo, hn_o long; uo < 0: a pencil that was not split, fe = n), scaled
 // by sc; mirrored entries v[n-1-i] = +-u[i]; lam: the n eigenvalues in the
-// same mode order. Outputs: V (component i of mode a at a n + i) and its
-// transpose VT in FP64 and, when Vp32 is set, both as tcgen05 A operands
-// (umma_a_index).
+// same mode order. Outputs: V (component i of mode a at a n + i) in FP64 and,
+// when Vp32 is set, it and its transpose as tcgen05 A operands (umma_a_index).
 struct BasisDev {
     int n, fe, hn_e, hn_o;
     long long ue, uo, lo;
     double sc;
-    double *V, *VT, *L;
+    double *V, *L;
     float *Vp32, *VTp32, *L32;
 };
 
@@ -1388,7 +1375,6 @@ __global__ void basis_build_kernel(const BasisDev *__restrict__ bs, const double
             v = (im < hn && im != i) ? (even ? b.sc : -b.sc) * u[im] : 0.0;
         }
         b.V[t] = v;
-        b.VT[(long long)i * n + a] = v;
         if (b.Vp32) {
             b.Vp32[umma_a_index(a, i, n)] = to_operand((float)v);
             b.VTp32[umma_a_index(i, a, n)] = to_operand((float)v);
@@ -1536,7 +1522,7 @@ int setup_fd(iga_batch *B)
     size_t tot64 = 0, tot32 = 0;
     for (const Basis &bb : bases) {
         const size_t n = (size_t)bb.n;
-        tot64 += 2 * al4(n * n) + al4(n);
+        tot64 += al4(n * n) + al4(n);
         if (mixed) tot32 += 2 * umma_a_size(bb.n) + al4(n);
     }
     double *b64 = nullptr;
@@ -1552,7 +1538,7 @@ int setup_fd(iga_batch *B)
         }
     }
     std::vector<BasisDev> bd(grids.size());
-    std::vector<double *> V64(grids.size()), VT64(grids.size()), L64(grids.size());
+    std::vector<double *> V64(grids.size()), L64(grids.size());
     std::vector<float *> Vp32(grids.size(), nullptr), VTp32(grids.size(), nullptr), L32(grids.size(), nullptr);
     {
         size_t o64 = 0, o32 = 0;
@@ -1560,9 +1546,8 @@ int setup_fd(iga_batch *B)
             const int n = bases[k].n;
             const size_t nn = (size_t)n * n;
             V64[k] = b64 + o64;
-            VT64[k] = V64[k] + al4(nn);
-            L64[k] = VT64[k] + al4(nn);
-            o64 += 2 * al4(nn) + al4(n);
+            L64[k] = V64[k] + al4(nn);
+            o64 += al4(nn) + al4(n);
             if (mixed) {
                 Vp32[k] = b32 + o32;
                 VTp32[k] = Vp32[k] + umma_a_size(n);
@@ -1579,7 +1564,6 @@ int setup_fd(iga_batch *B)
             d.lo = lo_of[k];
             d.sc = split[k] ? 1.0 / std::sqrt(2.0) : 1.0;
             d.V = V64[k];
-            d.VT = VT64[k];
             d.L = L64[k];
             d.Vp32 = Vp32[k];
             d.VTp32 = VTp32[k];
@@ -1625,7 +1609,6 @@ int setup_fd(iga_batch *B)
             const iga_plan *pl = B->plans[i];
             FdProb<T> &f = fp[i];
             f.Vx = pick(V64[bx[i]], nullptr);
-            f.VxT = pick(VT64[bx[i]], nullptr);
             f.Vxp = f64 ? nullptr : pick(nullptr, Vp32[bx[i]]);
             f.VxTp = f64 ? nullptr : pick(nullptr, VTp32[bx[i]]);
             f.lx = pick(L64[bx[i]], L32[bx[i]]);

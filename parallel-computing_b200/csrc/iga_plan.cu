@@ -445,12 +445,9 @@ static int split_for(int P, int prec, int geom)
 }
 
 // Rows per strip: the candidate whose CTA count fills the SMs best, with a
-// small penalty on short strips (more seam traffic). A MIXED plan launches
-// its FP64 and FP32 operators with different warps per CTA on the same
-// strips: each precision's cost is taken relative to its own best and the
-// candidate with the smallest sum wins. W: strips a CTA works on.
+// small penalty on short strips (more seam traffic).
 struct WarpShape {
-    int W;
+    int W;   // strips a CTA works on
     // also try the strip heights whose CTA count fills whole waves of SMs:
     // the kernels held back by each SM's own progress rather than by HBM (FP64
     // precomputed p >= 4, FP64 on-the-fly; p=4 1024^2: 57 rows, 144 CTAs,
@@ -488,28 +485,25 @@ int one_wave_rows(int nex, int ney, int P, int W, int nsm)
     return std::max({(int)((ney + nsy - 1) / nsy), P, 2});
 }
 
-static int rows_for(int nex, int ney, int P, const std::vector<WarpShape> &Ws, int nsm)
+static int rows_for(int nex, int ney, int P, WarpShape ws, int nsm)
 {
+    if (const int TY = one_wave_rows(nex, ney, P, ws.W, nsm)) return TY;
     const int NSX = (nex + kSW - 1) / kSW;
-    if (Ws.size() == 1)
-        if (const int TY = one_wave_rows(nex, ney, P, Ws[0].W, nsm)) return TY;
     std::vector<int> cands = {64, 56, 48, 40, 32, 28, 24, 20, 16};
-    for (const WarpShape &ws : Ws)
-        if (ws.waves)
-            for (int k = 1; k <= 16; ++k) {
-                const long long nsy = (long long)k * nsm * ws.W / NSX;   // strip rows of k full waves
-                if (nsy < 1) continue;
-                const int TY = (int)((ney + nsy - 1) / nsy);
-                if (TY >= 16 && TY <= 64 && std::find(cands.begin(), cands.end(), TY) == cands.end()) cands.push_back(TY);
-            }
-    std::vector<double> best_w(Ws.size(), 1e300);
-    for (size_t k = 0; k < Ws.size(); ++k)
-        for (int TY : cands) best_w[k] = std::min(best_w[k], strip_cost(NSX, ney, TY, Ws[k], nsm));
+    if (ws.waves)
+        for (int k = 1; k <= 16; ++k) {
+            const long long nsy = (long long)k * nsm * ws.W / NSX;   // strip rows of k full waves
+            if (nsy < 1) continue;
+            const int TY = (int)((ney + nsy - 1) / nsy);
+            if (TY >= 16 && TY <= 64 && std::find(cands.begin(), cands.end(), TY) == cands.end()) cands.push_back(TY);
+        }
+    double low = 1e300;
+    for (int TY : cands) low = std::min(low, strip_cost(NSX, ney, TY, ws, nsm));
+    // the first within 1e-9 of the lowest cost: the order above breaks ties
     int best = 64;
     double best_cost = 1e300;
     for (int TY : cands) {
-        double c = 0.0;
-        for (size_t k = 0; k < Ws.size(); ++k) c += strip_cost(NSX, ney, TY, Ws[k], nsm) / best_w[k];
+        const double c = strip_cost(NSX, ney, TY, ws, nsm) / low;
         if (c < best_cost - 1e-9) {
             best_cost = c;
             best = TY;
@@ -644,10 +638,9 @@ static int launch_apply_t(iga_plan *pl, const OperatorData &op, const T *x, T *y
     }
     const StripGrid &g = op.grid;
     const int rows = win.gyn >= 0 ? std::min(win.gyn, g.NSY - win.gy0) : g.NSY;
-    // shared x tables: a CTA's strips lie in at most two column strips when
-    // W - 1 <= rows, in one when W divides rows (one slot: the shared memory
-    // of the one-column layout, which matters where a kernel's spills live
-    // in L1: FP64 on-the-fly p=5 512^2 189 -> 257 us with a second slot)
+    // Shared x tables: a CTA's strips lie in at most two column strips when
+    // S - 1 <= rows, in one when S divides rows (one slot then, which leaves L1
+    // the other's shared memory).
     // Fewer strips than one wave of full CTAs: as many warps per CTA as spread
     // them over all SMs (p=3 512^2 FP64, 16-row strips: 33.1 us in 86 CTAs of
     // 12 warps, 29.4 us in 147 of 7).
@@ -851,9 +844,8 @@ int iga_plan_create(const iga_mesh_desc *d, const iga_opts *opts_in, iga_plan **
     auto rows_of = [&](int prec) {
         if (opts.rows_per_strip > 0) return opts.rows_per_strip;
         const bool waves = prec == IGA_FP64 && (opts.geometry == IGA_GEOM_ON_THE_FLY || P.p >= 4);
-        return rows_for(P.nex, P.ney, P.p, {{warps_for(P.p, prec, opts.geometry) / split_for(P.p, prec, opts.geometry),
-                                              waves}},
-                        nsm);
+        return rows_for(P.nex, P.ney, P.p,
+                        {warps_for(P.p, prec, opts.geometry) / split_for(P.p, prec, opts.geometry), waves}, nsm);
     };
     auto make_grid = [&](int TY) {
         StripGrid g;
