@@ -32,11 +32,6 @@
 
 namespace iga {
 
-// Largest geometry streamed with policy_once(): past it there is nothing of the
-// stream to keep, and a MatMult alone was slower with it (p=3 2048^2 FP64, 1.6
-// GB, 298 -> 301 us; FP32, 0.8 GB, 157 -> 156 us).
-constexpr size_t kOnceBytes = size_t(1) << 30;
-
 template <typename T>
 struct ApplyParams {
     const T *x;
@@ -62,8 +57,6 @@ struct ApplyParams {
     const int *ID = nullptr;
     // Polls of each wait for a G stage before it reports IGA_ERR_TIMEOUT.
     long long wait_polls = kWaitLimit;
-    // G streamed with policy_once(): geometry up to kOnceBytes
-    int g_once = 1;
 };
 
 // Stores sign * v for control point i = R m + C under boundary rule bc
@@ -286,7 +279,7 @@ __device__ __forceinline__ void apply_tile(const ApplyParams<T> &a, const T *__r
     // The policy is held in registers, except where those two make the kernel
     // spill more (FP32 p = 5, 800^2: 86 -> 93 us): made at each use there.
     constexpr bool HOLD = !(sizeof(T) == 4 && P == 5);
-    const uint64_t pol = GEOM == 0 && HOLD ? (a.g_once ? policy_once() : policy_normal()) : 0;
+    const uint64_t pol = GEOM == 0 && HOLD ? policy_once() : 0;
     auto fetch_g = [&](T *dst, const T *src, uint64_t *bar) {
         bulk_g2s(dst, src, S::GBYTES, bar, HOLD ? pol : policy_once());
     };

@@ -162,24 +162,19 @@ __device__ __forceinline__ void bulk_g2s(void *dst, const void *src, uint32_t by
 }
 
 // The same with an L2 policy. policy_once() is for data one kernel reads once
-// (a strip's geometry): its lines are the first to be replaced, so that a geometry larger than L2 does not push
-// out the vectors the next kernels read, and one about as large as L2 keeps
-// some of itself (an LRU of a cyclic stream keeps nothing). Measured, FP64 /
-// mixed PCG an iteration: p=3 512^2 78 -> 70 / 59 -> 58 us, 1024^2 232 -> 216 / 117
-// -> 107 us, 2048^2 1093 -> 1080 / 333 -> 316 us; MatMult p=3 1024^2 FP64 83.6 ->
-// 76.7 us, p=4 1024^2 FP32 72.5 -> 69.7 us. Marking a fixed part of it to stay
-// instead gained half of that.
+// (a strip's geometry): its lines are the first to be replaced, so that a
+// geometry larger than L2 does not push out the vectors the next kernels read,
+// and one about as large as L2 keeps some of itself (an LRU of a cyclic stream
+// keeps nothing). Measured: FP64 PCG an iteration, p=3 700^2 185 -> 172 us, 1024^2
+// 225 -> 212, 1600^2 596 -> 573, 2048^2 1063 -> 1050, p=4 1024^2 287 -> 277; MatMult
+// FP64 p=3 1024^2 80.9 -> 74.8 us, 1600^2 177 -> 165, 2048^2 298 -> 285, FP32 2048^2
+// 157 -> 154, 2600^2 261 -> 255, p=5 1700^2 351 -> 338 (at the full clock; a GPU held
+// at its power limit by a second of MatMults takes 309 and 305 us at FP64
+// 2048^2). Marking a fixed part of it to stay instead gained half of that.
 __device__ __forceinline__ uint64_t policy_once()
 {
     uint64_t p;
     asm volatile("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(p));
-    return p;
-}
-
-__device__ __forceinline__ uint64_t policy_normal()
-{
-    uint64_t p;
-    asm volatile("createpolicy.fractional.L2::evict_normal.b64 %0, 1.0;" : "=l"(p));
     return p;
 }
 

@@ -628,7 +628,6 @@ static int launch_apply_t(iga_plan *pl, const OperatorData &op, const T *x, T *y
     a.err = pl->d_err;
     a.ID = win.ID;
     if (pl->wait_polls >= 0) a.wait_polls = pl->wait_polls;
-    a.g_once = op.geom_bytes <= kOnceBytes;
     auto kern = apply_kernel<P, T, GEOM, NST>;
     static bool attr_set = false;   // per template instance: the most any launch below asks for
     if (!attr_set) {
