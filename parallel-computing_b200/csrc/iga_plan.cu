@@ -481,6 +481,10 @@ int one_wave_rows(int nex, int ney, int P, int W, int nsm)
 {
     const long long NSX = (nex + kSW - 1) / kSW, warps = (long long)nsm * W;
     if (NSX * ((ney + 15) / 16) > warps) return 0;
+    // three rows (p = 1: four) in one strip: the seams' launch costs more than
+    // they do (p=2 16 x 3 FP64 8.2 -> 6.2 us, p=1 12 x 4 on-the-fly 8.2 -> 6.4; p=2
+    // 12 x 4 on-the-fly 10.3 against 11.2 in one strip, so two)
+    if (NSX == 1 && ney <= 5 - P) return std::max({ney, P, 2});
     const long long nsy = warps / NSX;
     return std::max({(int)((ney + nsy - 1) / nsy), P, 2});
 }

@@ -257,3 +257,21 @@ def test_batch_vectors_start_anywhere(torch_cuda, ib, orc, prec):
         r = b[s:e] - orc.apply_mf(m, x[s:e], sign=1.0, bc=1)
         assert np.linalg.norm(r) <= 2e-10 * np.linalg.norm(b[s:e]), points[i]
     batch.close()
+
+
+# Patches of a few rows: one strip while one strip wide and three rows high (p =
+# 1: four), so that a MatMult is one launch; one row or column more and it is two.
+@pytest.mark.parametrize("p,nex,ney,one", [(1, 16, 4, True), (1, 12, 5, False), (1, 3, 3, True), (2, 16, 3, True),
+                                           (2, 5, 4, False), (2, 17, 3, False), (3, 9, 3, True), (4, 7, 1, True),
+                                           (5, 16, 1, True)])
+@pytest.mark.parametrize("geom", [0, 1])
+def test_patches_of_a_few_rows(torch_cuda, ib, orc, p, nex, ney, one, geom):
+    M = distorted(ib.unit_square(p, nex, ney))
+    x = splitmix_uniform(p * 10 + nex, -1.0, 1.0, (nex + p) * (ney + p))
+    plan = ib.Plan(M, geometry=geom)
+    assert (plan.info.rows_per_strip >= ney) == one
+    xd = torch_cuda.from_numpy(x).cuda()
+    yd = torch_cuda.full_like(xd, float("nan"))
+    plan.apply(xd, yd)
+    assert rel(yd.cpu().numpy(), orc.apply_mf(M, x)) < 1e-12
+    plan.close()
