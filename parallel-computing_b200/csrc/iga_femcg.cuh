@@ -183,22 +183,28 @@ __global__ void __launch_bounds__(kIcgMaxThreads, 1) icg_cluster_kernel(IcgArgs<
         mbar_arrive_expect_tx(&bar[1], tx2);
     }
 
+    // The x stiffness and mass go in scaled to about 1 by powers of two, which
+    // the y factors undo (exactly): K's products of the two are about 1 whatever
+    // the mesh width, so its rows overflow and underflow no earlier than p does.
+    auto scale = [](T v) { return v > T(0) && isfinite(v) ? (T)scalbn(T(1), -ilogb(v)) : T(1); };
+    const T sk = scale(a.kd[m / 2]), sm = scale(a.md[m / 2]), uk = T(1) / sk, um = T(1) / sm;
+
     // couplings of row j: none across the boundary ring
     for (int k = t; k < nr; k += nt) {
         const int j = j0 + k;
         const bool in = j > 0 && j < n - 1, lo = in && j - 1 >= 1, hi = in && j + 1 <= n - 2;
-        yc[6 * k + 0] = lo ? a.lo[j - 1] : T(0);
-        yc[6 * k + 1] = in ? a.ld[j] : T(0);
-        yc[6 * k + 2] = hi ? a.lo[j] : T(0);
-        yc[6 * k + 3] = lo ? a.no[j - 1] : T(0);
-        yc[6 * k + 4] = in ? a.nd[j] : T(0);
-        yc[6 * k + 5] = hi ? a.no[j] : T(0);
+        yc[6 * k + 0] = lo ? um * a.lo[j - 1] : T(0);
+        yc[6 * k + 1] = in ? um * a.ld[j] : T(0);
+        yc[6 * k + 2] = hi ? um * a.lo[j] : T(0);
+        yc[6 * k + 3] = lo ? uk * a.no[j - 1] : T(0);
+        yc[6 * k + 4] = in ? uk * a.nd[j] : T(0);
+        yc[6 * k + 5] = hi ? uk * a.no[j] : T(0);
     }
     const int i = t % m, k0 = (t / m) * L;   // this thread's column and first row of the band
     const int cnt = min(L, nr - k0);         // its rows (may be <= 0)
     const bool xin = i > 0 && i < m - 1, xlo = xin && i - 1 >= 1, xhi = xin && i + 1 <= m - 2;
-    const T kxl = xlo ? a.ko[i - 1] : T(0), kxd = xin ? a.kd[i] : T(0), kxr = xhi ? a.ko[i] : T(0);
-    const T mxl = xlo ? a.mo[i - 1] : T(0), mxd = xin ? a.md[i] : T(0), mxr = xhi ? a.mo[i] : T(0);
+    const T kxl = xlo ? sk * a.ko[i - 1] : T(0), kxd = xin ? sk * a.kd[i] : T(0), kxr = xhi ? sk * a.ko[i] : T(0);
+    const T mxl = xlo ? sm * a.mo[i - 1] : T(0), mxd = xin ? sm * a.md[i] : T(0), mxr = xhi ? sm * a.mo[i] : T(0);
     auto inv_diag = [&](int ii, int j) -> T {
         const bool in = ii > 0 && ii < m - 1 && j > 0 && j < n - 1;
         return in ? T(1) / (a.kd[ii] * a.nd[j] + a.md[ii] * a.ld[j]) : T(1);

@@ -163,3 +163,22 @@ def test_device_and_host_loops_agree(torch_cuda, ib, p, nex, ney, pc, prec):
             assert got[0][1:] == got[1][1:]
             assert torch.equal(got[0][0], got[1][0])
     plan.close()
+
+
+# Powers of two pass through the iteration unchanged while nothing overflows:
+# entries up to 2^126 of FP32's 2^128, and well inside the rest of both ranges,
+# although the mesh's stiffness factors are about 130 (64 elements) to 2000
+# (1000) and its mass factors as much under 1.
+@pytest.mark.parametrize("prec,k", [(1, 126), (1, -80), (0, 400), (0, -400)])
+@pytest.mark.parametrize("nex,ney", [(64, 64), (3, 1000), (40, 33)])
+def test_scaled_right_hand_sides(torch_cuda, ib, nex, ney, prec, k):
+    torch = torch_cuda
+    plan = ib.Plan(ib.unit_square(2, nex, ney))
+    r = random_vector(torch, plan, nex, torch.float32 if prec else torch.float64)
+    got = []
+    for scale in (1.0, 2.0 ** k):
+        z = torch.full_like(r, float("nan"))
+        plan.pc_apply(r * scale, z, pc=ib.PC_FEM_CG, precision=prec, pc_max_it=1)
+        got.append(z / scale)
+    assert torch.equal(got[0], got[1])
+    plan.close()
