@@ -210,6 +210,12 @@ __global__ void __launch_bounds__(kIcgMaxThreads, 1) icg_cluster_kernel(IcgArgs<
         return in ? T(1) / (a.kd[ii] * a.nd[j] + a.md[ii] * a.ld[j]) : T(1);
     };
 
+    // An infinite entry of the boundary ring is no neighbour of an interior one,
+    // but its zero coupling would make NaN of it there: the first direction holds
+    // 1 in its place, and r.z is NaN, which makes NaN of z and ends the solve
+    // after one iteration.
+    auto ring_inf = [&](int ii, int j, T p) { return isinf(p) && (ii == 0 || j == 0 || ii == m - 1 || j == n - 1); };
+
     T r[L], z[L], di[L];
     double v0 = 0.0, v1 = 0.0;
 #pragma unroll
@@ -221,8 +227,9 @@ __global__ void __launch_bounds__(kIcgMaxThreads, 1) icg_cluster_kernel(IcgArgs<
             r[l] = a.rhs[(size_t)j * m + i];
             di[l] = inv_diag(i, j);
             const T p = r[l] * di[l];
-            ps[(size_t)(k0 + l + 1) * m + i] = p;
-            v0 += (double)r[l] * (double)p;
+            const bool inf = ring_inf(i, j, p);
+            ps[(size_t)(k0 + l + 1) * m + i] = inf ? T(1) : p;
+            v0 += inf ? nan("") : (double)r[l] * (double)p;
             v1 += (double)r[l] * (double)r[l];
         }
     }
@@ -231,6 +238,7 @@ __global__ void __launch_bounds__(kIcgMaxThreads, 1) icg_cluster_kernel(IcgArgs<
         const int up = u >= m, ii = up ? u - m : u, j = up ? j0 + nr : j0 - 1;
         T p = T(0);
         if (nr > 0 && j >= 0 && j < n) p = a.rhs[(size_t)j * m + ii] * inv_diag(ii, j);
+        if (ring_inf(ii, j, p)) p = T(1);
         ps[(size_t)(up ? nr + 1 : 0) * m + ii] = p;
     }
     if (t == 0) ps[-1] = ps[(size_t)m * (rows + 2)] = T(0);

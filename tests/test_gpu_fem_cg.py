@@ -165,6 +165,24 @@ def test_device_and_host_loops_agree(torch_cuda, ib, p, nex, ney, pc, prec):
     plan.close()
 
 
+# An infinite entry of the boundary ring couples to no interior one: no
+# breakdown, but a residual norm without meaning, so NaN everywhere, in one
+# cluster (1, 8 and 16 CTAs) as past it (600 x 300: a launch per step).
+@pytest.mark.parametrize("prec", [0, 1])
+@pytest.mark.parametrize("nex,ney", [(20, 1), (40, 33), (255, 62), (600, 300)])
+@pytest.mark.parametrize("where", ["corner", "side", "top"])
+def test_infinity_on_the_boundary_ring(torch_cuda, ib, nex, ney, prec, where):
+    torch = torch_cuda
+    plan = ib.Plan(ib.unit_square(2, nex, ney))
+    m, n = nex + 2, ney + 2
+    r = random_vector(torch, plan, nex, torch.float32 if prec else torch.float64)
+    r[{"corner": 0, "side": (n // 2) * m, "top": (n - 1) * m + m // 2}[where]] = float("-inf")
+    z = torch.full_like(r, 3.0)
+    plan.pc_apply(r, z, pc=ib.PC_FEM_CG, precision=prec)
+    assert bool(torch.isnan(z).all())
+    plan.close()
+
+
 # Powers of two pass through the iteration unchanged while nothing overflows:
 # entries up to 2^126 of FP32's 2^128, and well inside the rest of both ranges,
 # although the mesh's stiffness factors are about 130 (64 elements) to 2000
