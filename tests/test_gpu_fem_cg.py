@@ -200,3 +200,61 @@ def test_scaled_right_hand_sides(torch_cuda, ib, nex, ney, prec, k):
         got.append(z / scale)
     assert torch.equal(got[0], got[1])
     plan.close()
+
+
+def fem_diagonal(gx, gy):
+    """Diagonal of the bilinear FEM matrix on the tensor grid gx x gy, 1 on the boundary ring."""
+    def factors(g):
+        h = np.diff(g)
+        return 1.0 / h[:-1] + 1.0 / h[1:], (h[:-1] + h[1:]) / 3.0
+    (kx, mx), (ky, my) = factors(gx), factors(gy)
+    d = np.ones((len(gy), len(gx)))
+    d[1:-1, 1:-1] = np.outer(my, kx) + np.outer(ky, mx)
+    return d.ravel()
+
+
+# A cap of one inner iteration: z = alpha p with p = r / diag and alpha = r.p /
+# p.Kp, in one cluster (rows per thread as above) and past it. A row of K p is
+# nine terms of about one rounding each and the sums are FP64: 1e-12 and 1e-5.
+@pytest.mark.parametrize("prec,tol", [(0, 1e-12), (1, 1e-5)])
+@pytest.mark.parametrize("p,nex,ney", [(2, 64, 64), (3, 40, 1), (1, 2, 30), (2, 17, 90), (3, 300, 125), (2, 600, 300)])
+def test_one_inner_iteration(torch_cuda, ib, orc, p, nex, ney, prec, tol):
+    torch = torch_cuda
+    plan = ib.Plan(ib.unit_square(p, nex, ney))
+    gx, gy = plan.fem_nodes()
+    rd = random_vector(torch, plan, nex + p, torch.float32 if prec else torch.float64)
+    z = torch.full_like(rd, float("nan"))
+    plan.pc_apply(rd, z, pc=ib.PC_FEM_CG, precision=prec, pc_rtol=1e-14, pc_max_it=1)
+    r = rd.double().cpu().numpy()
+    d = r / fem_diagonal(gx, gy)
+    ref = (r @ d) / (d @ orc.fem_matvec(gx, gy, d)) * d
+    assert np.abs(z.double().cpu().numpy() - ref).max() <= tol * np.abs(ref).max()
+    plan.close()
+
+
+# Inner caps and tolerances belong to the call: a plan that has solved with
+# others does as many inner iterations, and gives the same bits, as one that has
+# not.
+@pytest.mark.parametrize("prec", ["FP64", "MIXED", "MIXED_PC"])
+def test_inner_options_of_each_solve(torch_cuda, ib, prec):
+    torch = torch_cuda
+    mesh = ib.unit_square(2, 50, 44)
+    b = free_vector(torch, mesh, 12)
+    options = [dict(pc_max_it=4, pc_rtol=1e-10), dict(pc_max_it=9, pc_rtol=1e-10), dict(pc_max_it=500, pc_rtol=1e-2),
+               dict(pc_max_it=500, pc_rtol=1e-4), dict(pc_max_it=4, pc_rtol=1e-10)]
+
+    def solve(plan, kw):
+        x = torch.zeros_like(b)
+        st = plan.solve(b, x, check=False, precision=getattr(ib, prec), pc=ib.PC_FEM_CG, max_it=5, max_sweeps=2, **kw)
+        return x, st.iterations, st.pc_iterations
+
+    shared = ib.Plan(mesh, precision=ib.MIXED)
+    counts = []
+    for kw in options:
+        fresh = ib.Plan(mesh, precision=ib.MIXED)
+        (x, *n), (x2, *n2) = solve(shared, kw), solve(fresh, kw)
+        assert n == n2 and torch.equal(x, x2)
+        counts.append(n[1])
+        fresh.close()
+    assert len(set(counts)) == 4 and counts[0] == counts[4]
+    shared.close()

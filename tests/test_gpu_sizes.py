@@ -53,8 +53,8 @@ def test_strip_height_of_small_patches(torch_cuda, ib, orc, p, nex, ney, geom):
     plan.close()
 
 
-# The inner FEM-CG in one cluster: one row per thread (64^2), two, four and
-# eight, fewer grid rows than CTAs, a 3-node direction, the first sizes past
+# The inner FEM-CG in one cluster: one row per thread (40 x 1), two (1 x 1),
+# four (64^2) and eight (300 x 125), fewer grid rows than CTAs, a 3-node direction, the first sizes past
 # the cluster (600 x 300: the launch-per-step path). Its stop is the recurrence
 # residual at pc_rtol; the true residual may exceed it by the rounding of the
 # iteration, well under pc_rtol itself in FP64 (condition ~ 1e4 x 1e-16); in
@@ -74,7 +74,7 @@ def test_fem_cg_in_a_cluster(torch_cuda, ib, orc, p, nex, ney, prec):
     rr = rd.double().cpu().numpy()
     res = orc.fem_matvec(gx, gy, zd.double().cpu().numpy()) - rr
     assert np.linalg.norm(res) <= 2 * tol * np.linalg.norm(rr)
-    # the same call twice gives the same bits; one iteration at most: z = alpha r / diag
+    # the same call twice gives the same bits
     z2 = torch_cuda.full_like(rd, float("nan"))
     plan.pc_apply(rd, z2, pc=ib.PC_FEM_CG, precision=prec, pc_rtol=tol)
     assert torch_cuda.equal(zd, z2)
