@@ -48,14 +48,13 @@ inline size_t icg_smem(int m, int rows, int C, int nw)
 }
 
 // Shape k = 0 .. 3 in the order of preference (C = 0: does not fit, or no
-// further shape). Eight CTAs (the portable cluster size) before sixteen, whose
-// sums have twice the slots (64^2 with cluster
-// barriers: 3.2 us an iteration against 2.9), and four
-// rows per thread where the band has them: with fewer, more warps share the
-// SM's shuffle and shared-memory pipes for their sums (64^2, eight CTAs: 3.27
-// us with one row per thread, 3.15 with two, 2.90 with four), with eight a
-// thread's own rows dominate (4.13; 128^2: 5.0 us in eight CTAs of eight
-// rows, 4.1 in sixteen of four).
+// further shape). Four rows per thread before eight, whose own rows dominate
+// an iteration, and eight CTAs (the portable cluster size) before sixteen,
+// whose sums have twice the slots. FP64, us an iteration, in CTAs x rows per
+// thread: 64^2 8 x 4 2.25, 16 x 4 2.22, 8 x 8 3.65, 16 x 8 3.23; 128^2 16 x 4 2.85,
+// 8 x 8 4.35. Other shapes would be a little faster where they fit (64^2 8 x 2
+// 2.00, 16^2 8 x 1 1.05 against 1.14, 96^2 16 x 4 2.42 against 2.71): fewer rows
+// per thread lost only with the cluster barriers that the mbarriers replaced.
 template <typename T>
 inline IcgShape icg_shape(int m, int n, int k)
 {

@@ -629,10 +629,10 @@ int gemm_f64_launch(GemmOperand A, GemmOperand B, double *C, int ldc, int M, int
     // A GEMM lasts as long as the SM with the most tiles. A 64 x 64 tile takes
     // about a tenth less time than four of 32 x 32 (fewer fragment loads per
     // MMA), so the small ones are used where they give the fullest SM that
-    // much less: the preconditioner's two half-size transforms at p=3 512^2 (81
-    // tiles of 64 x 64 for 148 SMs) 50.2 -> 31.9 us in all, 700^2 105 -> 53,
-    // 1200^2 182 -> 165, 2048^2 681 -> 673; at 1024^2 (exactly two of 64 x 64
-    // an SM) 64 x 64 stays, 108 against 117.
+    // much less: the preconditioner at p=3 512^2 (transforms of 81 tiles of 64 x
+    // 64 for 148 SMs) 52 -> 31 us in all, 1200^2 173 -> 156, 2048^2 680 -> 673; at
+    // 1024^2 (two of 64 x 64 an SM) 64 x 64 stays, 105 against 115. The line does
+    // not see SMs left empty: at 700^2 (132 tiles) 64 x 64 stays with 58 against 50.
     const int nsm = device_sms();
     auto per_sm = [&](int t) {   // the most tiles of t x t an SM gets
         const long long n = (long long)tiles_along(Mst, t, split.on_n ? 0 : split.kb) *
